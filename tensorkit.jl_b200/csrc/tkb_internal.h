@@ -126,6 +126,11 @@ struct tkb_table {
   int64_t nrow_tasks = 0;
   TaskRec *row_rec = nullptr;
   int64_t row_pair_elems = 0;     // elements of row tasks that 16-byte pair accesses can copy
+  // tables with multi-tree groups that keep their fastest dim: records of the register recoupling
+  // kernel (multi_words words each, groups of at most multi_trees source trees)
+  int64_t nmulti_tasks = 0;
+  int multi_words = 0, multi_trees = 1;
+  int64_t *multi_rec = nullptr;
 };
 
 int tkb_transform_launch(tkb_ctx *ctx, const tkb_table *t, int dtype, void *dst,

@@ -60,7 +60,8 @@ __device__ __forceinline__ double finish(double v, double a, double b, const dou
 }
 __device__ __forceinline__ double2 finish(double2 v, double2 a, double2 b, const double2 *d,
                                           bool bz) {
-  double2 r = make_double2(a.x * v.x - a.y * v.y, a.x * v.y + a.y * v.x);
+  // one rounding order in every kernel, so that they agree bit for bit
+  double2 r = make_double2(fma(a.x, v.x, -__dmul_rn(a.y, v.y)), fma(a.x, v.y, __dmul_rn(a.y, v.x)));
   if (!bz) {
     double2 o = *d;
     r.x = fma(b.x, o.x, fma(-b.y, o.y, r.x));
@@ -439,6 +440,108 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 && !PAIRS) ? 6 : 4)
   }
 }
 
+// ---- register recoupling kernel for tables with multi-tree groups ---------------------------
+// A group (nsrc source trees, ndst destination trees, one shared sub-block shape) is
+// recoupled element by element: a thread loads the nsrc source values of P positions into
+// registers, forms the ndst combinations with U and stores them. Nothing is staged, so there is no
+// barrier between a tile's loads and its stores and the kernel is bound by the loads in flight.
+// Tiles are exact boxes of up to kMultiTile positions over three dims: a (fastest on both sides), b
+// (the next source dim) and c (the next destination dim); the runs that b and c make contiguous
+// meet in L2, which turns rows of 8 - 30 elements into whole sectors on both sides. A task's
+// record (bases and strides of every tree, U) is one contiguous run of words; the record of
+// the CTA's next task is fetched while the current one runs. Row decomposition by multiply-high as
+// in the row-copy kernel.
+// Permute ((1,3),(2,4)) of an SU(2) four-leg tensor (45.6 M elements, blocks of up to 5 trees, rows
+// of 8 - 30 elements): MULTI_FIGURES.
+constexpr int kMultiMaxTrees = 8;     // source trees per group held in registers
+constexpr int kMultiTile = 2048;      // positions per task at most
+constexpr int kMultiHdrWords = 4;     // MultiHdr
+constexpr int kMultiTreeWords = 3;    // MultiTree
+constexpr int kMultiMaxWords = 248;   // a record is fetched by one word per thread
+struct MultiHdr {
+  int32_t na, nb, nc, n;     // extents of the box and their product
+  int32_t nsrc, ndst;
+  uint32_t mul_a, mul_b;     // reciprocals of na and nb (0 for extent 1)
+};
+struct MultiTree {
+  int64_t base;              // element offset of the box's first element
+  int32_t sa, sb, sc, pad;   // strides of a, b, c
+};
+
+template <typename T, bool CONJ, int NS, int P>
+__global__ void __launch_bounds__(kThreads, NS * P * sizeof(T) <= 96 ? 3 : 2)
+    treetransform_multi_kernel(const int64_t *__restrict__ recs, int rec_words, int64_t ntasks,
+                               T *__restrict__ dst, const T *__restrict__ src, CDbl alpha_, CDbl beta_,
+                               int beta_zero) {
+  __shared__ __align__(16) int64_t buf[2][kThreads];
+  const T alpha = scalar_from<T>(alpha_);
+  const T beta = scalar_from<T>(beta_);
+  const bool bz = beta_zero != 0;
+  pdl_trigger();  // the next kernel may be scheduled; it waits for this grid before reading
+  int64_t task = blockIdx.x;
+  if ((int)threadIdx.x < rec_words) buf[0][threadIdx.x] = __ldg(recs + task * rec_words + threadIdx.x);
+  __syncthreads();
+  pdl_wait();  // the records are static; source and destination belong to earlier kernels
+  for (int cur = 0; task < ntasks; cur ^= 1) {
+    const int64_t next = task + gridDim.x;
+    int64_t word = 0;
+    const bool fetch = next < ntasks && (int)threadIdx.x < rec_words;
+    if (fetch) word = __ldg(recs + next * rec_words + threadIdx.x);
+    const MultiHdr h = *reinterpret_cast<const MultiHdr *>(buf[cur]);
+    const MultiTree *tr = reinterpret_cast<const MultiTree *>(buf[cur] + kMultiHdrWords);
+    const double *U = reinterpret_cast<const double *>(buf[cur] + kMultiHdrWords + kMultiTreeWords * (h.nsrc + h.ndst));
+    for (int e0 = 0; e0 < h.n; e0 += kThreads * P) {
+      int ia[P], ib[P], ic[P];
+      bool ok[P];
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+        const int e = e0 + p * kThreads + threadIdx.x;
+        ok[p] = e < h.n;
+        const int q = h.mul_a ? (int)__umulhi((unsigned)e, h.mul_a) : e;
+        ia[p] = e - q * h.na;
+        ic[p] = h.mul_b ? (int)__umulhi((unsigned)q, h.mul_b) : q;
+        ib[p] = q - ic[p] * h.nb;
+      }
+      T v[NS][P];
+#pragma unroll
+      for (int j = 0; j < NS; ++j) {
+        if (j < h.nsrc) {
+          const MultiTree t = tr[j];
+          const T *sp = src + t.base;
+#pragma unroll
+          for (int p = 0; p < P; ++p)
+            v[j][p] = ok[p] ? ld_val(sp + (ia[p] * t.sa + ib[p] * t.sb + ic[p] * t.sc), CONJ) : zero_val(T{});
+        }
+      }
+      for (int i = 0; i < h.ndst; ++i) {
+        const MultiTree t = tr[h.nsrc + i];
+        T *dp0 = dst + t.base;
+        T acc[P];
+#pragma unroll
+        for (int p = 0; p < P; ++p) acc[p] = zero_val(T{});
+#pragma unroll
+        for (int j = 0; j < NS; ++j) {
+          if (j < h.nsrc) {
+            const double u = U[i * h.nsrc + j];
+#pragma unroll
+            for (int p = 0; p < P; ++p) acc[p] = axpy_r(u, v[j][p], acc[p]);
+          }
+        }
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+          if (ok[p]) {
+            T *dp = dp0 + (ia[p] * t.sa + ib[p] * t.sb + ic[p] * t.sc);
+            *dp = finish(acc[p], alpha, beta, dp, bz);
+          }
+        }
+      }
+    }
+    if (fetch) buf[cur ^ 1][threadIdx.x] = word;
+    __syncthreads();
+    task = next;
+  }
+}
+
 // TKB_TRANSFORM_KERNEL selects a kernel for comparison: "plain" the non-pipelined kernel for
 // every table, "pipe" the staged ring for every single-tree table (no row-copy kernel)
 bool use_plain_transform() {
@@ -454,6 +557,76 @@ int64_t pow2ceil(int64_t x) {
   int64_t p = 1;
   while (p < x) p <<= 1;
   return p;
+}
+
+// A group whose U falls apart into independent pieces (no nonzero coefficient couples
+// them) is handed on as one group per piece: every piece reads and writes only the trees it needs.
+// Permutations that only exchange legs of one side, or none, have a diagonal U, so their tables
+// become tables of single-tree groups. A destination tree whose coefficients are all zero still
+// gets β·dst, so it joins the piece of the first source tree.
+struct SplitTable {
+  std::vector<int64_t> gsp, gdp, cp, sizes, sstr, soff, dstr, doff;
+  std::vector<double> coef;
+};
+
+bool split_groups(const tkb_table_desc *d, SplitTable *o) {
+  const int N = d->nind;
+  bool any = false;
+  o->gsp.push_back(0);
+  o->gdp.push_back(0);
+  o->cp.push_back(0);
+  std::vector<int> piece;  // piece of every source tree, then of every destination tree
+  for (int64_t g = 0; g < d->ngroups; ++g) {
+    const int64_t s0 = d->group_src_ptr[g], ns = d->group_src_ptr[g + 1] - s0;
+    const int64_t t0 = d->group_dst_ptr[g], nt = d->group_dst_ptr[g + 1] - t0;
+    const double *U = d->coeffs + d->coeff_ptr[g];
+    piece.resize((size_t)(ns + nt));
+    std::iota(piece.begin(), piece.end(), 0);
+    auto root = [&](int x) {
+      while (piece[x] != x) x = piece[x] = piece[piece[x]];
+      return x;
+    };
+    for (int64_t i = 0; i < nt; ++i) {
+      bool used = false;
+      for (int64_t j = 0; j < ns; ++j) {
+        if (U[i * ns + j] == 0.0) continue;
+        used = true;
+        piece[root((int)(ns + i))] = root((int)j);
+      }
+      if (!used) piece[root((int)(ns + i))] = root(0);
+    }
+    int64_t made = 0;
+    for (int64_t first = 0; first < ns; ++first) {
+      // one piece per root, at its first source tree
+      const int r = root((int)first);
+      bool seen = false;
+      for (int64_t j = 0; j < first && !seen; ++j) seen = root((int)j) == r;
+      if (seen) continue;
+      std::vector<int64_t> js, is;
+      for (int64_t j = first; j < ns; ++j)
+        if (root((int)j) == r) js.push_back(j);
+      for (int64_t i = 0; i < nt; ++i)
+        if (root((int)(ns + i)) == r) is.push_back(i);
+      if (is.empty()) continue;  // a source tree that no destination uses
+      ++made;
+      o->gsp.push_back(o->gsp.back() + (int64_t)js.size());
+      o->gdp.push_back(o->gdp.back() + (int64_t)is.size());
+      o->cp.push_back(o->cp.back() + (int64_t)(js.size() * is.size()));
+      for (int64_t i : is)
+        for (int64_t j : js) o->coef.push_back(U[i * ns + j]);
+      o->sizes.insert(o->sizes.end(), d->sizes + g * N, d->sizes + (g + 1) * N);
+      for (int64_t j : js) {
+        o->sstr.insert(o->sstr.end(), d->src_strides + (s0 + j) * N, d->src_strides + (s0 + j + 1) * N);
+        o->soff.push_back(d->src_offsets[s0 + j]);
+      }
+      for (int64_t i : is) {
+        o->dstr.insert(o->dstr.end(), d->dst_strides + (t0 + i) * N, d->dst_strides + (t0 + i + 1) * N);
+        o->doff.push_back(d->dst_offsets[t0 + i]);
+      }
+    }
+    any = any || made != 1 || (int64_t)o->gsp.back() - o->gsp[o->gsp.size() - 2] != ns;
+  }
+  return any;
 }
 
 }  // namespace
@@ -488,57 +661,27 @@ extern "C" int tkb_table_create(tkb_ctx *ctx, const tkb_table_desc *d, tkb_table
         return tkb_set_error(ctx, TKB_ERR_ARG, "perm is not a permutation");
     }
   }
-  const int64_t G = d->ngroups;
+  int64_t G = d->ngroups;
   if (G > 0 && (!d->group_src_ptr || !d->group_dst_ptr || !d->coeff_ptr || !d->coeffs ||
                 (N > 0 && (!d->sizes || !d->src_strides || !d->dst_strides)) ||
                 !d->src_offsets || !d->dst_offsets))
     return tkb_set_error(ctx, TKB_ERR_ARG, "null table array");
-
-  std::vector<TGroup> hg;
-  hg.reserve(G);
-  std::vector<int64_t> hsstr, hsoff, hdstr, hdoff;
-  std::vector<int32_t> htask;  // task → group
-  std::vector<int32_t> hidx;   // task → (tile a, tile b, outer multi-index)
-  std::vector<TaskRec> hrec;   // task → tree-0 bases and extents (single-tree tables)
-  std::vector<TaskRec> hrow;   // exact row tiles (single-tree tables, every group mode 0)
-  bool all_off32 = true, all_rows = true, row_off32 = true;
-  int64_t row_pair_elems = 0;  // elements of row tasks that can be copied in 16-byte pairs
-  int64_t row_transposed = 0;  // elements of transpose groups in the row tiles
-  std::vector<double> hcoef;
-  int64_t ntasks = 0, er = 0, ew = 0;
-  size_t smem_max_f64 = 0, smem_max_c128 = 0;
-  int max_trees = 1, max_dst = 1;
-  // tile target: 2048 elements per task, smaller when the whole transform would not give
-  // every SM about four tasks (small permutes are latency-bound, not bandwidth-bound)
-  int64_t kTileElems = kTileElemsMax, kRowTileElems = kTileElemsMax;
-  {
-    int64_t total = 0;
-    for (int64_t g = 0; g < G; ++g) {
-      int64_t vol = 1;
-      for (int k = 0; k < N; ++k) vol *= std::max<int64_t>(1, d->sizes[g * N + k]);
-      total += vol * (d->group_dst_ptr[g + 1] - d->group_dst_ptr[g]);
-    }
-    while (kTileElems > 256 && total / kTileElems < (int64_t)ctx->num_sms * 4) kTileElems >>= 1;
-    // row tiles: about two per SM at least; a row task costs a fixed record fetch and one load
-    // round trip, so small transforms run faster with fewer, larger row tasks
-    while (kRowTileElems > 256 && total / kRowTileElems < (int64_t)ctx->num_sms * 2) kRowTileElems >>= 1;
-  }
-
+  int64_t er = 0, ew = 0;
   for (int64_t g = 0; g < G; ++g) {
-    const int64_t s0 = d->group_src_ptr[g], s1 = d->group_src_ptr[g + 1];
-    const int64_t t0 = d->group_dst_ptr[g], t1 = d->group_dst_ptr[g + 1];
-    const int64_t c0 = d->coeff_ptr[g], c1 = d->coeff_ptr[g + 1];
-    const int64_t nsrc = s1 - s0, ndst = t1 - t0;
-    if (nsrc <= 0 || ndst <= 0 || c1 - c0 != nsrc * ndst)
+    const int64_t nsrc = d->group_src_ptr[g + 1] - d->group_src_ptr[g];
+    const int64_t ndst = d->group_dst_ptr[g + 1] - d->group_dst_ptr[g];
+    if (nsrc <= 0 || ndst <= 0 || d->coeff_ptr[g + 1] - d->coeff_ptr[g] != nsrc * ndst)
       return tkb_set_error(ctx, TKB_ERR_ARG, "inconsistent group pointers");
-    const int64_t *sz = d->sizes + g * N;
     int64_t vol = 1;
     for (int k = 0; k < N; ++k) {
-      if (sz[k] <= 0) return tkb_set_error(ctx, TKB_ERR_SIZE, "non-positive sub-block size");
-      vol *= sz[k];
+      if (d->sizes[g * N + k] <= 0) return tkb_set_error(ctx, TKB_ERR_SIZE, "non-positive sub-block size");
+      vol *= d->sizes[g * N + k];
     }
+    er += vol * nsrc;
+    ew += vol * ndst;
     // bounds validation of every tree (prevents any out-of-range device access)
-    for (int64_t j = s0; j < s1; ++j) {
+    const int64_t *sz = d->sizes + g * N;
+    for (int64_t j = d->group_src_ptr[g]; j < d->group_src_ptr[g + 1]; ++j) {
       int64_t hi = d->src_offsets[j];
       if (hi < 0) return tkb_set_error(ctx, TKB_ERR_SIZE, "negative source offset");
       for (int k = 0; k < N; ++k) {
@@ -549,7 +692,7 @@ extern "C" int tkb_table_create(tkb_ctx *ctx, const tkb_table_desc *d, tkb_table
       if (hi >= d->src_len)
         return tkb_set_error(ctx, TKB_ERR_SIZE, "source sub-block exceeds source data length");
     }
-    for (int64_t i = t0; i < t1; ++i) {
+    for (int64_t i = d->group_dst_ptr[g]; i < d->group_dst_ptr[g + 1]; ++i) {
       int64_t hi = d->dst_offsets[i];
       if (hi < 0) return tkb_set_error(ctx, TKB_ERR_SIZE, "negative destination offset");
       for (int k = 0; k < N; ++k) {
@@ -561,8 +704,69 @@ extern "C" int tkb_table_create(tkb_ctx *ctx, const tkb_table_desc *d, tkb_table
         return tkb_set_error(ctx, TKB_ERR_SIZE,
                              "destination sub-block exceeds destination data length");
     }
-    er += vol * nsrc;
-    ew += vol * ndst;
+  }
+  SplitTable pieces;
+  tkb_table_desc pd = *d;
+  if (split_groups(d, &pieces)) {
+    pd.ngroups = (int64_t)pieces.gsp.size() - 1;
+    pd.group_src_ptr = pieces.gsp.data();
+    pd.group_dst_ptr = pieces.gdp.data();
+    pd.coeff_ptr = pieces.cp.data();
+    pd.coeffs = pieces.coef.data();
+    pd.sizes = pieces.sizes.data();
+    pd.src_strides = pieces.sstr.data();
+    pd.src_offsets = pieces.soff.data();
+    pd.dst_strides = pieces.dstr.data();
+    pd.dst_offsets = pieces.doff.data();
+    d = &pd;
+    G = pd.ngroups;
+  }
+
+  std::vector<TGroup> hg;
+  hg.reserve(G);
+  std::vector<int64_t> hsstr, hsoff, hdstr, hdoff;
+  std::vector<int32_t> htask;  // task → group
+  std::vector<int32_t> hidx;   // task → (tile a, tile b, outer multi-index)
+  std::vector<TaskRec> hrec;   // task → tree-0 bases and extents (single-tree tables)
+  std::vector<TaskRec> hrow;   // exact row tiles (single-tree tables, every group mode 0)
+  bool all_off32 = true, all_rows = true, row_off32 = true;
+  int64_t row_pair_elems = 0;  // elements of row tasks that can be copied in 16-byte pairs
+  int64_t row_transposed = 0;  // elements of transpose groups in the row tiles
+  std::vector<int64_t> hmulti;        // records of the register recoupling kernel, back to back
+  std::vector<size_t> hmulti_at;      // first word of every record
+  bool all_multi = true, several = false;  // several: some group has more than one tree on a side
+  for (int64_t g = 0; g < G && !several; ++g) several = d->coeff_ptr[g + 1] - d->coeff_ptr[g] > 1;
+  int64_t multi_transposed = 0;       // elements of its boxes whose sides have different fastest dims
+  int multi_words = 0, multi_trees = 1;
+  std::vector<double> hcoef;
+  int64_t ntasks = 0;
+  size_t smem_max_f64 = 0, smem_max_c128 = 0;
+  int max_trees = 1, max_dst = 1;
+  // tile target: 2048 elements per task, smaller when the whole transform would not give
+  // every SM about four tasks (small permutes are latency-bound, not bandwidth-bound)
+  int64_t kTileElems = kTileElemsMax, kRowTileElems = kTileElemsMax, kMultiElems = kMultiTile;
+  {
+    int64_t total = 0;
+    for (int64_t g = 0; g < G; ++g) {
+      int64_t vol = 1;
+      for (int k = 0; k < N; ++k) vol *= std::max<int64_t>(1, d->sizes[g * N + k]);
+      total += vol * (d->group_dst_ptr[g + 1] - d->group_dst_ptr[g]);
+    }
+    while (kTileElems > 256 && total / kTileElems < (int64_t)ctx->num_sms * 4) kTileElems >>= 1;
+    // row tiles: about two per SM at least; a row task costs a fixed record fetch and one load
+    // round trip, so small transforms run faster with fewer, larger row tasks
+    while (kRowTileElems > 256 && total / kRowTileElems < (int64_t)ctx->num_sms * 2) kRowTileElems >>= 1;
+    while (kMultiElems > 256 && total / kMultiElems < (int64_t)ctx->num_sms * 4) kMultiElems >>= 1;
+  }
+
+  for (int64_t g = 0; g < G; ++g) {
+    const int64_t s0 = d->group_src_ptr[g], s1 = d->group_src_ptr[g + 1];
+    const int64_t t0 = d->group_dst_ptr[g], t1 = d->group_dst_ptr[g + 1];
+    const int64_t c0 = d->coeff_ptr[g], c1 = d->coeff_ptr[g + 1];
+    const int64_t nsrc = s1 - s0, ndst = t1 - t0;
+    const int64_t *sz = d->sizes + g * N;
+    int64_t vol = 1;
+    for (int k = 0; k < N; ++k) vol *= sz[k];
 
     // canonical dims in destination order: (size, src strides per tree, dst strides per tree)
     struct Dim {
@@ -785,6 +989,88 @@ extern "C" int tkb_table_create(tkb_ctx *ctx, const tkb_table_desc *d, tkb_table
     } else {
       all_rows = false;
     }
+    const int64_t rec_words = kMultiHdrWords + kMultiTreeWords * (nsrc + ndst) + nsrc * ndst;
+    if (several && all_multi && nsrc <= kMultiMaxTrees && rec_words <= kMultiMaxWords) {
+      if (fa != fs) multi_transposed += vol * nsrc;
+      multi_words = std::max<int>(multi_words, (int)rec_words);
+      multi_trees = std::max<int>(multi_trees, (int)nsrc);
+      // box dims: a = the destination's fastest, b = the source's next, c = the destination's next
+      int db3 = -1, dc3 = -1;
+      for (int k = 0; k < nd; ++k)
+        if (k != fa && (db3 < 0 || dims[k].ss[0] < dims[db3].ss[0])) db3 = k;
+      for (int k = 0; k < nd; ++k)
+        if (k != fa && k != db3 && (dc3 < 0 || dims[k].ds[0] < dims[dc3].ds[0])) dc3 = k;
+      const int64_t A = dims[fa].size, B = db3 >= 0 ? dims[db3].size : 1, Cn = dc3 >= 0 ? dims[dc3].size : 1;
+      auto even = [](int64_t len, int64_t most) {  // extent of equal tiles of at most `most`
+        const int64_t nt = (len + most - 1) / most;
+        return (len + nt - 1) / nt;
+      };
+      const int64_t xa = even(A, kMultiElems);
+      const int64_t room = std::max<int64_t>(1, kMultiElems / xa);
+      int64_t side = 1;  // b and c share the room about equally
+      while ((side + 1) * (side + 1) <= room) ++side;
+      int64_t xb = std::min<int64_t>(B, side);
+      const int64_t xc = even(Cn, std::max<int64_t>(1, room / xb));
+      xb = even(B, std::max<int64_t>(1, room / xc));
+      std::vector<int> rest;
+      int64_t nrest = 1;
+      for (int k = 0; k < nd; ++k)
+        if (k != fa && k != db3 && k != dc3) {
+          rest.push_back(k);
+          nrest *= dims[k].size;
+        }
+      // strides and in-box offsets in 32 bits
+      const int64_t lim = (int64_t)INT32_MAX;
+      auto fits = [&](const std::vector<int64_t> &sa, const std::vector<int64_t> &sb, const std::vector<int64_t> &sc,
+                      size_t t) {
+        const int64_t b = db3 >= 0 ? sb[t] : 0, c = dc3 >= 0 ? sc[t] : 0;
+        return sa[t] <= lim && b <= lim && c <= lim && (xa - 1) * sa[t] + (xb - 1) * b + (xc - 1) * c <= lim;
+      };
+      for (int64_t j = 0; j < nsrc; ++j)
+        if (!fits(dims[fa].ss, dims[db3 < 0 ? 0 : db3].ss, dims[dc3 < 0 ? 0 : dc3].ss, (size_t)j)) all_multi = false;
+      for (int64_t i = 0; i < ndst; ++i)
+        if (!fits(dims[fa].ds, dims[db3 < 0 ? 0 : db3].ds, dims[dc3 < 0 ? 0 : dc3].ds, (size_t)i)) all_multi = false;
+      for (int64_t o = 0; o < nrest && all_multi; ++o)
+        for (int64_t c0x = 0; c0x < Cn; c0x += xc)
+          for (int64_t b0x = 0; b0x < B; b0x += xb)
+            for (int64_t a0x = 0; a0x < A; a0x += xa) {
+              MultiHdr h;
+              h.na = (int32_t)std::min<int64_t>(xa, A - a0x);
+              h.nb = (int32_t)std::min<int64_t>(xb, B - b0x);
+              h.nc = (int32_t)std::min<int64_t>(xc, Cn - c0x);
+              h.n = h.na * h.nb * h.nc;
+              h.nsrc = (int32_t)nsrc;
+              h.ndst = (int32_t)ndst;
+              h.mul_a = h.na > 1 ? 0xFFFFFFFFu / (uint32_t)h.na + 1u : 0u;
+              h.mul_b = h.nb > 1 ? 0xFFFFFFFFu / (uint32_t)h.nb + 1u : 0u;
+              const size_t at = hmulti.size();
+              hmulti_at.push_back(at);
+              hmulti.resize(at + (size_t)rec_words);
+              std::memcpy(&hmulti[at], &h, sizeof(h));
+              for (int64_t t = 0; t < nsrc + ndst; ++t) {
+                const bool from = t < nsrc;
+                const size_t ti = (size_t)(from ? t : t - nsrc);
+                auto str = [&](int k) { return k < 0 ? (int64_t)0 : from ? dims[k].ss[ti] : dims[k].ds[ti]; };
+                MultiTree mt;
+                mt.base = (from ? d->src_offsets[s0 + (int64_t)ti] : d->dst_offsets[t0 + (int64_t)ti]) + a0x * str(fa) +
+                          b0x * str(db3) + c0x * str(dc3);
+                int64_t r = o;
+                for (int k : rest) {
+                  mt.base += (r % dims[k].size) * str(k);
+                  r /= dims[k].size;
+                }
+                mt.sa = (int32_t)str(fa);
+                mt.sb = (int32_t)str(db3);
+                mt.sc = (int32_t)str(dc3);
+                mt.pad = 0;
+                std::memcpy(&hmulti[at + kMultiHdrWords + (size_t)t * kMultiTreeWords], &mt, sizeof(mt));
+              }
+              std::memcpy(&hmulti[at + kMultiHdrWords + (size_t)(nsrc + ndst) * kMultiTreeWords], d->coeffs + c0,
+                          (size_t)(nsrc * ndst) * sizeof(double));
+            }
+    } else {
+      all_multi = false;
+    }
     hg.push_back(tg);
   }
   if (std::max(smem_max_f64, smem_max_c128) > ctx->smem_optin)
@@ -803,6 +1089,19 @@ extern "C" int tkb_table_create(tkb_ctx *ctx, const tkb_table_desc *d, tkb_table
   // whose leading leg has dimension 1, for example); otherwise the staged ring transposes
   if (t->single_tree && all_rows && row_off32 && row_transposed * 64 <= er) t->nrow_tasks = (int64_t)hrow.size();
   t->row_pair_elems = row_pair_elems;
+  // several trees per group, the fastest dim kept (transposed groups a small remainder, as above)
+  std::vector<int64_t> hmrec;
+  if (!t->single_tree && all_multi && multi_transposed * 64 <= er) {
+    t->nmulti_tasks = (int64_t)hmulti_at.size();
+    t->multi_words = multi_words;
+    t->multi_trees = multi_trees;
+    hmrec.assign(hmulti_at.size() * (size_t)multi_words, 0);
+    for (size_t r = 0; r < hmulti_at.size(); ++r) {
+      const size_t end = r + 1 < hmulti_at.size() ? hmulti_at[r + 1] : hmulti.size();
+      std::copy(hmulti.begin() + (int64_t)hmulti_at[r], hmulti.begin() + (int64_t)end,
+                hmrec.begin() + (int64_t)(r * (size_t)multi_words));
+    }
+  }
   t->smem_f64 = smem_max_f64;
   t->smem_c128 = smem_max_c128;
   t->src_len = d->src_len;
@@ -820,6 +1119,7 @@ extern "C" int tkb_table_create(tkb_ctx *ctx, const tkb_table_desc *d, tkb_table
   if (e == cudaSuccess && t->single_tree) e = up((void **)&t->task_rec, hrec.data(), hrec.size() * sizeof(TaskRec));
   if (e == cudaSuccess && t->nrow_tasks > 0)
     e = up((void **)&t->row_rec, hrow.data(), hrow.size() * sizeof(TaskRec));
+  if (e == cudaSuccess && t->nmulti_tasks > 0) e = up((void **)&t->multi_rec, hmrec.data(), hmrec.size() * 8);
   if (e == cudaSuccess) e = up((void **)&t->sstr, hsstr.data(), hsstr.size() * 8);
   if (e == cudaSuccess) e = up((void **)&t->soff, hsoff.data(), hsoff.size() * 8);
   if (e == cudaSuccess) e = up((void **)&t->dstr, hdstr.data(), hdstr.size() * 8);
@@ -841,6 +1141,7 @@ extern "C" int tkb_table_destroy(tkb_table *t) {
   cudaFree(t->task_idx);
   cudaFree(t->task_rec);
   cudaFree(t->row_rec);
+  cudaFree(t->multi_rec);
   cudaFree(t->sstr);
   cudaFree(t->soff);
   cudaFree(t->dstr);
@@ -857,6 +1158,34 @@ extern "C" int tkb_table_info(const tkb_table *t, int64_t *ntasks, int64_t *er, 
   if (ew) *ew = t->elems_written;
   return TKB_OK;
 }
+
+namespace {
+
+template <typename T, bool CONJ, int NS>
+int multi_launch(tkb_ctx *ctx, const tkb_table *t, T *dst, const T *src, CDbl a, CDbl b, int bz) {
+  auto k = treetransform_multi_kernel<T, CONJ, NS, sizeof(T) == 8 ? 4 : 2>;
+  const int per_sm = tkb_occupancy(ctx->device, (const void *)k, kThreads, 0);
+  if (per_sm <= 0) return tkb_set_error(ctx, TKB_ERR_CUDA, "recoupling transform: occupancy query failed");
+  const int grid = (int)std::min<int64_t>(t->nmulti_tasks, (int64_t)ctx->num_sms * per_sm);
+  TKB_CUDA_TRY(ctx, launch_pdl(k, dim3(grid), dim3(kThreads), 0, ctx->stream, t->multi_rec, t->multi_words,
+                               t->nmulti_tasks, dst, src, a, b, bz));
+  return TKB_OK;
+}
+
+template <typename T, bool CONJ>
+int multi_dispatch(tkb_ctx *ctx, const tkb_table *t, T *dst, const T *src, CDbl a, CDbl b, int bz) {
+  switch (t->multi_trees) {
+    case 1:
+    case 2: return multi_launch<T, CONJ, 2>(ctx, t, dst, src, a, b, bz);
+    case 3: return multi_launch<T, CONJ, 3>(ctx, t, dst, src, a, b, bz);
+    case 4: return multi_launch<T, CONJ, 4>(ctx, t, dst, src, a, b, bz);
+    case 5: return multi_launch<T, CONJ, 5>(ctx, t, dst, src, a, b, bz);
+    case 6: return multi_launch<T, CONJ, 6>(ctx, t, dst, src, a, b, bz);
+    default: return multi_launch<T, CONJ, 8>(ctx, t, dst, src, a, b, bz);
+  }
+}
+
+}  // namespace
 
 int tkb_transform_launch(tkb_ctx *ctx, const tkb_table *t, int dtype, void *dst,
                          const void *src, tkb_scalar alpha, tkb_scalar beta, int conj) {
@@ -935,6 +1264,17 @@ int tkb_transform_launch(tkb_ctx *ctx, const tkb_table *t, int dtype, void *dst,
     else
       TKB_CUDA_TRY(ctx, launch_pdl(kc, dim3(pgrid), dim3(kThreads), smem, ctx->stream, t->task_rec, t->ntasks,
                                    (double2 *)dst, (const double2 *)src, a, b, bz));
+    ctx->launches++;
+    TKB_CUDA_TRY(ctx, cudaGetLastError());
+    return TKB_OK;
+  }
+  if (t->nmulti_tasks > 0 && (dtype == TKB_F64 || dtype == TKB_C128) && !use_plain_transform()) {
+    if (dtype == TKB_F64 && (alpha.im != 0.0 || beta.im != 0.0))
+      return tkb_set_error(ctx, TKB_ERR_ARG, "complex scalar with real data");
+    const int rc = dtype == TKB_F64 ? multi_dispatch<double, false>(ctx, t, (double *)dst, (const double *)src, a, b, bz)
+                   : conj ? multi_dispatch<double2, true>(ctx, t, (double2 *)dst, (const double2 *)src, a, b, bz)
+                          : multi_dispatch<double2, false>(ctx, t, (double2 *)dst, (const double2 *)src, a, b, bz);
+    if (rc != TKB_OK) return rc;
     ctx->launches++;
     TKB_CUDA_TRY(ctx, cudaGetLastError());
     return TKB_OK;

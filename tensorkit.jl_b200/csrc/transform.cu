@@ -452,9 +452,11 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 && !PAIRS) ? 6 : 4)
 // the CTA's next task is fetched while the current one runs. Row decomposition by multiply-high as
 // in the row-copy kernel.
 // Permute ((1,3),(2,4)) of an SU(2) four-leg tensor (45.6 M elements, blocks of up to 5 trees, rows
-// of 8 - 30 elements): MULTI_FIGURES.
+// of 8 - 30 elements, 730 MB): 855 us staged, 197 us here (3.7 TB/s; 233 with four positions per
+// thread at 16 warps per SM instead of two at 32, 230 with one task per warp, whose boxes are too
+// small to share sectors, and 230 with the next batch's loads ahead of the stores).
 constexpr int kMultiMaxTrees = 8;     // source trees per group held in registers
-constexpr int kMultiTile = 2048;      // positions per task at most
+constexpr int kMultiTile = 4096;      // positions per task at most
 constexpr int kMultiHdrWords = 4;     // MultiHdr
 constexpr int kMultiTreeWords = 3;    // MultiTree
 constexpr int kMultiMaxWords = 248;   // a record is fetched by one word per thread
@@ -469,7 +471,7 @@ struct MultiTree {
 };
 
 template <typename T, bool CONJ, int NS, int P>
-__global__ void __launch_bounds__(kThreads, NS * P * sizeof(T) <= 96 ? 3 : 2)
+__global__ void __launch_bounds__(kThreads, NS * P * sizeof(T) <= 80 ? 4 : NS * P * sizeof(T) <= 96 ? 3 : 2)
     treetransform_multi_kernel(const int64_t *__restrict__ recs, int rec_words, int64_t ntasks,
                                T *__restrict__ dst, const T *__restrict__ src, CDbl alpha_, CDbl beta_,
                                int beta_zero) {
@@ -1163,7 +1165,7 @@ namespace {
 
 template <typename T, bool CONJ, int NS>
 int multi_launch(tkb_ctx *ctx, const tkb_table *t, T *dst, const T *src, CDbl a, CDbl b, int bz) {
-  auto k = treetransform_multi_kernel<T, CONJ, NS, sizeof(T) == 8 ? 4 : 2>;
+  auto k = treetransform_multi_kernel<T, CONJ, NS, sizeof(T) == 8 ? 2 : 1>;
   const int per_sm = tkb_occupancy(ctx->device, (const void *)k, kThreads, 0);
   if (per_sm <= 0) return tkb_set_error(ctx, TKB_ERR_CUDA, "recoupling transform: occupancy query failed");
   const int grid = (int)std::min<int64_t>(t->nmulti_tasks, (int64_t)ctx->num_sms * per_sm);

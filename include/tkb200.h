@@ -220,6 +220,13 @@ int tkb_reduce_noalloc(int device, void *stream, int kind, int dtype, const void
                        const int64_t *count, const int64_t *stride, const double *weight,
                        double *host_out);
 
+/* ---- vector-space operations ------------------------------------------------------------
+ * dst = β·dst + α·src over n elements of two data vectors of one space (add!, and scale! with
+ * src = dst and β = 0; src/tensors/vectorinterface.jl:60-99): same storage layout, so no
+ * table. dst and src are equal or do not overlap; with β = 0 dst is not read. */
+int tkb_axpby(tkb_ctx *ctx, int dtype, int64_t n, void *dst, const void *src, tkb_scalar alpha,
+              tkb_scalar beta);
+
 /* ---- CUDA graph capture of a sequence of calls on the context stream ---------------- */
 int tkb_graph_begin(tkb_ctx *ctx);
 int tkb_graph_end(tkb_ctx *ctx, tkb_graph **out);

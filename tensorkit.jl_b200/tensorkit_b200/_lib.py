@@ -30,7 +30,7 @@ EXPORTS = [
     "tkb_trace_table_destroy", "tkb_tracetransform", "tkb_gemm_plan_create", "tkb_gemm_plan_create_tuned",
     "tkb_gemm_plan_destroy", "tkb_gemm_plan_info", "tkb_gemm_plan_slices", "tkb_grouped_gemm",
     "tkb_rplan_create",
-    "tkb_rplan_destroy", "tkb_reduce", "tkb_reduce_async", "tkb_reduce_noalloc",
+    "tkb_rplan_destroy", "tkb_reduce", "tkb_reduce_async", "tkb_reduce_noalloc", "tkb_axpby",
     "tkb_graph_begin", "tkb_graph_end",
     "tkb_graph_launch", "tkb_graph_destroy",
 ]
@@ -116,6 +116,7 @@ def _declare(lib):
         "tkb_reduce_async": ([vp, vp, C.c_int, C.c_int, vp, vp, vp], C.c_int),
         "tkb_reduce_noalloc": ([C.c_int, vp, C.c_int, C.c_int, vp, vp, i64, i64, vp, vp, vp, vp,
                                 P(dbl)], C.c_int),
+        "tkb_axpby": ([vp, C.c_int, i64, vp, vp, tkb_scalar, tkb_scalar], C.c_int),
         "tkb_graph_begin": ([vp], C.c_int),
         "tkb_graph_end": ([vp, P(vp)], C.c_int),
         "tkb_graph_launch": ([vp, vp], C.c_int),

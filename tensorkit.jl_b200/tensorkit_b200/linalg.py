@@ -237,15 +237,31 @@ def tr(t):
     return float(r[0])
 
 
+def _axpby(ty: TensorMap, tx: TensorMap, alpha, beta):
+    """ty = β·ty + α·tx on the data vectors (one space: one storage layout); tx may be ty."""
+    _check_device(ty, tx)
+    if ty.data.dtype != tx.data.dtype:
+        raise TypeError("source and destination must share their scalar type")
+    code = dtype_code(ty.data)
+    ctx = get_context(ty.data.device.index)
+    _sync_in(ctx)
+    L.check(ctx.lib.tkb_axpby(ctx.handle, code, ty.data.numel(), C.c_void_p(ty.data.data_ptr()),
+                              C.c_void_p(tx.data.data_ptr()), _scalar(alpha), _scalar(beta)), ctx.handle)
+    _sync_out(ctx, ty)
+    return ty
+
+
 def scale_(t: TensorMap, alpha):
-    """t = α·t: an identity-permutation transform of a copy with β = 0."""
-    tmp = TensorMap(t.data.clone(), t.space)
-    return add_(t, tmp, alpha, 0.0)
+    """t = α·t in place."""
+    return _axpby(t, t, alpha, 0.0)
 
 
 def add_(ty: TensorMap, tx, alpha=1.0, beta=1.0):
-    """ty = β·ty + α·tx (TensorKit add!, src/tensors/vectorinterface.jl:93-99)."""
+    """ty = β·ty + α·tx (TensorKit add!, src/tensors/vectorinterface.jl:93-99). A lazy adjoint is
+    stored transposed, so it goes through the identity permutation."""
     if ty.space != tx.space:
         raise SpaceMismatch(f"{ty.space} ≠ {tx.space}")
+    if isinstance(tx, TensorMap):
+        return _axpby(ty, tx, alpha, beta)
     p = (tx.codomainind(), tx.domainind())
     return permute_(ty, tx, p, alpha, beta)

@@ -71,9 +71,16 @@ int tkb_ctx_create(int device, void *stream, size_t workspace_bytes, tkb_ctx **o
     delete ctx;
     return tkb_set_error(nullptr, TKB_ERR_OOM, "counter allocation failed");
   }
+  e = cudaHostAlloc((void **)&ctx->host_res, kHostSlots * 2 * sizeof(double), cudaHostAllocMapped | cudaHostAllocPortable);
+  if (e != cudaSuccess) {
+    cudaFree(ctx->counters);
+    delete ctx;
+    return tkb_set_error(nullptr, TKB_ERR_OOM, "result buffer allocation failed");
+  }
   const size_t ws = std::max<size_t>(workspace_bytes, 1 << 20);
   if (tkb_ensure_workspace(ctx, ws) != TKB_OK) {
     cudaFree(ctx->counters);
+    cudaFreeHost(ctx->host_res);
     delete ctx;
     return tkb_set_error(nullptr, TKB_ERR_OOM, "workspace allocation failed");
   }
@@ -86,6 +93,7 @@ int tkb_ctx_destroy(tkb_ctx *ctx) {
   cudaStreamSynchronize(ctx->stream);
   cudaFree(ctx->ws);
   cudaFree(ctx->counters);
+  cudaFreeHost(ctx->host_res);
   delete ctx;
   return TKB_OK;
 }
@@ -402,13 +410,37 @@ int tkb_reduce(tkb_ctx *ctx, const tkb_rplan *p, int kind, int dtype, const void
                const void *y, double *host_out) {
   if (!host_out) return tkb_set_error(ctx, TKB_ERR_ARG, "null output");
   if (!ctx) return tkb_set_error(nullptr, TKB_ERR_ARG, "null context");
-  // the last 32 bytes of the counter block hold the device-side result
-  double *dres = reinterpret_cast<double *>(ctx->counters + 32);
-  int rc = tkb_reduce_async(ctx, p, kind, dtype, x, y, dres);
-  if (rc != TKB_OK) return rc;
-  TKB_CUDA_TRY(ctx, cudaMemcpyAsync(host_out, dres, 2 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  TKB_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-  return TKB_OK;
+  // the kernel writes the result straight to host memory, in a slot that this call holds until it
+  // has read it (calls from several host threads overlap)
+  int slot = -1;
+  uint64_t busy = ctx->host_busy.load();
+  while (~busy != 0) {
+    const int free = __builtin_ctzll(~busy);
+    if (ctx->host_busy.compare_exchange_weak(busy, busy | (1ull << free))) {
+      slot = free;
+      break;
+    }
+  }
+  if (slot < 0) {  // every slot is held: through device memory (the last 32 bytes of the counters) and a copy
+    double *dres = reinterpret_cast<double *>(ctx->counters + 32);
+    const int rc = tkb_reduce_async(ctx, p, kind, dtype, x, y, dres);
+    if (rc != TKB_OK) return rc;
+    TKB_CUDA_TRY(ctx, cudaMemcpyAsync(host_out, dres, 2 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    TKB_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+    return TKB_OK;
+  }
+  double *res = ctx->host_res + 2 * slot;
+  int rc = tkb_reduce_async(ctx, p, kind, dtype, x, y, res);
+  if (rc == TKB_OK) {
+    const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+    if (e != cudaSuccess) rc = tkb_set_error(ctx, TKB_ERR_CUDA, std::string("reduction: ") + cudaGetErrorString(e));
+  }
+  if (rc == TKB_OK) {
+    host_out[0] = res[0];
+    host_out[1] = res[1];
+  }
+  ctx->host_busy.fetch_and(~(1ull << slot));
+  return rc;
 }
 
 // ---- graphs ----------------------------------------------------------------------------

@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
 #include <string>
@@ -19,6 +20,10 @@ struct tkb_ctx {
   size_t ws_bytes = 0;
   // device work-queue counters for persistent kernels (zeroed once, self-resetting)
   int *counters = nullptr;
+  // host memory that reductions write their results to (mapped; kHostSlots results of two
+  // doubles), and the bit mask of the slots that calls in progress hold
+  double *host_res = nullptr;
+  std::atomic<uint64_t> host_busy{0};
   int64_t launches = 0;
   std::string err;
   cudaGraph_t capturing = nullptr;
@@ -52,6 +57,9 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
+
+constexpr int kHostSlots = 64;
+constexpr int kReduceSlot = 12;  // ctx->counters: CTAs of a reduction that have arrived
 
 // status helpers ------------------------------------------------------------------------
 int tkb_set_error(tkb_ctx *ctx, int code, const std::string &msg);

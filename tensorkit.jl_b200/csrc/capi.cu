@@ -218,7 +218,7 @@ static int plan_create(tkb_ctx *ctx, const tkb_gemm_desc *d, const tkb_gemm_tuni
   p->lenA = d->lenA;
   p->lenB = d->lenB;
   p->lenC = d->lenC;
-  std::vector<GTile> tiles, sk;
+  std::vector<GTile> sk;
   double flops = 0;
   for (int64_t i = 0; i < nb; ++i) {
     GBlock b;
@@ -250,25 +250,16 @@ static int plan_create(tkb_ctx *ctx, const tkb_gemm_desc *d, const tkb_gemm_tuni
     if (b.skinny && b.m > 0 && b.n > 0) p->sk_dim = std::max<int>(p->sk_dim, (int)std::max(b.n, b.k));
     p->hblocks.push_back(b);
     if (b.m > 0 && b.n > 0) {
-      if (b.skinny) {
+      if (b.skinny)
         for (int64_t m0 = 0; m0 < b.m; m0 += kSkinnyTaskRows)
           sk.push_back({(int32_t)i, (int32_t)m0, 0, b.k > 0 ? 0 : 1});
-      } else {
-        for (int64_t m0 = 0; m0 < b.m; m0 += 64)
-          for (int64_t n0 = 0; n0 < b.n; n0 += 64)
-            tiles.push_back({(int32_t)i, (int32_t)m0, (int32_t)n0, b.k > 0 ? 0 : 1});
-      }
     }
   }
   p->nsk = (int64_t)sk.size();
-  std::stable_sort(tiles.begin(), tiles.end(), [&](const GTile &x, const GTile &y) {
-    return p->hblocks[x.block].k > p->hblocks[y.block].k;
-  });
   p->flops = flops;
-  p->ntiles = (int64_t)tiles.size();
   int rc = TKB_OK;
   if (d->precision == TKB_SPLIT_INT8) rc = tkb_gemm_split_prepare(ctx, p);
-  else rc = tkb_gemm_plain_prepare(ctx, p, tiles);
+  else rc = tkb_gemm_plain_prepare(ctx, p);
   if (rc != TKB_OK) {
     tkb_gemm_plan_destroy(p);
     return rc;
@@ -278,10 +269,6 @@ static int plan_create(tkb_ctx *ctx, const tkb_gemm_desc *d, const tkb_gemm_tuni
     e = cudaMalloc((void **)&p->blocks, p->hblocks.size() * sizeof(GBlock));
     if (e == cudaSuccess)
       e = cudaMemcpy(p->blocks, p->hblocks.data(), p->hblocks.size() * sizeof(GBlock), cudaMemcpyHostToDevice);
-  }
-  if (e == cudaSuccess && !tiles.empty()) {
-    e = cudaMalloc((void **)&p->tiles, tiles.size() * sizeof(GTile));
-    if (e == cudaSuccess) e = cudaMemcpy(p->tiles, tiles.data(), tiles.size() * sizeof(GTile), cudaMemcpyHostToDevice);
   }
   if (e == cudaSuccess && !sk.empty()) {
     e = cudaMalloc((void **)&p->sktasks, sk.size() * sizeof(GTile));
@@ -298,9 +285,9 @@ static int plan_create(tkb_ctx *ctx, const tkb_gemm_desc *d, const tkb_gemm_tuni
 int tkb_gemm_plan_destroy(tkb_plan *p) {
   if (!p) return TKB_OK;
   cudaFree(p->blocks);
-  cudaFree(p->tiles);
   cudaFree(p->sktasks);
   cudaFree(p->ptasks);
+  cudaFree(p->pstart);
   cudaFree(p->bstat);
   cudaFree(p->bslices);
   cudaFree(p->kstiles);

@@ -5,24 +5,27 @@
 // f64 kind, so the double-precision tensor pipe is reached through DMMA; the split-precision
 // path (gemm_split.cu) is the tcgen05 one.
 //
-// Work decomposition: 64×64 output tiles; when the tiles would leave resident CTA slots idle,
-// the K loops of the longest tiles are cut into pieces (split K) so that the pieces fill about
-// one wave. Tasks (tile, K range) are sorted by decreasing length and dealt round-robin to the
-// CTAs of the launch (a static, cost-ordered queue: no atomics to claim work). A piece of a split
-// tile stores its FP64 partial tile; the piece that arrives last on the tile's counter adds all
-// partials in piece order (deterministic, no piece waits for another) and applies α, β.
+// Work decomposition (tkb_gemm_plain_prepare): 64×64 output tiles (32×32 where those would leave most
+// of the chip idle), whose K loops are cut into pieces (split K) where that evens out the CTAs'
+// shares. Every CTA has a fixed list of tasks (tile, K range). A piece of a split tile stores its
+// FP64 partial tile; the piece that arrives last on the tile's counter adds all partials in piece
+// order (deterministic, no piece waits for another) and applies α, β.
 //
-// Real CTA: 4 warps in a 2×2 grid (each 32×32 = 2×4 m16n8k8 tiles, two accumulator sets: one
-// per K sub-step of 8), BK = 16, a three-stage cp.async ring (two stages in flight while one is
-// consumed; one barrier per K step; a stage's DMMA are issued before the refill copies).
-// Operand tiles are copied in 16-byte pairs when the block's layout keeps pairs aligned (op N,
-// even offsets and leading dimensions, 16-byte aligned base), else in 8-byte elements; elements
-// outside the block are zero-filled, so any lda/offset parity works. Complex blocks copy whole
-// 16-byte elements and issue four real DMMA per fragment pair.
+// Real CTA: 4 warps in a 2×2 grid, m16n8k8 tiles, BK = 16, a three-stage cp.async ring (two stages in
+// flight while one is consumed; one barrier per K step; a stage's DMMA are issued before the refill
+// copies). The ring runs through all tasks of the CTA without a break: the next tile's first stages
+// arrive while the last one's values are stored. Operand tiles are copied in 16-byte pairs when the
+// block's layout keeps pairs aligned (op N, even offsets and leading dimensions, 16-byte aligned base),
+// else in 8-byte elements; elements outside the block are zero-filled, so any lda/offset parity
+// works. Complex blocks copy whole 16-byte elements and issue four real DMMA per fragment pair.
 //
-// What bounds it: the DMMA pipe runs m16n8k8 at 64 cycles per SM sub-partition (37 TFLOP/s
-// measured on B200); the per-thread cp.async copies of a 16 KB stage cost the SM about a third
-// of that again (per-instruction load/store-unit work), so large blocks reach about 30 TFLOP/s.
+// What bounds it: the DMMA pipe runs m16n8k8 at 64 cycles per SM sub-partition (37 TFLOP/s measured on
+// B200), and every instruction issued beside it costs: with addresses and bounds resolved once per
+// task one 4096³ block runs at 33.5 TFLOP/s (30.1 when each copy worked out its own address), one
+// 4095³ block (8-byte copies) at 33.0 (26.8). The epilogue keeps one pointer per column of a thread:
+// 9 blocks of K ≤ 256 and a 59 MB output take 152 us (176 with an address per element, 37 us of it in
+// the epilogues). Taken back: fragments of the next sub-step loaded ahead of the DMMA (517 instead of
+// 489 us on a U(1) effective Hamiltonian; the DMMA wait for the loads issued before them).
 #include <algorithm>
 #include <cstring>
 
@@ -33,7 +36,7 @@ namespace {
 constexpr int BM = 64, BN = 64, BK = 16, NST = 3;
 constexpr int APAD = 4, BPAD = 4;      // real: keeps 16-byte row alignment, spreads banks
 constexpr int CAPAD = 2, CBPAD = 2;    // complex (16-byte elements)
-constexpr int kRealThreads = 128, kCplxThreads = 256;
+constexpr int kCplxThreads = 256;
 
 struct CDbl {
   double x, y;
@@ -98,74 +101,103 @@ __device__ __forceinline__ void dmma16(double (&c)[4], const double (&a)[4], con
 }
 
 // ---- real ----------------------------------------------------------------------------
-struct SmemR {
-  double A[NST][BK][BM + APAD];  // op(A) tile, [k][row]
-  double B[NST][BN][BK + BPAD];  // op(B) tile, [col][k]
+// Tile shape of a real kernel: BMxBN output tile, warps of WMxWN (m16n8k8 fragments)
+template <int BM_, int BN_, int WM_, int WN_, int NST_, int MINB_>
+struct RealCfg {
+  static constexpr int BM = BM_, BN = BN_, WM = WM_, WN = WN_, NST = NST_, MINB = MINB_;
+  static constexpr int WARPS_M = BM / WM, WARPS = (BM / WM) * (BN / WN), THREADS = 32 * WARPS;
+  static constexpr int MI = WM / 16, NI = WN / 8, NV = MI * NI * 4;
+  static constexpr int PA = BM + APAD, PB = BK + BPAD;  // pitches: op(A) tile [k][row], op(B) tile [col][k]
+  static constexpr int A_ELEMS = BK * PA, B_ELEMS = BN * PB, STAGE = A_ELEMS + B_ELEMS;
+  static constexpr size_t SMEM = (size_t)NST * STAGE * sizeof(double);
 };
 
-// vec: bit 0 = A tiles as 16-byte pairs, bit 1 = B tiles as 16-byte pairs
-__device__ __forceinline__ void load_tiles_r(SmemR &s, int st, const GBlock &b, const double *A,
-                                             const double *B, int64_t m0, int64_t n0, int64_t k0, int vec) {
-  const int tid = threadIdx.x;
-  if (vec & 1) {  // op N, pairs of rows: 32 pairs × BK columns
+// Copies of one operand's tiles, resolved once per task: the thread's first source element, the
+// step to its next copies of a stage and to the next stage. Copies of rows (columns) outside the block read
+// nothing and fill zeros; so do K positions beyond the block. Tiles inside the block on both counts
+// take a path without the tests: one address step and one copy per element (or pair), the place
+// in the stage an immediate offset. Instruction issue, not the copies' latency, is what a stage
+// costs besides its DMMA.
+//   kind 0: the tile's outer index (rows of op(A), columns of op(B)) is contiguous in memory
+//   kind 1: K is contiguous
+//   kind 2: 16-byte pairs along the contiguous direction that the stage keeps contiguous too
+template <int T, int OUTER, bool IS_A, int PITCH>
+struct TileCopy {
+  const double *p, *base;  // base: the operand's first element (where copies that read nothing point)
+  int64_t dr, dk;    // elements: between the copies of a stage, between stages
+  int kind, o, ext;  // outer position of the first copy in the block, the block's extent (clamped)
+  int l0, s0;        // K position and stage offset of the first copy
+  bool inside;       // the whole tile lies inside the block
+
+  // thread layout of a kind: first (outer, K) position and the steps between its copies
+  template <int KIND>
+  struct Lay {
+    static constexpr int COPIES = KIND == 2 ? OUTER * BK / (2 * T) : OUTER * BK / T;
+    static constexpr bool ALONG_K = KIND == 2 ? !IS_A : KIND == 1;  // neighbouring threads step along K
+    static constexpr int W = KIND == 2 ? 2 : 1;
+    static constexpr int LINE = (ALONG_K ? BK : OUTER) / W;         // threads per contiguous run
+    static constexpr int DO = ALONG_K ? T / LINE : 0, DL = ALONG_K ? 0 : T / LINE;
+    static constexpr int DS = IS_A ? DL * PITCH + DO : DO * PITCH + DL;
+    static_assert(T % LINE == 0, "whole runs per pass");
+  };
+  template <int KIND>
+  __device__ __forceinline__ void init_kind(int64_t so, int64_t sk, int64_t o0, int64_t kbeg) {
+    using L = Lay<KIND>;
+    const int a = (threadIdx.x % L::LINE) * L::W, b = threadIdx.x / L::LINE;
+    const int oo = L::ALONG_K ? b : a;
+    l0 = L::ALONG_K ? a : b;
+    p = base + (o0 + oo) * so + (kbeg + l0) * sk;
+    dr = L::DO * so + L::DL * sk;
+    s0 = IS_A ? l0 * PITCH + oo : oo * PITCH + l0;
+    o = oo;
+  }
+  __device__ __forceinline__ void init(const double *X, int64_t off, int64_t ld, bool outer_contig, int64_t o0,
+                                       int64_t extent, int64_t kbeg, bool pairs) {
+    const int64_t so = outer_contig ? 1 : ld, sk = outer_contig ? ld : 1;
+    base = X + off;
+    dk = BK * sk;
+    const int64_t rest = extent - o0;  // outer positions from the tile's first on
+    inside = rest >= OUTER;
+    ext = inside ? OUTER : (int)rest;
+    kind = pairs && outer_contig == IS_A ? 2 : outer_contig ? 0 : 1;
+    if (kind == 0) init_kind<0>(so, sk, o0, kbeg);
+    else if (kind == 1) init_kind<1>(so, sk, o0, kbeg);
+    else init_kind<2>(so, sk, o0, kbeg);
+  }
+  template <int KIND>
+  __device__ __forceinline__ void issue_kind(double *stage, int64_t left) {
+    using L = Lay<KIND>;
+    double *d = stage + s0;
+    const double *q = p;
+    if (inside && left >= BK) {
 #pragma unroll
-    for (int r = 0; r < (BM * BK) / (2 * kRealThreads); ++r) {
-      const int e = tid + r * kRealThreads;
-      const int i2 = e % (BM / 2), l = e / (BM / 2);
-      const int64_t gi = m0 + 2 * i2, gl = k0 + l;
-      const int bytes = (gl < b.k && gi < b.m) ? (gi + 1 < b.m ? 16 : 8) : 0;
-      const double *p = A + b.offA + (bytes ? gi + gl * b.lda : 0);
-      cp_async16(&s.A[st][l][2 * i2], p, bytes);
-    }
-  } else if (b.opA == TKB_OP_N) {
+      for (int r = 0; r < L::COPIES; ++r, q += dr) {
+        if constexpr (KIND == 2) cp_async16(d + r * L::DS, q, 16);
+        else cp_async8(d + r * L::DS, q, true);
+      }
+    } else {
 #pragma unroll
-    for (int r = 0; r < (BM * BK) / kRealThreads; ++r) {
-      const int e = tid + r * kRealThreads;
-      const int i = e % BM, l = e / BM;
-      const int64_t gi = m0 + i, gl = k0 + l;
-      const bool ok = gi < b.m && gl < b.k;
-      cp_async8(&s.A[st][l][i], A + b.offA + (ok ? gi + gl * b.lda : 0), ok);
-    }
-  } else {
-#pragma unroll
-    for (int r = 0; r < (BM * BK) / kRealThreads; ++r) {
-      const int e = tid + r * kRealThreads;
-      const int l = e % BK, i = e / BK;
-      const int64_t gi = m0 + i, gl = k0 + l;
-      const bool ok = gi < b.m && gl < b.k;
-      cp_async8(&s.A[st][l][i], A + b.offA + (ok ? gl + gi * b.lda : 0), ok);
+      for (int r = 0; r < L::COPIES; ++r, q += dr) {
+        const int oo = o + r * L::DO, l = l0 + r * L::DL;
+        if constexpr (KIND == 2) {  // the pair's second element may lie outside
+          const bool v = oo < ext && l < left;
+          const bool w = L::ALONG_K ? l + 1 < left : oo + 1 < ext;
+          cp_async16(d + r * L::DS, v ? q : base, v ? (w ? 16 : 8) : 0);
+        } else {
+          const bool v = oo < ext && l < left;
+          cp_async8(d + r * L::DS, v ? q : base, v);
+        }
+      }
     }
   }
-  if (vec & 2) {  // op N, pairs along K: BK/2 pairs × BN columns
-#pragma unroll
-    for (int r = 0; r < (BN * BK) / (2 * kRealThreads); ++r) {
-      const int e = tid + r * kRealThreads;
-      const int l2 = e % (BK / 2), j = e / (BK / 2);
-      const int64_t gl = k0 + 2 * l2, gj = n0 + j;
-      const int bytes = (gj < b.n && gl < b.k) ? (gl + 1 < b.k ? 16 : 8) : 0;
-      const double *p = B + b.offB + (bytes ? gl + gj * b.ldb : 0);
-      cp_async16(&s.B[st][j][2 * l2], p, bytes);
-    }
-  } else if (b.opB == TKB_OP_N) {
-#pragma unroll
-    for (int r = 0; r < (BN * BK) / kRealThreads; ++r) {
-      const int e = tid + r * kRealThreads;
-      const int l = e % BK, j = e / BK;
-      const int64_t gl = k0 + l, gj = n0 + j;
-      const bool ok = gl < b.k && gj < b.n;
-      cp_async8(&s.B[st][j][l], B + b.offB + (ok ? gl + gj * b.ldb : 0), ok);
-    }
-  } else {
-#pragma unroll
-    for (int r = 0; r < (BN * BK) / kRealThreads; ++r) {
-      const int e = tid + r * kRealThreads;
-      const int j = e % BN, l = e / BN;
-      const int64_t gl = k0 + l, gj = n0 + j;
-      const bool ok = gl < b.k && gj < b.n;
-      cp_async8(&s.B[st][j][l], B + b.offB + (ok ? gj + gl * b.ldb : 0), ok);
-    }
+  // the copies of the next stage into `stage`; left: K positions of the block from this stage on
+  __device__ __forceinline__ void issue(double *stage, int64_t left) {
+    if (kind == 0) issue_kind<0>(stage, left);
+    else if (kind == 1) issue_kind<1>(stage, left);
+    else issue_kind<2>(stage, left);
+    p += dk;
   }
-}
+};
 
 // 16-byte pairs are usable for an operand in op N whose offset and leading dimension are even
 // (the base pointer's alignment is checked at launch)
@@ -231,96 +263,138 @@ __device__ __forceinline__ bool splitk_reduce(const PTask &t, double (&v)[NV], d
   return true;
 }
 
-__global__ void __launch_bounds__(kRealThreads, 2)
-    gemm_f64_kernel(const GBlock *__restrict__ blocks, const PTask *__restrict__ tasks, int ntasks,
-                    double *__restrict__ C, const double *__restrict__ A, const double *__restrict__ B,
-                    double alpha, double beta, double *__restrict__ part, int *__restrict__ pcnt, int base_ok) {
+template <typename CFG>
+__global__ void __launch_bounds__(CFG::THREADS, CFG::MINB)
+    gemm_f64_kernel(const GBlock *__restrict__ blocks, const PTask *__restrict__ tasks,
+                    const int32_t *__restrict__ start, double *__restrict__ C, const double *__restrict__ A,
+                    const double *__restrict__ B, double alpha, double beta, double *__restrict__ part,
+                    int *__restrict__ pcnt, int base_ok) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  SmemR &s = *reinterpret_cast<SmemR *>(smem_raw);
+  double *sm = reinterpret_cast<double *>(smem_raw);
   __shared__ int ticket;
   PL_STAMP(0);
-  pdl_wait();  // operands, output and the split-K counters belong to earlier kernels too
-  pdl_trigger();
-  PL_STAMP(1);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int wm = warp & 1, wn = warp >> 1;
+  const int wm = (warp % CFG::WARPS_M) * CFG::WM, wn = (warp / CFG::WARPS_M) * CFG::WN;
   const int g = lane >> 2, t = lane & 3;
+  const int t_begin = start[blockIdx.x], t_end = start[blockIdx.x + 1];
+  // The stages of all the CTA's tasks form one stream through the ring: the copies run NST − 1 stages
+  // ahead of the products and go on into the next task while this one finishes.
+  TileCopy<CFG::THREADS, CFG::BM, true, CFG::PA> ca;
+  TileCopy<CFG::THREADS, CFG::BN, false, CFG::PB> cb;
+  int next = t_begin, ahead = 0;  // the next task to copy, stages of the current one not yet copied
+  int64_t left = 0;               // K positions of its block from the next stage on
+  auto advance = [&]() {
+    while (ahead == 0 && next < t_end) {
+      const PTask q = tasks[next++];
+      ahead = q.kind == 0 ? q.ke - q.kb : 0;
+      if (ahead == 0) continue;
+      const GBlock &b = blocks[q.block];
+      const int vec = vec_flags(b, base_ok);
+      const int64_t k0 = (int64_t)q.kb * BK;
+      ca.init(A, b.offA, b.lda, b.opA == TKB_OP_N, q.m0, b.m, k0, vec & 1);
+      cb.init(B, b.offB, b.ldb, b.opB != TKB_OP_N, q.n0, b.n, k0, vec & 2);
+      left = b.k - k0;
+    }
+  };
+  auto produce = [&](int slot) {
+    advance();
+    if (ahead > 0) {
+      ca.issue(sm + slot * CFG::STAGE, left);
+      cb.issue(sm + slot * CFG::STAGE + CFG::A_ELEMS, left);
+      left -= BK;
+      --ahead;
+    }
+    cp_async_commit();  // one group per stage, possibly empty
+  };
+  advance();   // the task tables are static
+  pdl_wait();  // operands, output and the split-K counters belong to earlier kernels too
+  PL_STAMP(1);
+#pragma unroll
+  for (int st = 0; st < CFG::NST - 1; ++st) produce(st);
+  int slot = 0;
   [[maybe_unused]] int ntask = 0;
-  for (int ti = blockIdx.x; ti < ntasks; ti += gridDim.x, ++ntask) {
+  for (int ti = t_begin; ti < t_end; ++ti, ++ntask) {
     const PTask task = tasks[ti];
-    const GBlock b = blocks[task.block];
-    const int64_t m0 = task.m0, n0 = task.n0;
-    const int vec = vec_flags(b, base_ok);
-    // two accumulator sets, one per K sub-step of 8 in a stage (the 16 DMMA of a stage are
-    // independent); their sum is (sub-step 0) + (sub-step 8)
-    double acc[32], acc2[32];
+    double acc[CFG::NV];
 #pragma unroll
-    for (int q = 0; q < 32; ++q) acc[q] = acc2[q] = 0.0;
-    if (task.kind == 0 && task.ke > task.kb) {
-      k_loop<NST>(task.kb, task.ke,
-             [&](int st, int64_t k0) { load_tiles_r(s, st, b, A, B, m0, n0, k0, vec); },
-             [&](int st) {
-               // the warp's 32×32 as 2 × 4 blocks of 16×8 (m16n8k8), K in steps of 8
+    for (int q = 0; q < CFG::NV; ++q) acc[q] = 0.0;
+    const int nk = task.kind == 0 ? task.ke - task.kb : 0;
+    for (int kt = 0; kt < nk; ++kt) {
+      cp_async_wait<CFG::NST - 2>();
+      __syncthreads();  // this stage is visible to all; every warp is done with the slot before it
+      const double *sa = sm + slot * CFG::STAGE + wm + g, *sb = sm + slot * CFG::STAGE + CFG::A_ELEMS;
 #pragma unroll
-               for (int kk = 0; kk < BK; kk += 8) {
-                 double *ac = kk == 0 ? acc : acc2;
-                 double af[2][4], bf[4][2];
+      for (int kk = 0; kk < BK; kk += 8) {
+        double af[CFG::MI][4], bf[CFG::NI][2];
 #pragma unroll
-                 for (int mi = 0; mi < 2; ++mi) {
-                   const int r = wm * 32 + mi * 16 + g;
-                   af[mi][0] = s.A[st][kk + t][r];
-                   af[mi][1] = s.A[st][kk + t][r + 8];
-                   af[mi][2] = s.A[st][kk + t + 4][r];
-                   af[mi][3] = s.A[st][kk + t + 4][r + 8];
-                 }
+        for (int mi = 0; mi < CFG::MI; ++mi) {
+          af[mi][0] = sa[(kk + t) * CFG::PA + mi * 16];
+          af[mi][1] = sa[(kk + t) * CFG::PA + mi * 16 + 8];
+          af[mi][2] = sa[(kk + t + 4) * CFG::PA + mi * 16];
+          af[mi][3] = sa[(kk + t + 4) * CFG::PA + mi * 16 + 8];
+        }
 #pragma unroll
-                 for (int ni = 0; ni < 4; ++ni) {
-                   bf[ni][0] = s.B[st][wn * 32 + ni * 8 + g][kk + t];
-                   bf[ni][1] = s.B[st][wn * 32 + ni * 8 + g][kk + t + 4];
-                 }
+        for (int ni = 0; ni < CFG::NI; ++ni) {
+          bf[ni][0] = sb[(wn + ni * 8 + g) * CFG::PB + kk + t];
+          bf[ni][1] = sb[(wn + ni * 8 + g) * CFG::PB + kk + t + 4];
+        }
 #pragma unroll
-                 for (int mi = 0; mi < 2; ++mi)
+        for (int mi = 0; mi < CFG::MI; ++mi)
 #pragma unroll
-                   for (int ni = 0; ni < 4; ++ni)
-                     dmma16(*reinterpret_cast<double(*)[4]>(&ac[(mi * 4 + ni) * 4]), af[mi], bf[ni]);
-               }
-             });
-#pragma unroll
-      for (int q = 0; q < 32; ++q) acc[q] += acc2[q];
+          for (int ni = 0; ni < CFG::NI; ++ni)
+            dmma16(*reinterpret_cast<double(*)[4]>(&acc[(mi * CFG::NI + ni) * 4]), af[mi], bf[ni]);
+      }
+      // the refill of the slot read in the previous iteration is issued while the DMMA execute
+      produce(slot == 0 ? CFG::NST - 1 : slot - 1);
+      slot = slot + 1 == CFG::NST ? 0 : slot + 1;
     }
     if (ntask == 0) PL_STAMP(2);
-    const bool fin = splitk_reduce<32, kRealThreads>(task, acc, part, pcnt, &ticket);
+    if (ti + 1 == t_end) pdl_trigger();
+    const bool fin = splitk_reduce<CFG::NV, CFG::THREADS>(task, acc, part, pcnt, &ticket);
     if (ntask == 0) {
       PL_STAMP(3);
       PL_SET(6, 2ull * task.nsplit + (fin ? 1 : 0));
     }
     if (!fin) continue;
-    // epilogue: C = α·acc + β·C, in four row groups of 8 (the old values of a group are loaded
-    // before its first store). Row group R, value q (column block q/2, column 2t + q%2) is
-    // acc[((R/2)·4 + q/2)·4 + (R%2)·2 + q%2] (the m16n8k8 fragments)
+    const GBlock &b = blocks[task.block];
+    // epilogue: C = α·acc + β·C, column by column of the thread (column fragment q/2, column 2t + q%2);
+    // its rows are 8 apart, so one pointer per column serves them all. Row h is
+    // acc[((h/2)·NI + q/2)·4 + (h%2)·2 + q%2]
+    const int64_t i0 = task.m0 + wm + g, j0 = task.n0 + wn + 2 * t;
+    const int rows = (int)min((int64_t)CFG::WM, b.m - i0);  // valid rows from i0 on (may be ≤ 0)
+    const int cols = (int)min((int64_t)CFG::WN, b.n - j0);
+    double *pc = C + b.offC + i0 + j0 * b.ldc;
+    const int64_t ldc = b.ldc;
 #pragma unroll
-    for (int mi = 0; mi < 4; ++mi) {
-      const int64_t i = m0 + wm * 32 + mi * 8 + g;
-      double old[8];
+    for (int q = 0; q < 2 * CFG::NI; ++q) {
+      if ((q / 2) * 8 + (q % 2) >= cols) continue;
+      double *p = pc + ((q / 2) * 8 + (q % 2)) * ldc;
+      double old[2 * CFG::MI];
+      if (beta != 0.0) {
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int64_t j = n0 + wn * 32 + (q / 2) * 8 + 2 * t + (q % 2);
-        old[q] = (beta != 0.0 && i < b.m && j < b.n) ? C[b.offC + i + j * b.ldc] : 0.0;
+        for (int h = 0; h < 2 * CFG::MI; ++h) old[h] = h * 8 < rows ? p[h * 8] : 0.0;
       }
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int64_t j = n0 + wn * 32 + (q / 2) * 8 + 2 * t + (q % 2);
-        if (i < b.m && j < b.n) {
-          double r = alpha * acc[((mi >> 1) * 4 + (q >> 1)) * 4 + (mi & 1) * 2 + (q & 1)];
-          if (beta != 0.0) r = fma(beta, old[q], r);
-          C[b.offC + i + j * b.ldc] = r;
+      for (int h = 0; h < 2 * CFG::MI; ++h) {
+        if (h * 8 < rows) {
+          double r = alpha * acc[((h >> 1) * CFG::NI + (q >> 1)) * 4 + (h & 1) * 2 + (q & 1)];
+          if (beta != 0.0) r = fma(beta, old[h], r);
+          p[h * 8] = r;
         }
       }
     }
   }
+  cp_async_wait<0>();
   PL_SET(5, ntask);
   PL_STAMP(4);
 }
+
+// LargeTile: two CTAs of four 32×32 warps per SM (194 registers; three at 168 registers ran 4096³ at
+// 32.5 instead of 33.8 TFLOP/s, eight 32×16 warps at 29.7). SmallTile: six CTAs of four 16×16 warps
+// per SM, for launches whose 64×64 tiles would leave most of the chip to one CTA per SM, which spends
+// 0.87 us per K step where its DMMA take 0.52.
+using LargeTile = RealCfg<64, 64, 32, 32, 3, 2>;
+using SmallTile = RealCfg<32, 32, 16, 16, 3, 6>;
 
 // ---- complex ---------------------------------------------------------------------------
 struct SmemC {
@@ -372,8 +446,8 @@ __device__ __forceinline__ void load_tiles_c(SmemC &s, int st, const GBlock &b, 
 }
 
 __global__ void __launch_bounds__(kCplxThreads, 2)
-    gemm_c128_kernel(const GBlock *__restrict__ blocks, const PTask *__restrict__ tasks, int ntasks,
-                     double2 *__restrict__ C, const double2 *__restrict__ A, const double2 *__restrict__ B,
+    gemm_c128_kernel(const GBlock *__restrict__ blocks, const PTask *__restrict__ tasks,
+                     const int32_t *__restrict__ start, double2 *__restrict__ C, const double2 *__restrict__ A, const double2 *__restrict__ B,
                      CDbl alpha, CDbl beta, double *__restrict__ part, int *__restrict__ pcnt) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SmemC &s = *reinterpret_cast<SmemC *>(smem_raw);
@@ -384,7 +458,8 @@ __global__ void __launch_bounds__(kCplxThreads, 2)
   const int wm = warp & 1, wn = warp >> 1;                      // warp tile 32 x 16
   const int g = lane >> 2, t = lane & 3;
   const bool bz = beta.x == 0.0 && beta.y == 0.0;
-  for (int ti = blockIdx.x; ti < ntasks; ti += gridDim.x) {
+  const int t_end = start[blockIdx.x + 1];
+  for (int ti = start[blockIdx.x]; ti < t_end; ++ti) {
     const PTask task = tasks[ti];
     const GBlock b = blocks[task.block];
     // conjugation of an operand flips the sign of its imaginary part
@@ -646,14 +721,47 @@ int tkb_gemm_skinny_launch(tkb_ctx *ctx, const tkb_plan *p, void *C, const void 
   return TKB_OK;
 }
 
-int tkb_gemm_plain_prepare(tkb_ctx *ctx, tkb_plan *p, const std::vector<GTile> &tiles) {
+// Work decomposition of a plain GEMM: the tile shape and the tasks of every CTA.
+// - SmallTile runs while its tiles are at most 1.5 per SM: an SU(2) environment update (two products and
+// two permutes) takes 10.3 instead of 14.4 us at V dim 280, 15.9 instead of 22.8 at 870, 22.7
+// instead of 26.7 at 1816 (155 tiles), but 34.9 instead of 32.8 at 2410 (290 tiles).
+// - Fewer tiles than resident CTAs: the K loops of the longest tiles are cut into equal pieces of the
+//   shortest length (at least min_piece_steps K steps) whose count still fits, one task per CTA.
+// - Otherwise every CTA gets an equal share of all K steps (plus kTileCost steps per tile for its
+//   epilogue), as a contiguous range of the tiles in order of falling K; a tile that a share ends in
+//   is cut there. Whole tiles alone leave CTAs idle for up to a tile each: on a U(1) effective
+//   Hamiltonian's second product (394 tiles of up to 109 steps for 296 CTAs) SMs were active for
+//   70 % of the launch. A CTA runs its cut tiles first, so their partial sums meet while it goes on.
+constexpr int kTileCost = 2;
+
+int tkb_gemm_plain_prepare(tkb_ctx *ctx, tkb_plan *p) {
   const bool cplx = p->dtype == TKB_C128;
-  const void *kfn = cplx ? (const void *)gemm_c128_kernel : (const void *)gemm_f64_kernel;
-  const int threads = cplx ? kCplxThreads : kRealThreads;
-  const size_t smem = cplx ? sizeof(SmemC) : sizeof(SmemR);
+  int64_t small_tiles = 0;
+  for (const GBlock &b : p->hblocks)
+    if (!b.skinny) small_tiles += ((b.m + 31) / 32) * ((b.n + 31) / 32);
+  const bool small = !cplx && small_tiles * 2 <= (int64_t)ctx->num_sms * 3;
+  p->tile_m = p->tile_n = small ? SmallTile::BM : BM;
+  const void *kfn = cplx    ? (const void *)gemm_c128_kernel
+                    : small ? (const void *)gemm_f64_kernel<SmallTile>
+                            : (const void *)gemm_f64_kernel<LargeTile>;
+  const int threads = cplx ? kCplxThreads : small ? SmallTile::THREADS : LargeTile::THREADS;
+  const size_t smem = cplx ? sizeof(SmemC) : small ? SmallTile::SMEM : LargeTile::SMEM;
+  const int tm = p->tile_m, tn = p->tile_n;
+  // a piece's partial sums cost as much as twice as many steps of the smaller tile
+  const int min_steps = p->min_piece_steps * (small ? 2 : 1);
   const int per_sm = tkb_occupancy(ctx->device, kfn, threads, smem);
   if (per_sm <= 0) return tkb_set_error(ctx, TKB_ERR_CUDA, "plain GEMM: occupancy query failed");
   const int64_t slots = (int64_t)ctx->num_sms * per_sm;
+  std::vector<GTile> tiles;
+  for (size_t i = 0; i < p->hblocks.size(); ++i) {
+    const GBlock &b = p->hblocks[i];
+    if (b.skinny) continue;
+    for (int64_t m0 = 0; m0 < b.m; m0 += tm)
+      for (int64_t n0 = 0; n0 < b.n; n0 += tn)
+        tiles.push_back({(int32_t)i, (int32_t)m0, (int32_t)n0, b.k > 0 ? 0 : 1});
+  }
+  std::stable_sort(tiles.begin(), tiles.end(),
+                   [&](const GTile &x, const GTile &y) { return p->hblocks[x.block].k > p->hblocks[y.block].k; });
   const int64_t nt = (int64_t)tiles.size();
   int64_t total = 0, maxnk = 1;
   std::vector<int64_t> nks(nt);
@@ -663,46 +771,102 @@ int tkb_gemm_plain_prepare(tkb_ctx *ctx, tkb_plan *p, const std::vector<GTile> &
     total += nks[i];
     maxnk = std::max(maxnk, nks[i]);
   }
-  auto pieces = [&](int64_t nk, int64_t target) {
-    return (int)std::min<int64_t>(p->max_pieces, std::max<int64_t>(1, (nk + target - 1) / target));
-  };
-  // the shortest piece length (at least min_piece_steps) whose tasks still fit the resident slots
-  int64_t target = maxnk;
+  std::vector<std::vector<PTask>> lists;  // per CTA
+  int nslots = 0, npart = 0;
   if (nt < slots) {
-    target = std::max<int64_t>(p->min_piece_steps, (total + slots - 1) / slots);
+    auto pieces = [&](int64_t nk, int64_t target) {
+      return (int)std::min<int64_t>(p->max_pieces, std::max<int64_t>(1, (nk + target - 1) / target));
+    };
+    int64_t target = std::max<int64_t>(min_steps, (total + slots - 1) / slots);
     for (; target < maxnk; ++target) {
       int64_t cnt = 0;
       for (int64_t i = 0; i < nt; ++i) cnt += pieces(nks[i], target);
       if (cnt <= slots) break;
     }
-  }
-  std::vector<PTask> tasks;
-  int nslots = 0, npart = 0;
-  for (int64_t i = 0; i < nt; ++i) {
-    const GTile &t = tiles[i];
-    const int nk = (int)nks[i];
-    const int ks = t.kind == 0 ? pieces(nk, target) : 1;
-    if (ks == 1) {
-      tasks.push_back({t.block, t.m0, t.n0, t.kind, 0, nk, -1, 1, 0, 0});
-    } else {
-      const int slot = nslots++;
+    for (int64_t i = 0; i < nt; ++i) {
+      const GTile &t = tiles[i];
+      const int nk = (int)nks[i];
+      const int ks = t.kind == 0 ? pieces(nk, target) : 1;
+      const int slot = ks > 1 ? nslots++ : -1;
       for (int s = 0; s < ks; ++s)
-        tasks.push_back({t.block, t.m0, t.n0, t.kind, s * nk / ks, (s + 1) * nk / ks, slot, ks, s, npart});
+        lists.push_back({PTask{t.block, t.m0, t.n0, t.kind, (int32_t)((int64_t)s * nk / ks),
+                               (int32_t)((int64_t)(s + 1) * nk / ks), slot, ks, s, ks > 1 ? npart : 0}});
+      if (ks > 1) npart += ks;
+    }
+    std::stable_sort(lists.begin(), lists.end(), [](const std::vector<PTask> &x, const std::vector<PTask> &y) {
+      return x[0].ke - x[0].kb > y[0].ke - y[0].kb;
+    });
+  } else {
+    lists.resize((size_t)slots);
+    std::vector<std::vector<PTask>> whole((size_t)slots);
+    const double share = (double)(total + kTileCost * nt) / (double)slots;
+    double pos = 0.0;  // steps given out so far
+    int64_t cta = 0;
+    for (int64_t i = 0; i < nt; ++i) {
+      const GTile &t = tiles[i];
+      int64_t kb = 0;
+      std::vector<std::pair<int64_t, PTask>> cut;  // (CTA, piece)
+      while (true) {
+        const int64_t len = nks[i] - kb;
+        while (cta + 1 < slots && pos >= share * (double)(cta + 1)) ++cta;
+        const double room = share * (double)(cta + 1) - pos;
+        int64_t head = (int64_t)room;  // steps of this piece that fit the CTA's share
+        const bool may_cut = cta + 1 < slots && (int64_t)cut.size() + 1 < p->max_pieces;
+        if (!may_cut || len - head < min_steps) {
+          head = len;  // the rest of the tile, where what would be left over is not worth a piece
+        } else if (head < min_steps) {
+          ++cta;       // the share ends here
+          continue;
+        }
+        cut.push_back({cta, PTask{t.block, t.m0, t.n0, t.kind, (int32_t)kb, (int32_t)(kb + head), -1, 1, 0, 0}});
+        kb += head;
+        pos += (double)head;
+        if (kb >= nks[i]) break;
+      }
+      pos += kTileCost;
+      const int ks = (int)cut.size();
+      if (ks == 1) {
+        whole[cut[0].first].push_back(cut[0].second);
+        continue;
+      }
+      for (int s = 0; s < ks; ++s) {
+        PTask q = cut[s].second;
+        q.slot = nslots;
+        q.nsplit = ks;
+        q.sid = s;
+        q.pbase = npart;
+        lists[cut[s].first].push_back(q);
+      }
+      ++nslots;
       npart += ks;
     }
+    for (int64_t c = 0; c < slots; ++c) lists[c].insert(lists[c].end(), whole[c].begin(), whole[c].end());
+    lists.erase(std::remove_if(lists.begin(), lists.end(), [](const std::vector<PTask> &l) { return l.empty(); }),
+                lists.end());
   }
-  // longest first; CTA b takes tasks b, b + grid, ... (a static cost-ordered queue)
-  std::stable_sort(tasks.begin(), tasks.end(),
-                   [](const PTask &x, const PTask &y) { return (x.ke - x.kb) > (y.ke - y.kb); });
+  std::vector<PTask> tasks;
+  std::vector<int32_t> start{0};
+  for (const auto &l : lists) {
+    tasks.insert(tasks.end(), l.begin(), l.end());
+    start.push_back((int32_t)tasks.size());
+  }
+  for (const auto &l : lists) {  // then the K steps of every CTA
+    int32_t n = 0;
+    for (const PTask &q : l) n += q.kind == 0 ? q.ke - q.kb : 0;
+    start.push_back(n);
+  }
   p->nptasks = (int64_t)tasks.size();
-  p->pgrid = (int)std::min<int64_t>(p->nptasks, slots);
+  p->pgrid = (int)lists.size();
   cudaError_t e = cudaSuccess;
   if (!tasks.empty()) {
     e = cudaMalloc(&p->ptasks, tasks.size() * sizeof(PTask));
     if (e == cudaSuccess) e = cudaMemcpy(p->ptasks, tasks.data(), tasks.size() * sizeof(PTask), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMalloc((void **)&p->pstart, start.size() * sizeof(int32_t));
+    if (e == cudaSuccess)
+      e = cudaMemcpy(p->pstart, start.data(), start.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
   }
   if (e == cudaSuccess && nslots > 0) {
-    e = cudaMalloc((void **)&p->part, (size_t)npart * BM * BN * (cplx ? 2 : 1) * sizeof(double));
+    e = cudaMalloc((void **)&p->part, (size_t)npart * tm * tn * (cplx ? 2 : 1) * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc((void **)&p->pcnt, nslots * sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(p->pcnt, 0, nslots * sizeof(int));
   }
@@ -717,11 +881,13 @@ int tkb_gemm_launch(tkb_ctx *ctx, const tkb_plan *p, void *C, const void *A, con
   if (p->dtype == TKB_F64) {
     if (alpha.im != 0.0 || beta.im != 0.0)
       return tkb_set_error(ctx, TKB_ERR_ARG, "complex scalar with real data");
-    const size_t smem = sizeof(SmemR);
-    TKB_CUDA_TRY(ctx, cudaFuncSetAttribute(gemm_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const bool small = p->tile_m == SmallTile::BM;
+    const auto kfn = small ? gemm_f64_kernel<SmallTile> : gemm_f64_kernel<LargeTile>;
+    const size_t smem = small ? SmallTile::SMEM : LargeTile::SMEM;
+    TKB_CUDA_TRY(ctx, cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int base_ok = (((uintptr_t)A & 15) == 0 ? 1 : 0) | (((uintptr_t)B & 15) == 0 ? 2 : 0);
-    TKB_CUDA_TRY(ctx, launch_pdl(gemm_f64_kernel, dim3(p->pgrid), dim3(kRealThreads), smem, ctx->stream, p->blocks,
-                                 (const PTask *)p->ptasks, (int)p->nptasks, (double *)C, (const double *)A,
+    TKB_CUDA_TRY(ctx, launch_pdl(kfn, dim3(p->pgrid), dim3(small ? SmallTile::THREADS : LargeTile::THREADS), smem, ctx->stream, p->blocks,
+                                 (const PTask *)p->ptasks, (const int32_t *)p->pstart, (double *)C, (const double *)A,
                                  (const double *)B, alpha.re, beta.re, p->part, p->pcnt, base_ok));
   } else {
     if ((((uintptr_t)A | (uintptr_t)B | (uintptr_t)C) & 15) != 0)
@@ -729,7 +895,7 @@ int tkb_gemm_launch(tkb_ctx *ctx, const tkb_plan *p, void *C, const void *A, con
     const size_t smem = sizeof(SmemC);
     TKB_CUDA_TRY(ctx, cudaFuncSetAttribute(gemm_c128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     TKB_CUDA_TRY(ctx, launch_pdl(gemm_c128_kernel, dim3(p->pgrid), dim3(kCplxThreads), smem, ctx->stream, p->blocks,
-                                 (const PTask *)p->ptasks, (int)p->nptasks, (double2 *)C, (const double2 *)A,
+                                 (const PTask *)p->ptasks, (const int32_t *)p->pstart, (double2 *)C, (const double2 *)A,
                                  (const double2 *)B, CDbl{alpha.re, alpha.im}, CDbl{beta.re, beta.im}, p->part,
                                  p->pcnt));
   }

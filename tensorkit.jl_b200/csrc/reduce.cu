@@ -95,8 +95,8 @@ __global__ void __launch_bounds__(RT)
                   const T *__restrict__ x, const T *__restrict__ y, double2 *__restrict__ partial, int *arrived,
                   double *out) {
   __shared__ int last;
-  pdl_trigger();
   pdl_wait();  // the vectors, the partial sums and the counter belong to earlier kernels too
+  pdl_trigger();
   const int64_t per = (total + gridDim.x - 1) / gridDim.x;
   const int64_t cb = (int64_t)blockIdx.x * per;
   const int64_t ce = min(total, cb + per);

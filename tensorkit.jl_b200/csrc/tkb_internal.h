@@ -33,7 +33,9 @@ struct tkb_ctx {
 // programmatic dependent launch: a kernel launched with the programmatic-serialization
 // attribute may start while the previous kernel of the stream still runs; it must call
 // pdl_wait() before touching anything that kernel writes (a no-op without the attribute).
-// pdl_trigger() lets the next kernel be scheduled once every CTA of this one has called it.
+// pdl_trigger() lets the next kernel be scheduled once every CTA of this one has called it. It comes
+// after pdl_wait(): a kernel that triggers while it still waits lets the one after it occupy the SMs
+// that the kernel before it leaves first, which packs a grid of less than one wave onto them.
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
@@ -206,7 +208,7 @@ struct GTile {
 struct tkb_plan {
   tkb_ctx *owner = nullptr;
   int dtype = 0, precision = 0, slices = 0;
-  int64_t nblocks = 0, ntiles = 0;
+  int64_t nblocks = 0;
   GTile *sktasks = nullptr;     // skinny blocks: (block, first row) tasks of kSkinnyTaskRows rows
   int64_t nsk = 0;
   int sk_dim = 0;               // max(n, k) over the skinny blocks
@@ -214,7 +216,6 @@ struct tkb_plan {
   int64_t lenA = 0, lenB = 0, lenC = 0;
   std::vector<GBlock> hblocks;
   GBlock *blocks = nullptr;
-  GTile *tiles = nullptr;
   // split precision
   size_t ws_bytes = 0;          // workspace needed for slices + exponents
   int64_t slice_rows_A = 0, slice_rows_B = 0;  // total padded rows for the slicing pass
@@ -223,8 +224,9 @@ struct tkb_plan {
   int64_t expo_off = 0, expo_bytes = 0;  // exponent region inside the workspace
   void *kstiles = nullptr;      // tcgen05 product tasks (tile, K range, split slot)
   int64_t nkstiles = 0;
-  // plain precision: split-K tasks (tile, K range) in a static cost-ordered queue
+  // plain precision: tasks (tile, K range), CTA b runs [pstart[b], pstart[b + 1])
   void *ptasks = nullptr;
+  int32_t *pstart = nullptr;
   int64_t nptasks = 0;
   int pgrid = 0;                // CTAs of the plain launch
   double *part = nullptr;       // split-K FP64 partial tiles (rewritten every launch)
@@ -241,7 +243,7 @@ struct tkb_plan {
   int max_pieces = 8, min_piece_steps = 4;
 };
 
-int tkb_gemm_plain_prepare(tkb_ctx *ctx, tkb_plan *p, const std::vector<GTile> &tiles);
+int tkb_gemm_plain_prepare(tkb_ctx *ctx, tkb_plan *p);
 int tkb_gemm_launch(tkb_ctx *ctx, const tkb_plan *p, void *C, const void *A, const void *B,
                     tkb_scalar alpha, tkb_scalar beta);
 int tkb_gemm_split_prepare(tkb_ctx *ctx, tkb_plan *p);

@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 8 ? 3 : 2)
   const T beta = scalar_from<T>(beta_);
   const bool bz = beta_zero != 0;
   pdl_wait();     // source and destination belong to earlier kernels of the stream too
-  pdl_trigger();  // the next kernel may be scheduled; it waits for this grid before reading
+  pdl_trigger();
 
   // Each CTA walks a contiguous range of tasks (tasks of one group are contiguous, so the
   // group metadata stays in L1); the task → group map was built on the host.
@@ -271,7 +271,6 @@ __global__ void __launch_bounds__(kThreads)
   const T alpha = scalar_from<T>(alpha_);
   const T beta = scalar_from<T>(beta_);
   const bool bz = beta_zero != 0;
-  pdl_trigger();  // the next kernel may be scheduled; it waits for this grid before reading
   const int64_t per = (ntasks + gridDim.x - 1) / gridDim.x;  // ≤ kRecCache (host)
   const int64_t t_begin = (int64_t)blockIdx.x * per;
   const int64_t t_end = min(ntasks, t_begin + per);
@@ -283,6 +282,7 @@ __global__ void __launch_bounds__(kThreads)
   }
   __syncthreads();
   pdl_wait();  // the records are static; source and destination belong to earlier kernels
+  pdl_trigger();
 
   auto issue = [&](int64_t task, T *stage) {
     const TaskRec &R = rs[task - t_begin];
@@ -360,7 +360,6 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 && !PAIRS) ? 6 : 4)
   const T alpha = scalar_from<T>(alpha_);
   const T beta = scalar_from<T>(beta_);
   const bool bz = beta_zero != 0;
-  pdl_trigger();  // the next kernel may be scheduled; it waits for this grid before reading
   const int64_t per = (ntasks + gridDim.x - 1) / gridDim.x;  // ≤ kRecCache (host)
   const int64_t t_begin = (int64_t)blockIdx.x * per;
   const int64_t t_end = min(ntasks, t_begin + per);
@@ -372,6 +371,7 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 && !PAIRS) ? 6 : 4)
   }
   __syncthreads();
   pdl_wait();  // the records are static; source and destination belong to earlier kernels
+  pdl_trigger();
 
   for (int64_t task = t_begin; task < t_end; ++task) {
     const TaskRec &R = rs[task - t_begin];
@@ -479,11 +479,11 @@ __global__ void __launch_bounds__(kThreads, NS * P * sizeof(T) <= 80 ? 4 : NS * 
   const T alpha = scalar_from<T>(alpha_);
   const T beta = scalar_from<T>(beta_);
   const bool bz = beta_zero != 0;
-  pdl_trigger();  // the next kernel may be scheduled; it waits for this grid before reading
   int64_t task = blockIdx.x;
   if ((int)threadIdx.x < rec_words) buf[0][threadIdx.x] = __ldg(recs + task * rec_words + threadIdx.x);
   __syncthreads();
   pdl_wait();  // the records are static; source and destination belong to earlier kernels
+  pdl_trigger();
   for (int cur = 0; task < ntasks; cur ^= 1) {
     const int64_t next = task + gridDim.x;
     int64_t word = 0;

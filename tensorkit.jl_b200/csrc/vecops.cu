@@ -56,8 +56,8 @@ __global__ void __launch_bounds__(kVecThreads)
                  int odd) {
   using T = typename OP::T;
   const bool bz = beta_zero != 0;
-  pdl_trigger();
   pdl_wait();  // both vectors belong to earlier kernels of the stream
+  pdl_trigger();
   const int64_t step = (int64_t)gridDim.x * kVecThreads * kVecBatch;
   for (int64_t e0 = (int64_t)blockIdx.x * kVecThreads * kVecBatch + threadIdx.x; e0 < n; e0 += step) {
     T x[kVecBatch], y[kVecBatch];

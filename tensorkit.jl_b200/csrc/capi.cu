@@ -219,6 +219,9 @@ static int plan_create(tkb_ctx *ctx, const tkb_gemm_desc *d, const tkb_gemm_tuni
   p->lenB = d->lenB;
   p->lenC = d->lenC;
   std::vector<GTile> sk;
+  std::vector<ThinTask> th;
+  int64_t thin_k = 0;
+  int nthin = 0;
   double flops = 0;
   for (int64_t i = 0; i < nb; ++i) {
     GBlock b;
@@ -247,15 +250,32 @@ static int plan_create(tkb_ctx *ctx, const tkb_gemm_desc *d, const tkb_gemm_tuni
     }
     flops += (d->dtype == TKB_C128 ? 8.0 : 2.0) * (double)b.m * (double)b.n * (double)b.k;
     b.skinny = (b.n <= kSkinnyMax && b.k <= kSkinnyMax && b.m >= kSkinnyMinRows) ? 1 : 0;
-    if (b.skinny && b.m > 0 && b.n > 0) p->sk_dim = std::max<int>(p->sk_dim, (int)std::max(b.n, b.k));
+    if (!b.skinny && b.m > 0 && b.n > 0 && b.m <= kThinMax && b.n <= kThinMax && b.k >= kThinMinK) {
+      b.skinny = 2;
+      p->th_dim = std::max<int>(p->th_dim, (int)std::max(b.m, b.n));
+      thin_k += b.k;
+      ++nthin;
+    }
+    if (b.skinny == 1 && b.m > 0 && b.n > 0) p->sk_dim = std::max<int>(p->sk_dim, (int)std::max(b.n, b.k));
     p->hblocks.push_back(b);
     if (b.m > 0 && b.n > 0) {
-      if (b.skinny)
+      if (b.skinny == 1)
         for (int64_t m0 = 0; m0 < b.m; m0 += kSkinnyTaskRows)
           sk.push_back({(int32_t)i, (int32_t)m0, 0, b.k > 0 ? 0 : 1});
     }
   }
   p->nsk = (int64_t)sk.size();
+  // thin blocks: about two K ranges per SM over all of them, 1024 values at least
+  const int64_t range = std::max<int64_t>(1024, (thin_k + 2 * ctx->num_sms - 1) / (2 * ctx->num_sms));
+  for (int64_t i = 0, slot = 0; i < nb && nthin > 0; ++i) {
+    const GBlock &b = p->hblocks[i];
+    if (b.skinny != 2) continue;
+    const int32_t parts = (int32_t)((b.k + range - 1) / range), base = (int32_t)th.size();
+    for (int32_t s = 0; s < parts; ++s)
+      th.push_back({s * b.k / parts, (s + 1) * b.k / parts, (int32_t)i, (int32_t)slot, parts, s, base, 0});
+    ++slot;
+  }
+  p->nth = (int64_t)th.size();
   p->flops = flops;
   int rc = TKB_OK;
   if (d->precision == TKB_SPLIT_INT8) rc = tkb_gemm_split_prepare(ctx, p);
@@ -274,6 +294,14 @@ static int plan_create(tkb_ctx *ctx, const tkb_gemm_desc *d, const tkb_gemm_tuni
     e = cudaMalloc((void **)&p->sktasks, sk.size() * sizeof(GTile));
     if (e == cudaSuccess) e = cudaMemcpy(p->sktasks, sk.data(), sk.size() * sizeof(GTile), cudaMemcpyHostToDevice);
   }
+  if (e == cudaSuccess && !th.empty()) {
+    const size_t vals = (size_t)kThinMax * kThinMax * (p->dtype == TKB_C128 ? 2 : 1);
+    e = cudaMalloc((void **)&p->thtasks, th.size() * sizeof(ThinTask));
+    if (e == cudaSuccess) e = cudaMemcpy(p->thtasks, th.data(), th.size() * sizeof(ThinTask), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMalloc((void **)&p->thpart, th.size() * vals * sizeof(double));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&p->thcnt, nthin * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(p->thcnt, 0, nthin * sizeof(int));
+  }
   if (e != cudaSuccess) {
     tkb_gemm_plan_destroy(p);
     return tkb_set_error(ctx, TKB_ERR_CUDA, std::string("plan upload: ") + cudaGetErrorString(e));
@@ -286,6 +314,9 @@ int tkb_gemm_plan_destroy(tkb_plan *p) {
   if (!p) return TKB_OK;
   cudaFree(p->blocks);
   cudaFree(p->sktasks);
+  cudaFree(p->thtasks);
+  cudaFree(p->thpart);
+  cudaFree(p->thcnt);
   cudaFree(p->ptasks);
   cudaFree(p->pstart);
   cudaFree(p->bstat);
@@ -327,7 +358,8 @@ int tkb_grouped_gemm(tkb_ctx *ctx, const tkb_plan *p, void *C, const void *A, co
   if (p->owner != ctx) return tkb_set_error(ctx, TKB_ERR_ARG, "plan belongs to another context");
   if (p->nblocks > 0 && (!C || (p->flops > 0 && (!A || !B))))
     return tkb_set_error(ctx, TKB_ERR_ARG, "null data pointer");
-  const int rc = tkb_gemm_skinny_launch(ctx, p, C, A, B, alpha, beta);
+  int rc = tkb_gemm_skinny_launch(ctx, p, C, A, B, alpha, beta);
+  if (rc == TKB_OK) rc = tkb_gemm_thin_launch(ctx, p, C, A, B, alpha, beta);
   if (rc != TKB_OK) return rc;
   if (p->precision == TKB_SPLIT_INT8) return tkb_gemm_split_launch(ctx, p, C, A, B, alpha, beta);
   return tkb_gemm_launch(ctx, p, C, A, B, alpha, beta);

@@ -184,7 +184,7 @@ struct GBlock {
   // split precision: workspace offsets of the sliced operands and exponents
   int64_t wsA, wsB, wsEA, wsEB;
   int32_t mpad, npad, kpad;   // padded extents (tile multiples) of the sliced operands
-  int32_t skinny;             // 1: n, k ≤ 16 — memory-bound row kernel in every precision
+  int32_t skinny;             // 1: n, k ≤ 16 — memory-bound row kernel in every precision; 2: thin output, long K
   int32_t fp64only;           // split precision: K too long for two exact int32 pieces — FP64 tiles
 };
 
@@ -193,11 +193,24 @@ constexpr int kSkinnyMinRows = 2048;  // smaller blocks go to the tiled kernels
 constexpr int kSkinnyRows = 256;       // threads of a skinny CTA (one row each per pass)
 constexpr int kSkinnyTaskRows = 1024;  // rows of one skinny task
 
+constexpr int kThinMax = 4;        // m and n bound of the thin path (a few dot products over a long K)
+constexpr int kThinMinK = 512;     // shorter K goes to the tiled kernels
+// one task of the thin kernel: a K range of one block's products
+struct ThinTask {
+  int64_t l0, l1;
+  int32_t block, slot;          // slot: the block's arrival counter
+  int32_t nsplit, sid, pbase;   // tasks of the block, this task's index, first of their partial sums
+  int32_t pad;
+};
+
 // CTAs per SM of a kernel (cached per kernel and device; sets the dynamic shared memory limit)
 int tkb_occupancy(int device, const void *kfn, int threads, size_t smem);
 
 int tkb_gemm_skinny_launch(tkb_ctx *ctx, const tkb_plan *p, void *C, const void *A,
                            const void *B, tkb_scalar alpha, tkb_scalar beta);
+
+int tkb_gemm_thin_launch(tkb_ctx *ctx, const tkb_plan *p, void *C, const void *A, const void *B,
+                         tkb_scalar alpha, tkb_scalar beta);
 
 struct GTile {
   int32_t block;
@@ -212,6 +225,11 @@ struct tkb_plan {
   GTile *sktasks = nullptr;     // skinny blocks: (block, first row) tasks of kSkinnyTaskRows rows
   int64_t nsk = 0;
   int sk_dim = 0;               // max(n, k) over the skinny blocks
+  ThinTask *thtasks = nullptr;  // thin blocks: K ranges, their partial sums and arrival counters
+  int64_t nth = 0;
+  int th_dim = 0;               // max(m, n) over the thin blocks
+  double *thpart = nullptr;
+  int *thcnt = nullptr;
   double flops = 0;
   int64_t lenA = 0, lenB = 0, lenC = 0;
   std::vector<GBlock> hblocks;

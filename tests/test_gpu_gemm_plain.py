@@ -22,7 +22,7 @@ def _op(X, op):
     return X if op == L.TKB_OP_N else X.T if op == L.TKB_OP_T else X.conj().T
 
 
-def _run(shapes, cplx, ops, odd, tuning=None, alpha=0.7, beta=-1.3, shift=0, seed=0):
+def _run(shapes, cplx, ops, odd, tuning=None, alpha=0.7, beta=-1.3, shift=0, seed=0, prec=L.TKB_PLAIN):
     """shapes: (m, n, k) per block; checks C = α·op(A)·op(B) + β·C."""
     rng = np.random.default_rng(seed)
     rnd = lambda n: rng.standard_normal(n) + (1j * rng.standard_normal(n) if cplx else 0)  # noqa: E731
@@ -41,7 +41,7 @@ def _run(shapes, cplx, ops, odd, tuning=None, alpha=0.7, beta=-1.3, shift=0, see
     Ad, Bd, Cd = put(A), put(B), put(Cv)
     torch.cuda.synchronize()
     ctx = tk.get_context(0)
-    plan = GemmPlan(ctx, rows, (len(A), len(B), len(Cv)), L.TKB_C128 if cplx else L.TKB_F64, L.TKB_PLAIN, 0, tuning)
+    plan = GemmPlan(ctx, rows, (len(A), len(B), len(Cv)), L.TKB_C128 if cplx else L.TKB_F64, prec, 0, tuning)
     sc = lambda x: L.tkb_scalar(complex(x).real, complex(x).imag)  # noqa: E731
     for _ in range(2):  # twice: the split-K counters clear themselves
         Cd.copy_(put(Cv))
@@ -83,6 +83,17 @@ def test_plain_blocks(shapes, ops, odd, cplx):
 @pytest.mark.parametrize("shapes", [FEW, MANY], ids=["few", "many"])
 def test_plain_tuned(shapes, cplx, tuning):
     _run(shapes, cplx, [(N, N), (T, T)], 1, tuning, beta=0.0)
+
+
+THIN = [(1, 1, 512), (1, 1, 513), (1, 1, 511), (4, 4, 3000), (2, 3, 70001), (1, 4, 2048), (5, 1, 2000), (64, 48, 40)]
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("ops", OPS, ids=["NN", "TN-NT", "mixed"])
+@pytest.mark.parametrize("shapes", [THIN, THIN[:1], THIN[:3]], ids=["mixed", "one", "dots"])
+def test_thin_blocks(shapes, ops, cplx):
+    _run(shapes, cplx, ops, 1)
+    _run(shapes[:6], cplx, ops, 0, beta=0.0, prec=L.TKB_SPLIT_INT8)  # thin blocks run in FP64 in either precision
 
 
 def test_plain_unaligned_base():

@@ -1,7 +1,7 @@
 // Plain FP64 / ComplexF64 grouped block GEMM: one launch for all coupled-sector blocks of a
 // TensorKit mul! (src/tensors/linalg.jl:330-370).
 //
-// Tensor path: FP64 DMMA (mma.sync m16n8k8 for real data, m8n8k4 for complex). tcgen05 has no
+// Tensor path: FP64 DMMA (mma.sync m16n8k8; four of them per complex fragment pair). tcgen05 has no
 // f64 kind, so the double-precision tensor pipe is reached through DMMA; the split-precision
 // path (gemm_split.cu) is the tcgen05 one.
 //
@@ -11,7 +11,7 @@
 // FP64 partial tile; the piece that arrives last on the tile's counter adds all partials in piece
 // order (deterministic, no piece waits for another) and applies α, β.
 //
-// Real CTA: 4 warps in a 2×2 grid, m16n8k8 tiles, BK = 16, a three-stage cp.async ring (two stages in
+// CTA: 4 warps in a 2×2 grid, m16n8k8 tiles, BK = 16, a three-stage cp.async ring (two stages in
 // flight while one is consumed; one barrier per K step; a stage's DMMA are issued before the refill
 // copies). The ring runs through all tasks of the CTA without a break: the next tile's first stages
 // arrive while the last one's values are stored. Operand tiles are copied in 16-byte pairs when the
@@ -33,10 +33,7 @@
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16, NST = 3;
-constexpr int APAD = 4, BPAD = 4;      // real: keeps 16-byte row alignment, spreads banks
-constexpr int CAPAD = 2, CBPAD = 2;    // complex (16-byte elements)
-constexpr int kCplxThreads = 256;
+constexpr int BK = 16;  // K positions per stage
 
 struct CDbl {
   double x, y;
@@ -86,11 +83,6 @@ __device__ __forceinline__ unsigned long long pl_now() {
 #endif
 #define PL_STAMP(k) PL_SET(k, pl_now())
 
-__device__ __forceinline__ void dmma(double &c0, double &c1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(c0), "+d"(c1)
-               : "d"(a), "d"(b));
-}
 // D(16×8) += A(16×8) B(8×8), FP64. Lane (g = lane/4, t = lane%4): a = A[g][t], A[g+8][t],
 // A[g][t+4], A[g+8][t+4]; b = B[t][g], B[t+4][g]; c = D[g][2t], D[g][2t+1], D[g+8][2t],
 // D[g+8][2t+1] (checked against a host product on the device)
@@ -100,16 +92,20 @@ __device__ __forceinline__ void dmma16(double (&c)[4], const double (&a)[4], con
                : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
-// ---- real ----------------------------------------------------------------------------
-// Tile shape of a real kernel: BMxBN output tile, warps of WMxWN (m16n8k8 fragments)
-template <int BM_, int BN_, int WM_, int WN_, int NST_, int MINB_>
-struct RealCfg {
+// ---- tiled kernel ------------------------------------------------------------------------
+// Tile shape of a kernel for elements E (double, or double2 for complex data): BMxBN output tile, warps
+// of WMxWN (m16n8k8 fragments). The pitches spread the fragments of a warp over the banks.
+template <typename E_, int BM_, int BN_, int WM_, int WN_, int NST_, int MINB_>
+struct TileCfg {
+  using E = E_;
+  static constexpr bool CPLX = sizeof(E) == 16;
   static constexpr int BM = BM_, BN = BN_, WM = WM_, WN = WN_, NST = NST_, MINB = MINB_;
   static constexpr int WARPS_M = BM / WM, WARPS = (BM / WM) * (BN / WN), THREADS = 32 * WARPS;
-  static constexpr int MI = WM / 16, NI = WN / 8, NV = MI * NI * 4;
-  static constexpr int PA = BM + APAD, PB = BK + BPAD;  // pitches: op(A) tile [k][row], op(B) tile [col][k]
+  static constexpr int MI = WM / 16, NI = WN / 8, NV = MI * NI * (CPLX ? 8 : 4);  // NV: accumulators per thread
+  // pitches: op(A) tile [k][row], op(B) tile [col][k]
+  static constexpr int PA = BM + (CPLX ? 2 : 4), PB = BK + 4;
   static constexpr int A_ELEMS = BK * PA, B_ELEMS = BN * PB, STAGE = A_ELEMS + B_ELEMS;
-  static constexpr size_t SMEM = (size_t)NST * STAGE * sizeof(double);
+  static constexpr size_t SMEM = (size_t)NST * STAGE * sizeof(E);
 };
 
 // Copies of one operand's tiles, resolved once per task: the thread's first source element, the
@@ -121,9 +117,9 @@ struct RealCfg {
 //   kind 0: the tile's outer index (rows of op(A), columns of op(B)) is contiguous in memory
 //   kind 1: K is contiguous
 //   kind 2: 16-byte pairs along the contiguous direction that the stage keeps contiguous too
-template <int T, int OUTER, bool IS_A, int PITCH>
+template <typename E, int T, int OUTER, bool IS_A, int PITCH>
 struct TileCopy {
-  const double *p, *base;  // base: the operand's first element (where copies that read nothing point)
+  const E *p, *base;  // base: the operand's first element (where copies that read nothing point)
   int64_t dr, dk;    // elements: between the copies of a stage, between stages
   int kind, o, ext;  // outer position of the first copy in the block, the block's extent (clamped)
   int l0, s0;        // K position and stage offset of the first copy
@@ -151,7 +147,7 @@ struct TileCopy {
     s0 = IS_A ? l0 * PITCH + oo : oo * PITCH + l0;
     o = oo;
   }
-  __device__ __forceinline__ void init(const double *X, int64_t off, int64_t ld, bool outer_contig, int64_t o0,
+  __device__ __forceinline__ void init(const E *X, int64_t off, int64_t ld, bool outer_contig, int64_t o0,
                                        int64_t extent, int64_t kbeg, bool pairs) {
     const int64_t so = outer_contig ? 1 : ld, sk = outer_contig ? ld : 1;
     base = X + off;
@@ -162,18 +158,22 @@ struct TileCopy {
     kind = pairs && outer_contig == IS_A ? 2 : outer_contig ? 0 : 1;
     if (kind == 0) init_kind<0>(so, sk, o0, kbeg);
     else if (kind == 1) init_kind<1>(so, sk, o0, kbeg);
-    else init_kind<2>(so, sk, o0, kbeg);
+    else if constexpr (sizeof(E) == 8) init_kind<2>(so, sk, o0, kbeg);
+  }
+  static __device__ __forceinline__ void copy(E *d, const E *q, bool v) {
+    if constexpr (sizeof(E) == 8) cp_async8(d, q, v);
+    else cp_async16(d, q, v ? 16 : 0);
   }
   template <int KIND>
-  __device__ __forceinline__ void issue_kind(double *stage, int64_t left) {
+  __device__ __forceinline__ void issue_kind(E *stage, int64_t left) {
     using L = Lay<KIND>;
-    double *d = stage + s0;
-    const double *q = p;
+    E *d = stage + s0;
+    const E *q = p;
     if (inside && left >= BK) {
 #pragma unroll
       for (int r = 0; r < L::COPIES; ++r, q += dr) {
         if constexpr (KIND == 2) cp_async16(d + r * L::DS, q, 16);
-        else cp_async8(d + r * L::DS, q, true);
+        else copy(d + r * L::DS, q, true);
       }
     } else {
 #pragma unroll
@@ -185,16 +185,16 @@ struct TileCopy {
           cp_async16(d + r * L::DS, v ? q : base, v ? (w ? 16 : 8) : 0);
         } else {
           const bool v = oo < ext && l < left;
-          cp_async8(d + r * L::DS, v ? q : base, v);
+          copy(d + r * L::DS, v ? q : base, v);
         }
       }
     }
   }
   // the copies of the next stage into `stage`; left: K positions of the block from this stage on
-  __device__ __forceinline__ void issue(double *stage, int64_t left) {
+  __device__ __forceinline__ void issue(E *stage, int64_t left) {
     if (kind == 0) issue_kind<0>(stage, left);
     else if (kind == 1) issue_kind<1>(stage, left);
-    else issue_kind<2>(stage, left);
+    else if constexpr (sizeof(E) == 8) issue_kind<2>(stage, left);
     p += dk;
   }
 };
@@ -206,31 +206,6 @@ __device__ __forceinline__ int vec_flags(const GBlock &b, int base_ok) {
   if ((base_ok & 1) && b.opA == TKB_OP_N && !(b.offA & 1) && !(b.lda & 1)) v |= 1;
   if ((base_ok & 2) && b.opB == TKB_OP_N && !(b.offB & 1) && !(b.ldb & 1)) v |= 2;
   return v;
-}
-
-// K loop of one task through an NS-stage ring: `load(st, k0)` fills ring slot st with the
-// tiles at K offset k0, `step(st)` consumes slot st. Every iteration commits one group (possibly
-// empty), so wait_group<NS-2> always means "the group of this iteration's stage has landed".
-template <int NS, typename Load, typename Step>
-__device__ __forceinline__ void k_loop(int kb, int ke, Load &&load, Step &&step) {
-  const int nk = ke - kb;
-#pragma unroll
-  for (int st = 0; st < NS - 1; ++st) {
-    if (st < nk) load(st, (int64_t)(kb + st) * BK);
-    cp_async_commit();
-  }
-  for (int kt = 0; kt < nk; ++kt) {
-    cp_async_wait<NS - 2>();
-    __syncthreads();  // stage kt visible to all; every warp is done with stage kt-1's slot
-    const int nxt = kt + NS - 1;
-    // this stage's DMMA first, then the refill of the slot read in the previous iteration: the
-    // copies are issued while the DMMA execute
-    step(kt % NS);
-    if (nxt < nk) load(nxt % NS, (int64_t)(kb + nxt) * BK);
-    cp_async_commit();
-  }
-  cp_async_wait<0>();
-  __syncthreads();  // the ring may be refilled by the next task
 }
 
 // Split-K: store this piece's values (q-major: value q of every thread, so warps store
@@ -263,24 +238,91 @@ __device__ __forceinline__ bool splitk_reduce(const PTask &t, double (&v)[NV], d
   return true;
 }
 
+// v with its sign flipped where mask is 0x80000000
+__device__ __forceinline__ double flip(double v, int mask) {
+  return __hiloint2double(__double2hiint(v) ^ mask, __double2loint(v));
+}
+
+// the products of one stage: op(A) tile sa (offset to the warp's rows), op(B) tile sb
+template <typename CFG>
+__device__ __forceinline__ void stage_products(double (&acc)[CFG::NV], const typename CFG::E *sa,
+                                               const typename CFG::E *sb, int t, int conjA, int conjB) {
+#pragma unroll
+  for (int kk = 0; kk < BK; kk += 8) {
+    if constexpr (!CFG::CPLX) {
+      double af[CFG::MI][4], bf[CFG::NI][2];
+#pragma unroll
+      for (int mi = 0; mi < CFG::MI; ++mi)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) af[mi][q] = sa[(kk + t + 4 * (q >> 1)) * CFG::PA + mi * 16 + 8 * (q & 1)];
+#pragma unroll
+      for (int ni = 0; ni < CFG::NI; ++ni)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) bf[ni][q] = sb[ni * 8 * CFG::PB + kk + t + 4 * q];
+#pragma unroll
+      for (int mi = 0; mi < CFG::MI; ++mi)
+#pragma unroll
+        for (int ni = 0; ni < CFG::NI; ++ni)
+          dmma16(*reinterpret_cast<double(*)[4]>(&acc[(mi * CFG::NI + ni) * 4]), af[mi], bf[ni]);
+    } else {
+      double br[CFG::NI][2], bi[CFG::NI][2];
+#pragma unroll
+      for (int ni = 0; ni < CFG::NI; ++ni)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const double2 v = sb[ni * 8 * CFG::PB + kk + t + 4 * q];
+          br[ni][q] = v.x;
+          bi[ni][q] = flip(v.y, conjB);
+        }
+#pragma unroll
+      for (int mi = 0; mi < CFG::MI; ++mi) {
+        double ar[4], ai[4], an[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const double2 v = sa[(kk + t + 4 * (q >> 1)) * CFG::PA + mi * 16 + 8 * (q & 1)];
+          ar[q] = v.x;
+          ai[q] = flip(v.y, conjA);
+          an[q] = flip(ai[q], (int)0x80000000);
+        }
+        // real products of all column fragments, then the imaginary ones: no two neighbours share
+        // an accumulator
+#pragma unroll
+        for (int ni = 0; ni < CFG::NI; ++ni) {
+          double *c = &acc[(mi * CFG::NI + ni) * 8];
+          dmma16(*reinterpret_cast<double(*)[4]>(c), ar, br[ni]);
+          dmma16(*reinterpret_cast<double(*)[4]>(c + 4), ar, bi[ni]);
+        }
+#pragma unroll
+        for (int ni = 0; ni < CFG::NI; ++ni) {
+          double *c = &acc[(mi * CFG::NI + ni) * 8];
+          dmma16(*reinterpret_cast<double(*)[4]>(c), an, bi[ni]);
+          dmma16(*reinterpret_cast<double(*)[4]>(c + 4), ai, br[ni]);
+        }
+      }
+    }
+  }
+}
+
 template <typename CFG>
 __global__ void __launch_bounds__(CFG::THREADS, CFG::MINB)
-    gemm_f64_kernel(const GBlock *__restrict__ blocks, const PTask *__restrict__ tasks,
-                    const int32_t *__restrict__ start, double *__restrict__ C, const double *__restrict__ A,
-                    const double *__restrict__ B, double alpha, double beta, double *__restrict__ part,
-                    int *__restrict__ pcnt, int base_ok) {
+    gemm_plain_kernel(const GBlock *__restrict__ blocks, const PTask *__restrict__ tasks,
+                      const int32_t *__restrict__ start, typename CFG::E *__restrict__ C,
+                      const typename CFG::E *__restrict__ A, const typename CFG::E *__restrict__ B, CDbl alpha,
+                      CDbl beta, double *__restrict__ part, int *__restrict__ pcnt, int base_ok) {
+  using E = typename CFG::E;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double *sm = reinterpret_cast<double *>(smem_raw);
+  E *sm = reinterpret_cast<E *>(smem_raw);
   __shared__ int ticket;
   PL_STAMP(0);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wm = (warp % CFG::WARPS_M) * CFG::WM, wn = (warp / CFG::WARPS_M) * CFG::WN;
   const int g = lane >> 2, t = lane & 3;
+  const bool bz = beta.x == 0.0 && beta.y == 0.0;
   const int t_begin = start[blockIdx.x], t_end = start[blockIdx.x + 1];
   // The stages of all the CTA's tasks form one stream through the ring: the copies run NST − 1 stages
   // ahead of the products and go on into the next task while this one finishes.
-  TileCopy<CFG::THREADS, CFG::BM, true, CFG::PA> ca;
-  TileCopy<CFG::THREADS, CFG::BN, false, CFG::PB> cb;
+  TileCopy<E, CFG::THREADS, CFG::BM, true, CFG::PA> ca;
+  TileCopy<E, CFG::THREADS, CFG::BN, false, CFG::PB> cb;
   int next = t_begin, ahead = 0;  // the next task to copy, stages of the current one not yet copied
   int64_t left = 0;               // K positions of its block from the next stage on
   auto advance = [&]() {
@@ -289,7 +331,7 @@ __global__ void __launch_bounds__(CFG::THREADS, CFG::MINB)
       ahead = q.kind == 0 ? q.ke - q.kb : 0;
       if (ahead == 0) continue;
       const GBlock &b = blocks[q.block];
-      const int vec = vec_flags(b, base_ok);
+      const int vec = CFG::CPLX ? 0 : vec_flags(b, base_ok);
       const int64_t k0 = (int64_t)q.kb * BK;
       ca.init(A, b.offA, b.lda, b.opA == TKB_OP_N, q.m0, b.m, k0, vec & 1);
       cb.init(B, b.offB, b.ldb, b.opB != TKB_OP_N, q.n0, b.n, k0, vec & 2);
@@ -315,6 +357,12 @@ __global__ void __launch_bounds__(CFG::THREADS, CFG::MINB)
   [[maybe_unused]] int ntask = 0;
   for (int ti = t_begin; ti < t_end; ++ti, ++ntask) {
     const PTask task = tasks[ti];
+    // conjugation of an operand flips the sign of its imaginary part
+    int conjA = 0, conjB = 0;
+    if constexpr (CFG::CPLX) {
+      conjA = blocks[task.block].opA == TKB_OP_C ? (int)0x80000000 : 0;
+      conjB = blocks[task.block].opB == TKB_OP_C ? (int)0x80000000 : 0;
+    }
     double acc[CFG::NV];
 #pragma unroll
     for (int q = 0; q < CFG::NV; ++q) acc[q] = 0.0;
@@ -322,28 +370,8 @@ __global__ void __launch_bounds__(CFG::THREADS, CFG::MINB)
     for (int kt = 0; kt < nk; ++kt) {
       cp_async_wait<CFG::NST - 2>();
       __syncthreads();  // this stage is visible to all; every warp is done with the slot before it
-      const double *sa = sm + slot * CFG::STAGE + wm + g, *sb = sm + slot * CFG::STAGE + CFG::A_ELEMS;
-#pragma unroll
-      for (int kk = 0; kk < BK; kk += 8) {
-        double af[CFG::MI][4], bf[CFG::NI][2];
-#pragma unroll
-        for (int mi = 0; mi < CFG::MI; ++mi) {
-          af[mi][0] = sa[(kk + t) * CFG::PA + mi * 16];
-          af[mi][1] = sa[(kk + t) * CFG::PA + mi * 16 + 8];
-          af[mi][2] = sa[(kk + t + 4) * CFG::PA + mi * 16];
-          af[mi][3] = sa[(kk + t + 4) * CFG::PA + mi * 16 + 8];
-        }
-#pragma unroll
-        for (int ni = 0; ni < CFG::NI; ++ni) {
-          bf[ni][0] = sb[(wn + ni * 8 + g) * CFG::PB + kk + t];
-          bf[ni][1] = sb[(wn + ni * 8 + g) * CFG::PB + kk + t + 4];
-        }
-#pragma unroll
-        for (int mi = 0; mi < CFG::MI; ++mi)
-#pragma unroll
-          for (int ni = 0; ni < CFG::NI; ++ni)
-            dmma16(*reinterpret_cast<double(*)[4]>(&acc[(mi * CFG::NI + ni) * 4]), af[mi], bf[ni]);
-      }
+      const E *st = sm + slot * CFG::STAGE;
+      stage_products<CFG>(acc, st + wm + g, st + CFG::A_ELEMS + (wn + g) * CFG::PB, t, conjA, conjB);
       // the refill of the slot read in the previous iteration is issued while the DMMA execute
       produce(slot == 0 ? CFG::NST - 1 : slot - 1);
       slot = slot + 1 == CFG::NST ? 0 : slot + 1;
@@ -358,28 +386,40 @@ __global__ void __launch_bounds__(CFG::THREADS, CFG::MINB)
     if (!fin) continue;
     const GBlock &b = blocks[task.block];
     // epilogue: C = α·acc + β·C, column by column of the thread (column fragment q/2, column 2t + q%2);
-    // its rows are 8 apart, so one pointer per column serves them all. Row h is
-    // acc[((h/2)·NI + q/2)·4 + (h%2)·2 + q%2]
+    // its rows are 8 apart, so one pointer per column serves them all. Row h of column q is value
+    // (h%2)·2 + q%2 of fragment (h/2, q/2) (complex: the imaginary part four values further)
     const int64_t i0 = task.m0 + wm + g, j0 = task.n0 + wn + 2 * t;
     const int rows = (int)min((int64_t)CFG::WM, b.m - i0);  // valid rows from i0 on (may be ≤ 0)
     const int cols = (int)min((int64_t)CFG::WN, b.n - j0);
-    double *pc = C + b.offC + i0 + j0 * b.ldc;
     const int64_t ldc = b.ldc;
+    E *pc = C + b.offC + i0 + j0 * ldc;
 #pragma unroll
     for (int q = 0; q < 2 * CFG::NI; ++q) {
       if ((q / 2) * 8 + (q % 2) >= cols) continue;
-      double *p = pc + ((q / 2) * 8 + (q % 2)) * ldc;
-      double old[2 * CFG::MI];
-      if (beta != 0.0) {
+      E *p = pc + ((q / 2) * 8 + (q % 2)) * ldc;
+      E old[2 * CFG::MI];
+      if (!bz) {
 #pragma unroll
-        for (int h = 0; h < 2 * CFG::MI; ++h) old[h] = h * 8 < rows ? p[h * 8] : 0.0;
+        for (int h = 0; h < 2 * CFG::MI; ++h)
+          if (h * 8 < rows) old[h] = p[h * 8];
       }
 #pragma unroll
       for (int h = 0; h < 2 * CFG::MI; ++h) {
         if (h * 8 < rows) {
-          double r = alpha * acc[((h >> 1) * CFG::NI + (q >> 1)) * 4 + (h & 1) * 2 + (q & 1)];
-          if (beta != 0.0) r = fma(beta, old[h], r);
-          p[h * 8] = r;
+          const double *f = &acc[((h >> 1) * CFG::NI + (q >> 1)) * (CFG::CPLX ? 8 : 4) + (h & 1) * 2 + (q & 1)];
+          if constexpr (!CFG::CPLX) {
+            double r = alpha.x * f[0];
+            if (!bz) r = fma(beta.x, old[h], r);
+            p[h * 8] = r;
+          } else {
+            double rr = alpha.x * f[0] - alpha.y * f[4];
+            double ri = alpha.x * f[4] + alpha.y * f[0];
+            if (!bz) {
+              rr = fma(beta.x, old[h].x, fma(-beta.y, old[h].y, rr));
+              ri = fma(beta.x, old[h].y, fma(beta.y, old[h].x, ri));
+            }
+            p[h * 8] = make_double2(rr, ri);
+          }
         }
       }
     }
@@ -393,141 +433,12 @@ __global__ void __launch_bounds__(CFG::THREADS, CFG::MINB)
 // 32.5 instead of 33.8 TFLOP/s, eight 32×16 warps at 29.7). SmallTile: six CTAs of four 16×16 warps
 // per SM, for launches whose 64×64 tiles would leave most of the chip to one CTA per SM, which spends
 // 0.87 us per K step where its DMMA take 0.52.
-using LargeTile = RealCfg<64, 64, 32, 32, 3, 2>;
-using SmallTile = RealCfg<32, 32, 16, 16, 3, 6>;
-
-// ---- complex ---------------------------------------------------------------------------
-struct SmemC {
-  double2 A[NST][BK][BM + CAPAD];  // op(A) tile, [k][row], whole complex elements
-  double2 B[NST][BN][BK + CBPAD];  // op(B) tile, [col][k]
-};
-
-__device__ __forceinline__ void load_tiles_c(SmemC &s, int st, const GBlock &b, const double2 *A,
-                                             const double2 *B, int64_t m0, int64_t n0, int64_t k0) {
-  const int tid = threadIdx.x;
-  if (b.opA == TKB_OP_N) {
-#pragma unroll
-    for (int r = 0; r < (BM * BK) / kCplxThreads; ++r) {
-      const int e = tid + r * kCplxThreads;
-      const int i = e % BM, l = e / BM;
-      const int64_t gi = m0 + i, gl = k0 + l;
-      const bool ok = gi < b.m && gl < b.k;
-      cp_async16(&s.A[st][l][i], A + b.offA + (ok ? gi + gl * b.lda : 0), ok ? 16 : 0);
-    }
-  } else {
-#pragma unroll
-    for (int r = 0; r < (BM * BK) / kCplxThreads; ++r) {
-      const int e = tid + r * kCplxThreads;
-      const int l = e % BK, i = e / BK;
-      const int64_t gi = m0 + i, gl = k0 + l;
-      const bool ok = gi < b.m && gl < b.k;
-      cp_async16(&s.A[st][l][i], A + b.offA + (ok ? gl + gi * b.lda : 0), ok ? 16 : 0);
-    }
-  }
-  if (b.opB == TKB_OP_N) {
-#pragma unroll
-    for (int r = 0; r < (BN * BK) / kCplxThreads; ++r) {
-      const int e = tid + r * kCplxThreads;
-      const int l = e % BK, j = e / BK;
-      const int64_t gl = k0 + l, gj = n0 + j;
-      const bool ok = gl < b.k && gj < b.n;
-      cp_async16(&s.B[st][j][l], B + b.offB + (ok ? gl + gj * b.ldb : 0), ok ? 16 : 0);
-    }
-  } else {
-#pragma unroll
-    for (int r = 0; r < (BN * BK) / kCplxThreads; ++r) {
-      const int e = tid + r * kCplxThreads;
-      const int j = e % BN, l = e / BN;
-      const int64_t gl = k0 + l, gj = n0 + j;
-      const bool ok = gl < b.k && gj < b.n;
-      cp_async16(&s.B[st][j][l], B + b.offB + (ok ? gj + gl * b.ldb : 0), ok ? 16 : 0);
-    }
-  }
-}
-
-__global__ void __launch_bounds__(kCplxThreads, 2)
-    gemm_c128_kernel(const GBlock *__restrict__ blocks, const PTask *__restrict__ tasks,
-                     const int32_t *__restrict__ start, double2 *__restrict__ C, const double2 *__restrict__ A, const double2 *__restrict__ B,
-                     CDbl alpha, CDbl beta, double *__restrict__ part, int *__restrict__ pcnt) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  SmemC &s = *reinterpret_cast<SmemC *>(smem_raw);
-  __shared__ int ticket;
-  pdl_wait();
-  pdl_trigger();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;  // 8 warps: 2 (m) x 4 (n)
-  const int wm = warp & 1, wn = warp >> 1;                      // warp tile 32 x 16
-  const int g = lane >> 2, t = lane & 3;
-  const bool bz = beta.x == 0.0 && beta.y == 0.0;
-  const int t_end = start[blockIdx.x + 1];
-  for (int ti = start[blockIdx.x]; ti < t_end; ++ti) {
-    const PTask task = tasks[ti];
-    const GBlock b = blocks[task.block];
-    // conjugation of an operand flips the sign of its imaginary part
-    const double sa = (b.opA == TKB_OP_C) ? -1.0 : 1.0;
-    const double sb = (b.opB == TKB_OP_C) ? -1.0 : 1.0;
-    const int64_t m0 = task.m0, n0 = task.n0;
-    // acc[(mi*2 + ni)*4 + {0,1}] = Re (columns 2t, 2t+1), +{2,3} = Im
-    double acc[32];
-#pragma unroll
-    for (int q = 0; q < 32; ++q) acc[q] = 0.0;
-    if (task.kind == 0 && task.ke > task.kb) {
-      k_loop<NST>(task.kb, task.ke, [&](int st, int64_t k0) { load_tiles_c(s, st, b, A, B, m0, n0, k0); },
-             [&](int st) {
-#pragma unroll
-               for (int kk = 0; kk < BK; kk += 4) {
-                 double fr[4], fi[4], fin[4], gr[2], gi[2];
-#pragma unroll
-                 for (int mi = 0; mi < 4; ++mi) {
-                   const double2 v = s.A[st][kk + t][wm * 32 + mi * 8 + g];
-                   fr[mi] = v.x;
-                   fi[mi] = sa * v.y;
-                   fin[mi] = -fi[mi];
-                 }
-#pragma unroll
-                 for (int ni = 0; ni < 2; ++ni) {
-                   const double2 v = s.B[st][wn * 16 + ni * 8 + g][kk + t];
-                   gr[ni] = v.x;
-                   gi[ni] = sb * v.y;
-                 }
-#pragma unroll
-                 for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-                   for (int ni = 0; ni < 2; ++ni) {
-                     double *a = &acc[(mi * 2 + ni) * 4];
-                     dmma(a[0], a[1], fr[mi], gr[ni]);
-                     dmma(a[0], a[1], fin[mi], gi[ni]);
-                     dmma(a[2], a[3], fr[mi], gi[ni]);
-                     dmma(a[2], a[3], fi[mi], gr[ni]);
-                   }
-               }
-             });
-    }
-    if (!splitk_reduce<32, kCplxThreads>(task, acc, part, pcnt, &ticket)) continue;
-#pragma unroll
-    for (int mi = 0; mi < 4; ++mi) {
-      const int64_t i = m0 + wm * 32 + mi * 8 + g;
-      if (i >= b.m) continue;
-#pragma unroll
-      for (int ni = 0; ni < 2; ++ni) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int64_t j = n0 + wn * 16 + ni * 8 + 2 * t + h;
-          if (j >= b.n) continue;
-          double2 *p = C + b.offC + i + j * b.ldc;
-          const double vr = acc[(mi * 2 + ni) * 4 + h], vi = acc[(mi * 2 + ni) * 4 + 2 + h];
-          double rr = alpha.x * vr - alpha.y * vi;
-          double ri = alpha.x * vi + alpha.y * vr;
-          if (!bz) {
-            const double2 o = *p;
-            rr = fma(beta.x, o.x, fma(-beta.y, o.y, rr));
-            ri = fma(beta.x, o.y, fma(beta.y, o.x, ri));
-          }
-          *p = make_double2(rr, ri);
-        }
-      }
-    }
-  }
-}
+using LargeTile = TileCfg<double, 64, 64, 32, 32, 3, 2>;
+using SmallTile = TileCfg<double, 32, 32, 16, 16, 3, 6>;
+// Complex fragments hold twice the values, so the large tile is half as wide (212 registers; 64×64 spills
+// at the 128 registers of two CTAs).
+using LargeTileC = TileCfg<double2, 64, 32, 32, 16, 3, 2>;
+using SmallTileC = TileCfg<double2, 32, 32, 16, 16, 3, 3>;
 
 // ---- skinny blocks (n, k ≤ 16): one thread per output row, op(B) in shared memory -----------
 // Such blocks (tall-skinny GEMMs against small MPO bonds) are bound by reading op(A) and
@@ -851,32 +762,55 @@ int tkb_gemm_thin_launch(tkb_ctx *ctx, const tkb_plan *p, void *C, const void *A
 // Work decomposition of a plain GEMM: the tile shape and the tasks of every CTA.
 // - SmallTile runs while its tiles are at most 1.5 per SM: an SU(2) environment update (two products and
 // two permutes) takes 10.3 instead of 14.4 us at V dim 280, 15.9 instead of 22.8 at 870, 22.7
-// instead of 26.7 at 1816 (155 tiles), but 34.9 instead of 32.8 at 2410 (290 tiles).
+// instead of 26.7 at 1816 (155 tiles), but 34.9 instead of 32.8 at 2410 (290 tiles). Complex launches
+// keep it up to 16 tiles per SM: 142.9 instead of 162.7 us at V dim 3632 (620 tiles and 310 of
+// 64×32), but 30.6 instead of 32.1 TFLOP/s on one 2048³ block (4096 tiles).
 // - Fewer tiles than resident CTAs: the K loops of the longest tiles are cut into equal pieces of the
 //   shortest length (at least min_piece_steps K steps) whose count still fits, one task per CTA.
-// - Otherwise every CTA gets an equal share of all K steps (plus kTileCost steps per tile for its
+// - Otherwise every CTA gets an equal share of all K steps (plus tile_cost steps per tile for its
 //   epilogue), as a contiguous range of the tiles in order of falling K; a tile that a share ends in
 //   is cut there. Whole tiles alone leave CTAs idle for up to a tile each: on a U(1) effective
 //   Hamiltonian's second product (394 tiles of up to 109 steps for 296 CTAs) SMs were active for
 //   70 % of the launch. A CTA runs its cut tiles first, so their partial sums meet while it goes on.
-constexpr int kTileCost = 2;
+
+namespace {
+struct PlainKernel {
+  const void *fn;
+  int threads, bm, bn;
+  size_t smem;
+};
+template <typename CFG>
+PlainKernel plain_kernel_of() {
+  return PlainKernel{(const void *)gemm_plain_kernel<CFG>, CFG::THREADS, CFG::BM, CFG::BN, CFG::SMEM};
+}
+PlainKernel plain_kernel(bool cplx, bool small) {
+  return cplx ? (small ? plain_kernel_of<SmallTileC>() : plain_kernel_of<LargeTileC>())
+              : (small ? plain_kernel_of<SmallTile>() : plain_kernel_of<LargeTile>());
+}
+template <typename CFG>
+cudaError_t plain_launch(tkb_ctx *ctx, const tkb_plan *p, void *C, const void *A, const void *B, tkb_scalar alpha,
+                         tkb_scalar beta, int base_ok) {
+  using E = typename CFG::E;
+  // the shared-memory limit was raised when the plan queried the kernel's occupancy
+  return launch_pdl(gemm_plain_kernel<CFG>, dim3(p->pgrid), dim3(CFG::THREADS), CFG::SMEM, ctx->stream, p->blocks,
+                    (const PTask *)p->ptasks, (const int32_t *)p->pstart, (E *)C, (const E *)A, (const E *)B,
+                    CDbl{alpha.re, alpha.im}, CDbl{beta.re, beta.im}, p->part, p->pcnt, base_ok);
+}
+}  // namespace
 
 int tkb_gemm_plain_prepare(tkb_ctx *ctx, tkb_plan *p) {
   const bool cplx = p->dtype == TKB_C128;
   int64_t small_tiles = 0;
   for (const GBlock &b : p->hblocks)
     if (!b.skinny) small_tiles += ((b.m + 31) / 32) * ((b.n + 31) / 32);
-  const bool small = !cplx && small_tiles * 2 <= (int64_t)ctx->num_sms * 3;
-  p->tile_m = p->tile_n = small ? SmallTile::BM : BM;
-  const void *kfn = cplx    ? (const void *)gemm_c128_kernel
-                    : small ? (const void *)gemm_f64_kernel<SmallTile>
-                            : (const void *)gemm_f64_kernel<LargeTile>;
-  const int threads = cplx ? kCplxThreads : small ? SmallTile::THREADS : LargeTile::THREADS;
-  const size_t smem = cplx ? sizeof(SmemC) : small ? SmallTile::SMEM : LargeTile::SMEM;
-  const int tm = p->tile_m, tn = p->tile_n;
-  // a piece's partial sums cost as much as twice as many steps of the smaller tile
-  const int min_steps = p->min_piece_steps * (small ? 2 : 1);
-  const int per_sm = tkb_occupancy(ctx->device, kfn, threads, smem);
+  p->plain_small = cplx ? small_tiles <= (int64_t)ctx->num_sms * 16 : small_tiles * 2 <= (int64_t)ctx->num_sms * 3;
+  const PlainKernel pk = plain_kernel(cplx, p->plain_small);
+  const int tm = pk.bm, tn = pk.bn;
+  // a piece's partial sums cost as much as twice as many steps of the smaller tile; a complex step is
+  // four real ones
+  const int min_steps = std::max(1, p->min_piece_steps * (p->plain_small ? 2 : 1) / (cplx ? 4 : 1));
+  const int tile_cost = cplx ? 1 : 2;
+  const int per_sm = tkb_occupancy(ctx->device, pk.fn, pk.threads, pk.smem);
   if (per_sm <= 0) return tkb_set_error(ctx, TKB_ERR_CUDA, "plain GEMM: occupancy query failed");
   const int64_t slots = (int64_t)ctx->num_sms * per_sm;
   std::vector<GTile> tiles;
@@ -926,7 +860,7 @@ int tkb_gemm_plain_prepare(tkb_ctx *ctx, tkb_plan *p) {
   } else {
     lists.resize((size_t)slots);
     std::vector<std::vector<PTask>> whole((size_t)slots);
-    const double share = (double)(total + kTileCost * nt) / (double)slots;
+    const double share = (double)(total + tile_cost * nt) / (double)slots;
     double pos = 0.0;  // steps given out so far
     int64_t cta = 0;
     for (int64_t i = 0; i < nt; ++i) {
@@ -950,7 +884,7 @@ int tkb_gemm_plain_prepare(tkb_ctx *ctx, tkb_plan *p) {
         pos += (double)head;
         if (kb >= nks[i]) break;
       }
-      pos += kTileCost;
+      pos += tile_cost;
       const int ks = (int)cut.size();
       if (ks == 1) {
         whole[cut[0].first].push_back(cut[0].second);
@@ -1008,23 +942,14 @@ int tkb_gemm_launch(tkb_ctx *ctx, const tkb_plan *p, void *C, const void *A, con
   if (p->dtype == TKB_F64) {
     if (alpha.im != 0.0 || beta.im != 0.0)
       return tkb_set_error(ctx, TKB_ERR_ARG, "complex scalar with real data");
-    const bool small = p->tile_m == SmallTile::BM;
-    const auto kfn = small ? gemm_f64_kernel<SmallTile> : gemm_f64_kernel<LargeTile>;
-    const size_t smem = small ? SmallTile::SMEM : LargeTile::SMEM;
-    TKB_CUDA_TRY(ctx, cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int base_ok = (((uintptr_t)A & 15) == 0 ? 1 : 0) | (((uintptr_t)B & 15) == 0 ? 2 : 0);
-    TKB_CUDA_TRY(ctx, launch_pdl(kfn, dim3(p->pgrid), dim3(small ? SmallTile::THREADS : LargeTile::THREADS), smem, ctx->stream, p->blocks,
-                                 (const PTask *)p->ptasks, (const int32_t *)p->pstart, (double *)C, (const double *)A,
-                                 (const double *)B, alpha.re, beta.re, p->part, p->pcnt, base_ok));
+    TKB_CUDA_TRY(ctx, p->plain_small ? plain_launch<SmallTile>(ctx, p, C, A, B, alpha, beta, base_ok)
+                                     : plain_launch<LargeTile>(ctx, p, C, A, B, alpha, beta, base_ok));
   } else {
     if ((((uintptr_t)A | (uintptr_t)B | (uintptr_t)C) & 15) != 0)
       return tkb_set_error(ctx, TKB_ERR_ARG, "ComplexF64 data must be 16-byte aligned");
-    const size_t smem = sizeof(SmemC);
-    TKB_CUDA_TRY(ctx, cudaFuncSetAttribute(gemm_c128_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    TKB_CUDA_TRY(ctx, launch_pdl(gemm_c128_kernel, dim3(p->pgrid), dim3(kCplxThreads), smem, ctx->stream, p->blocks,
-                                 (const PTask *)p->ptasks, (const int32_t *)p->pstart, (double2 *)C, (const double2 *)A,
-                                 (const double2 *)B, CDbl{alpha.re, alpha.im}, CDbl{beta.re, beta.im}, p->part,
-                                 p->pcnt));
+    TKB_CUDA_TRY(ctx, p->plain_small ? plain_launch<SmallTileC>(ctx, p, C, A, B, alpha, beta, 0)
+                                     : plain_launch<LargeTileC>(ctx, p, C, A, B, alpha, beta, 0));
   }
   ctx->launches++;
   TKB_CUDA_TRY(ctx, cudaGetLastError());

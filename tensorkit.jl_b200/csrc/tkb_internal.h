@@ -256,7 +256,7 @@ struct tkb_plan {
   void *sjobs = nullptr;        // slicing tasks (block, operand, rows)
   int64_t nsrows = 0;           // slicing tasks
   int64_t nsctasks = 0;         // of which the first are staged (one CTA each)
-  int tile_m = 64, tile_n = 64;
+  bool plain_small = false;     // plain precision: 32×32 tiles
   // split-K knobs (tkb_gemm_plan_create_tuned): pieces per tile at most, K steps per piece at least
   int max_pieces = 8, min_piece_steps = 4;
 };

@@ -64,6 +64,11 @@ int tkb_version(void);
 int tkb_ctx_create(int device, void *stream, size_t workspace_bytes, tkb_ctx **out);
 int tkb_ctx_destroy(tkb_ctx *ctx);
 int tkb_ctx_set_stream(tkb_ctx *ctx, void *stream);
+/* Stream ordering for callers whose data lives on a stream of their own: later work of the context
+ * waits for what `stream` holds now (tkb_ctx_after), later work on `stream` waits for what the context
+ * has enqueued (tkb_ctx_before). Nothing to do when `stream` is the context's own. */
+int tkb_ctx_after(tkb_ctx *ctx, void *stream);
+int tkb_ctx_before(tkb_ctx *ctx, void *stream);
 /* Waits for the context's stream. Returns TKB_ERR_TIMEOUT (and clears the record) when a
  * bounded device wait of an earlier launch on this context gave up; tkb_last_error names it. */
 int tkb_ctx_synchronize(tkb_ctx *ctx);

@@ -71,14 +71,22 @@ int tkb_ctx_create(int device, void *stream, size_t workspace_bytes, tkb_ctx **o
     delete ctx;
     return tkb_set_error(nullptr, TKB_ERR_OOM, "counter allocation failed");
   }
+  e = cudaEventCreateWithFlags(&ctx->order, cudaEventDisableTiming);
+  if (e != cudaSuccess) {
+    cudaFree(ctx->counters);
+    delete ctx;
+    return tkb_set_error(nullptr, TKB_ERR_CUDA, cudaGetErrorString(e));
+  }
   e = cudaHostAlloc((void **)&ctx->host_res, kHostSlots * 2 * sizeof(double), cudaHostAllocMapped | cudaHostAllocPortable);
   if (e != cudaSuccess) {
+    cudaEventDestroy(ctx->order);
     cudaFree(ctx->counters);
     delete ctx;
     return tkb_set_error(nullptr, TKB_ERR_OOM, "result buffer allocation failed");
   }
   const size_t ws = std::max<size_t>(workspace_bytes, 1 << 20);
   if (tkb_ensure_workspace(ctx, ws) != TKB_OK) {
+    cudaEventDestroy(ctx->order);
     cudaFree(ctx->counters);
     cudaFreeHost(ctx->host_res);
     delete ctx;
@@ -92,6 +100,7 @@ int tkb_ctx_destroy(tkb_ctx *ctx) {
   if (!ctx) return TKB_OK;
   cudaStreamSynchronize(ctx->stream);
   cudaFree(ctx->ws);
+  cudaEventDestroy(ctx->order);
   cudaFree(ctx->counters);
   cudaFreeHost(ctx->host_res);
   delete ctx;
@@ -103,6 +112,31 @@ int tkb_ctx_set_stream(tkb_ctx *ctx, void *stream) {
   if (ctx->in_capture) return tkb_set_error(ctx, TKB_ERR_ARG, "cannot change stream during capture");
   ctx->stream = (cudaStream_t)stream;
   return TKB_OK;
+}
+
+// `later` waits for what `earlier` holds now
+static int order_streams(tkb_ctx *ctx, cudaStream_t earlier, cudaStream_t later) {
+  if (earlier == later) return TKB_OK;
+  std::lock_guard<std::mutex> lock(ctx->order_mu);
+  // the default stream is the current device's
+  int prev = ctx->device;
+  cudaError_t e = cudaGetDevice(&prev);
+  if (e == cudaSuccess && prev != ctx->device) e = cudaSetDevice(ctx->device);
+  if (e == cudaSuccess) e = cudaEventRecord(ctx->order, earlier);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(later, ctx->order, 0);
+  if (prev != ctx->device) cudaSetDevice(prev);
+  if (e != cudaSuccess) return tkb_set_error(ctx, TKB_ERR_CUDA, std::string("stream order: ") + cudaGetErrorString(e));
+  return TKB_OK;
+}
+
+int tkb_ctx_after(tkb_ctx *ctx, void *stream) {
+  if (!ctx) return tkb_set_error(nullptr, TKB_ERR_ARG, "null context");
+  return order_streams(ctx, (cudaStream_t)stream, ctx->stream);
+}
+
+int tkb_ctx_before(tkb_ctx *ctx, void *stream) {
+  if (!ctx) return tkb_set_error(nullptr, TKB_ERR_ARG, "null context");
+  return order_streams(ctx, ctx->stream, (cudaStream_t)stream);
 }
 
 // ctx->counters[kErrSlot]: codes of bounded device waits that gave up (kernels set it with

@@ -5,6 +5,7 @@
 #include <atomic>
 #include <cstdint>
 #include <cstdio>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -24,6 +25,10 @@ struct tkb_ctx {
   // doubles), and the bit mask of the slots that calls in progress hold
   double *host_res = nullptr;
   std::atomic<uint64_t> host_busy{0};
+  // event of tkb_ctx_after / tkb_ctx_before: recorded on one stream and waited for on the other under
+  // the lock, so that threads do not re-record it between the two
+  cudaEvent_t order = nullptr;
+  std::mutex order_mu;
   int64_t launches = 0;
   std::string err;
   cudaGraph_t capturing = nullptr;

@@ -30,7 +30,7 @@ EXPORTS = [
     "tkb_trace_table_destroy", "tkb_tracetransform", "tkb_gemm_plan_create", "tkb_gemm_plan_create_tuned",
     "tkb_gemm_plan_destroy", "tkb_gemm_plan_info", "tkb_gemm_plan_slices", "tkb_grouped_gemm",
     "tkb_rplan_create",
-    "tkb_rplan_destroy", "tkb_reduce", "tkb_reduce_async", "tkb_reduce_noalloc", "tkb_axpby",
+    "tkb_rplan_destroy", "tkb_reduce", "tkb_reduce_async", "tkb_reduce_noalloc", "tkb_axpby", "tkb_ctx_after", "tkb_ctx_before",
     "tkb_graph_begin", "tkb_graph_end",
     "tkb_graph_launch", "tkb_graph_destroy",
 ]
@@ -94,6 +94,8 @@ def _declare(lib):
         "tkb_ctx_destroy": ([vp], C.c_int),
         "tkb_ctx_set_stream": ([vp, vp], C.c_int),
         "tkb_ctx_synchronize": ([vp], C.c_int),
+        "tkb_ctx_after": ([vp, vp], C.c_int),
+        "tkb_ctx_before": ([vp, vp], C.c_int),
         "tkb_selftest_bounded_wait": ([vp, i64], C.c_int),
         "tkb_ctx_launch_count": ([vp, P(i64)], C.c_int),
         "tkb_last_error": ([vp], C.c_char_p),

@@ -69,9 +69,10 @@ class _LRU(OrderedDict):
         self.on_evict = on_evict
 
     def get_or(self, key, make):
-        if key in self:
+        v = self.get(key)
+        if v is not None:
             self.move_to_end(key)
-            return self[key]
+            return v
         v = make()
         self[key] = v
         if len(self) > self.maxsize:
@@ -211,6 +212,11 @@ class Context:
         self.device = device
         self.torch_device = torch.device("cuda", device)
         self.stream = torch.cuda.Stream(device=self.torch_device)
+        self.stream_handle = self.stream.cuda_stream
+        # handle of torch's current stream on a device, without the Stream object around it where torch
+        # gives it
+        self.raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+            lambda d: torch.cuda.current_stream(d).cuda_stream)
         h = C.c_void_p()
         L.check(self.lib.tkb_ctx_create(device, C.c_void_p(self.stream.cuda_stream),
                                         workspace_bytes, C.byref(h)))
@@ -218,6 +224,9 @@ class Context:
         self.tables = _LRU(_DEFAULT_CACHE, lambda t: t.free())
         self.plans = _LRU(_DEFAULT_CACHE, lambda p: p.free())
         self.rplans = _LRU(_DEFAULT_CACHE, lambda p: p.free())
+        # lowered calls by structure (spaces, index tuples, scalar types): which transforms and which GEMM a
+        # call runs; they refer to entries of the caches above, which may be freed under them
+        self.recipes = _LRU(_DEFAULT_CACHE)
 
     def synchronize(self):
         L.check(self.lib.tkb_ctx_synchronize(self.handle), self.handle)
@@ -228,6 +237,7 @@ class Context:
         return v.value
 
     def empty_caches(self):
+        self.recipes.clear()
         for cache in (self.tables, self.plans, self.rplans):
             for v in cache.values():
                 v.free()

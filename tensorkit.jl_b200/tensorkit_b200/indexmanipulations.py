@@ -57,6 +57,9 @@ def dtype_code(t):
     raise TypeError(f"unsupported dtype {t.dtype}; the path computes in float64/complex128")
 
 
+_ONE, _ZERO = L.tkb_scalar(1.0, 0.0), L.tkb_scalar(0.0, 0.0)
+
+
 def _scalar(x):
     x = complex(x)
     return L.tkb_scalar(x.real, x.imag)
@@ -99,41 +102,45 @@ def add_transform_(tdst: TensorMap, tsrc, p, table: DeviceTable, alpha=1.0, beta
     conj = 1 if (isinstance(tsrc, AdjointTensorMap) and tsrc.is_complex()) else 0
     if LAUNCH_LOG is not None:
         LAUNCH_LOG.append(("transform", table, tdst, tsrc, complex(alpha), complex(beta), conj))
-    _sync_in(ctx, tdst, tsrc)
-    L.check(ctx.lib.tkb_treetransform(ctx.handle, table.handle, code,
-                                      C.c_void_p(tdst.data.data_ptr()),
-                                      C.c_void_p(tsrc.data.data_ptr()),
+    _sync_in(ctx)
+    L.check(ctx.lib.tkb_treetransform(ctx.handle, table.handle, code, tdst.data.data_ptr(), tsrc.data.data_ptr(),
                                       _scalar(alpha), _scalar(beta), conj), ctx.handle)
     _sync_out(ctx, tdst)
     return tdst
 
 
-def _sync_in(ctx, *ts):
+def _current_stream(ctx) -> int:
+    """Handle of torch's current stream on the context's device."""
+    return ctx.raw_stream(ctx.device)
+
+
+def _sync_in(ctx):
     """Order the library stream after the torch current stream (data producers)."""
-    import torch
-    cur = torch.cuda.current_stream(ctx.torch_device)
-    if cur.cuda_stream != ctx.stream.cuda_stream:
-        ctx.stream.wait_stream(cur)
+    cur = _current_stream(ctx)
+    if cur != ctx.stream_handle:
+        L.check(ctx.lib.tkb_ctx_after(ctx.handle, cur), ctx.handle)
 
 
 def _sync_out(ctx, *ts):
-    import torch
-    cur = torch.cuda.current_stream(ctx.torch_device)
-    if cur.cuda_stream != ctx.stream.cuda_stream:
-        cur.wait_stream(ctx.stream)
+    cur = _current_stream(ctx)
+    if cur != ctx.stream_handle:
+        L.check(ctx.lib.tkb_ctx_before(ctx.handle, cur), ctx.handle)
         for t in ts:
             t.data.record_stream(ctx.stream)
+
+
+def _braid_table(ctx, tdst_space, tsrc, p, levels):
+    lv = tuple(levels)
+    n1 = tsrc.numout()
+    return device_table(ctx, tdst_space, tsrc, p, (lv[:n1], lv[n1:]))
 
 
 def braid_(tdst: TensorMap, tsrc, p, levels, alpha=1.0, beta=0.0):
     p = _norm_p(p)
     if tsrc.space.permute(p) != tdst.space:
         raise SpaceMismatch(f"tsrc = {tsrc.space}, tdst = {tdst.space}, p = {p}")
-    lv = tuple(levels)
-    l1 = tuple(lv[i - 1] for i in tsrc.codomainind())
-    l2 = tuple(lv[i - 1] for i in tsrc.domainind())
     ctx = get_context(tdst.data.device.index)
-    table = device_table(ctx, tdst.space, tsrc, p, (l1, l2))
+    table = _braid_table(ctx, tdst.space, tsrc, p, levels)
     return add_transform_(tdst, tsrc, p, table, alpha, beta)
 
 

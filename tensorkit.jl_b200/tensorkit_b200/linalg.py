@@ -159,9 +159,8 @@ def mul_(tC: TensorMap, tA, tB, alpha=1.0, beta=0.0, prec=None, slices=None):
     if _im.LAUNCH_LOG is not None:
         _im.LAUNCH_LOG.append(("gemm", plan, tC, tA, tB, complex(alpha), complex(beta)))
     _sync_in(ctx)
-    L.check(ctx.lib.tkb_grouped_gemm(ctx.handle, plan.handle, C.c_void_p(tC.data.data_ptr()),
-                                     C.c_void_p(tA.data.data_ptr()), C.c_void_p(tB.data.data_ptr()),
-                                     _scalar(alpha), _scalar(beta)), ctx.handle)
+    L.check(ctx.lib.tkb_grouped_gemm(ctx.handle, plan.handle, tC.data.data_ptr(), tA.data.data_ptr(),
+                                     tB.data.data_ptr(), _scalar(alpha), _scalar(beta)), ctx.handle)
     _sync_out(ctx, tC)
     return tC
 
@@ -174,16 +173,18 @@ def compose(tA, tB):
 
 
 def _rplan(ctx, key, segs, length):
-    return ctx.rplans.get_or(key, lambda: ReducePlan(ctx, segs, length))
+    """The reduction plan of a structure; `segs()` lists its segments."""
+    return ctx.rplans.get_or(key, lambda: ReducePlan(ctx, segs(), length))
+
+
+_Pair = C.c_double * 2
 
 
 def _reduce(ctx, plan, kind, x, y=None):
-    import numpy as np
-    out = np.zeros(2)
+    out = _Pair()
     _sync_in(ctx)
-    L.check(ctx.lib.tkb_reduce(ctx.handle, plan.handle, kind, dtype_code(x),
-                               C.c_void_p(x.data_ptr()), C.c_void_p(y.data_ptr() if y is not None else 0),
-                               out.ctypes.data_as(C.POINTER(C.c_double))), ctx.handle)
+    L.check(ctx.lib.tkb_reduce(ctx.handle, plan.handle, kind, dtype_code(x), x.data_ptr(),
+                               y.data_ptr() if y is not None else None, out), ctx.handle)
     return out
 
 
@@ -201,7 +202,7 @@ def norm(t) -> float:
     data, W, _ = _tensor_data_space(t)
     _check_device(t)
     ctx = get_context(data.device.index)
-    plan = _rplan(ctx, ("norm", W), _block_segments(W), data.numel())
+    plan = _rplan(ctx, ("norm", W), lambda: _block_segments(W), data.numel())
     r = _reduce(ctx, plan, L.TKB_NORM2, data)
     return math.sqrt(max(r[0], 0.0))
 
@@ -214,7 +215,7 @@ def inner(tx, ty):
         raise NotImplementedError("inner of lazy adjoints: materialise with permute first")
     _check_device(tx, ty)
     ctx = get_context(tx.data.device.index)
-    plan = _rplan(ctx, ("norm", tx.space), _block_segments(tx.space), tx.data.numel())
+    plan = _rplan(ctx, ("norm", tx.space), lambda: _block_segments(tx.space), tx.data.numel())
     r = _reduce(ctx, plan, L.TKB_INNER, tx.data, ty.data)
     return complex(r[0], r[1]) if tx.is_complex() else float(r[0])
 
@@ -228,8 +229,8 @@ def tr(t):
     data, W, isadj = _tensor_data_space(t)
     _check_device(t)
     ctx = get_context(data.device.index)
-    segs = [(a, d1, d1 + 1, float(c.dim())) for c, ((d1, d2), (a, _)) in blockstructure(W).items()]
-    plan = _rplan(ctx, ("tr", W), segs, data.numel())
+    plan = _rplan(ctx, ("tr", W), lambda: [(a, d1, d1 + 1, float(c.dim()))
+                                           for c, ((d1, d2), (a, _)) in blockstructure(W).items()], data.numel())
     r = _reduce(ctx, plan, L.TKB_TRACE, data)
     if data.is_complex():
         v = complex(r[0], r[1])
@@ -245,8 +246,8 @@ def _axpby(ty: TensorMap, tx: TensorMap, alpha, beta):
     code = dtype_code(ty.data)
     ctx = get_context(ty.data.device.index)
     _sync_in(ctx)
-    L.check(ctx.lib.tkb_axpby(ctx.handle, code, ty.data.numel(), C.c_void_p(ty.data.data_ptr()),
-                              C.c_void_p(tx.data.data_ptr()), _scalar(alpha), _scalar(beta)), ctx.handle)
+    L.check(ctx.lib.tkb_axpby(ctx.handle, code, ty.data.numel(), ty.data.data_ptr(), tx.data.data_ptr(),
+                              _scalar(alpha), _scalar(beta)), ctx.handle)
     _sync_out(ctx, ty)
     return ty
 

@@ -27,9 +27,21 @@ class SpaceMismatch(ValueError):
     """Raised when spaces of tensors do not match (TensorKit's `SpaceMismatch`)."""
 
 
+# One tuple object per set of sectors, so that comparing equal spaces compares identities (bounded;
+# spaces whose tuples differ as objects still compare by value)
+_KEYSETS: dict = {}
+_MAX_KEYSETS = 4096
+
+
+def _shared_keys(keys):
+    if len(_KEYSETS) >= _MAX_KEYSETS:
+        _KEYSETS.clear()
+    return _KEYSETS.setdefault(keys, keys)
+
+
 class GradedSpace:
     """⨁_c ℂ^{n_c} ⊗ R_c for sectors c of one sector type."""
-    __slots__ = ("_keys", "_degs", "dual_flag", "_unit", "_h", "_sectors", "_dimmap")
+    __slots__ = ("_keys", "_degs", "dual_flag", "_unit", "_h", "_sectors", "_dimmap", "_dual")
 
     def __init__(self, dims, dual: bool = False, unit: Sector | None = None):
         items = list(dims.items()) if isinstance(dims, dict) else list(dims)
@@ -38,7 +50,7 @@ class GradedSpace:
         for i in range(1, len(items)):
             if items[i][0] == items[i - 1][0]:
                 raise ValueError("duplicate sector in GradedSpace")
-        self._keys = tuple(c for c, _ in items)
+        self._keys = _shared_keys(tuple(c for c, _ in items))
         self._degs = tuple(d for _, d in items)
         self.dual_flag = bool(dual)
         if unit is None:
@@ -49,6 +61,7 @@ class GradedSpace:
         self._h = hash((self._keys, self._degs, self.dual_flag))
         self._sectors = tuple(c.dual() for c in self._keys) if self.dual_flag else self._keys
         self._dimmap = dict(zip(self._keys, self._degs))
+        self._dual = None
 
     # -- basic queries ----------------------------------------------------------------
     def sectors(self):
@@ -75,7 +88,12 @@ class GradedSpace:
         return range(off, off + c.dim() * self.dim(c))
 
     def dual(self) -> "GradedSpace":
-        return GradedSpace(list(zip(self._keys, self._degs)), not self.dual_flag, self._unit)
+        d = self._dual
+        if d is None:
+            d = GradedSpace(list(zip(self._keys, self._degs)), not self.dual_flag, self._unit)
+            d._dual = self
+            self._dual = d
+        return d
 
     conj = dual
 
@@ -90,8 +108,8 @@ class GradedSpace:
                            self._unit).dual()
 
     def __eq__(self, o):
-        return (isinstance(o, GradedSpace) and o._keys == self._keys and o._degs == self._degs
-                and o.dual_flag == self.dual_flag)
+        return self is o or (isinstance(o, GradedSpace) and o._h == self._h and o.dual_flag == self.dual_flag
+                             and o._degs == self._degs and o._keys == self._keys)
 
     def __hash__(self):
         return self._h
@@ -137,7 +155,8 @@ class ProductSpace:
         return iter(self.spaces)
 
     def __eq__(self, o):
-        return isinstance(o, ProductSpace) and o.spaces == self.spaces and o._unit == self._unit
+        return self is o or (isinstance(o, ProductSpace) and o._h == self._h and o.spaces == self.spaces
+                             and o._unit == self._unit)
 
     def __hash__(self):
         return self._h
@@ -241,7 +260,7 @@ def _as_product(x, unit=None) -> ProductSpace:
 
 class HomSpace:
     """Space of morphisms codomain ← domain."""
-    __slots__ = ("codomain", "domain", "_h")
+    __slots__ = ("codomain", "domain", "_h", "_dim", "_adjoint", "_selected")
 
     def __init__(self, codomain, domain, unit: Sector | None = None):
         cod = _as_product(codomain, unit)
@@ -251,6 +270,9 @@ class HomSpace:
         self.codomain = cod
         self.domain = dom
         self._h = hash((cod, dom))
+        self._dim = None       # the space is immutable: dim, adjoint and selections are kept
+        self._adjoint = None
+        self._selected = {}
 
     # -- structure ------------------------------------------------------------------
     def numout(self):
@@ -273,7 +295,8 @@ class HomSpace:
         return self.codomain[i - 1] if i <= n1 else self.domain[i - n1 - 1].dual()
 
     def __eq__(self, o):
-        return isinstance(o, HomSpace) and o.codomain == self.codomain and o.domain == self.domain
+        return self is o or (isinstance(o, HomSpace) and o._h == self._h and o.codomain == self.codomain
+                             and o.domain == self.domain)
 
     def __hash__(self):
         return self._h
@@ -285,16 +308,27 @@ class HomSpace:
         return self.codomain.dims() + self.domain.dims()
 
     def adjoint(self) -> "HomSpace":
-        return HomSpace(self.domain, self.codomain, self.unit())
+        a = self._adjoint
+        if a is None:
+            a = HomSpace(self.domain, self.codomain, self.unit())
+            a._adjoint = self
+            self._adjoint = a
+        return a
 
     def dual(self) -> "HomSpace":
         return HomSpace(self.domain.dual(), self.codomain.dual(), self.unit())
 
     def select(self, p) -> "HomSpace":
-        p1, p2 = p
-        cod = ProductSpace(tuple(self[n] for n in p1), self.unit())
-        dom = ProductSpace(tuple(self[n].dual() for n in p2), self.unit())
-        return HomSpace(cod, dom, self.unit())
+        p1, p2 = tuple(p[0]), tuple(p[1])
+        W = self._selected.get((p1, p2))
+        if W is None:
+            cod = ProductSpace(tuple(self[n] for n in p1), self.unit())
+            dom = ProductSpace(tuple(self[n].dual() for n in p2), self.unit())
+            W = HomSpace(cod, dom, self.unit())
+            if len(self._selected) >= 64:
+                self._selected.clear()
+            self._selected[(p1, p2)] = W
+        return W
 
     def permute(self, p) -> "HomSpace":
         p1, p2 = p
@@ -338,8 +372,10 @@ class HomSpace:
         return [c for c in cod.blocksectors() if dom.hasblock(c)]
 
     def dim(self) -> int:
-        from .structure import degeneracystructure
-        return degeneracystructure(self).totaldim
+        if self._dim is None:
+            from .structure import degeneracystructure
+            self._dim = degeneracystructure(self).totaldim
+        return self._dim
 
     def sectorkey(self):
         return (tuple(v.sectorhash_key() for v in self.codomain),

@@ -35,7 +35,9 @@ _ALLOC_LOG: list | None = None
 
 def new_tensor(W: HomSpace, dtype, device) -> "TensorMap":
     torch = _torch()
-    t = TensorMap(torch.empty(W.dim(), dtype=dtype, device=device), W)
+    t = TensorMap.__new__(TensorMap)  # the vector has the space's length by construction
+    t.data = torch.empty(W.dim(), dtype=dtype, device=device)
+    t.space = W
     if _ALLOC_LOG is not None:
         _ALLOC_LOG.append(t.data)
     return t

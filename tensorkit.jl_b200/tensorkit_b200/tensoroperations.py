@@ -20,11 +20,17 @@ destinations of the blockwise `mul!`.
 from __future__ import annotations
 
 import re
+from functools import lru_cache
 
-from .indexmanipulations import permute, permute_
-from .linalg import mul_
+from . import _lib as L
+from . import indexmanipulations as _im
+from . import linalg as _la
+from .backend import get_context, precision
+from .indexmanipulations import (_ONE, _ZERO, _braid_table, _current_stream, _scalar, dtype_code, permute,
+                                 permute_)
+from .linalg import gemm_plan, mul_
 from .spaces import HomSpace, SpaceMismatch
-from .tensor import AdjointTensorMap, TensorMap, new_tensor
+from .tensor import AbstractTensorMap, AdjointTensorMap, TensorMap, new_tensor
 
 __all__ = ["tensoradd_", "tensorcontract_", "tensorcontract", "contract_", "blas_contract_",
            "tensortrace_", "tensortrace", "tensortrace_structure",
@@ -133,7 +139,8 @@ def _dim(t):
     return t.space.dim() if not isinstance(t, AdjointTensorMap) else t.parent.space.dim()
 
 
-def contract_(C, A, pA, B, pB, pAB, alpha=1.0, beta=0.0):
+def _choose_order(C, A, pA, B, pB, pAB):
+    """The index order that moves the least data: (exchange A and B, pX, pY, pXY)."""
     if len(pA[1]) != len(pB[0]):
         raise IndexError("number of contracted indices does not match")
     pA1, pB1, pA2, pB2, pABp = _contract_candidates(pA, pB, pAB)
@@ -144,12 +151,16 @@ def contract_(C, A, pA, B, pB, pAB, alpha=1.0, beta=0.0):
     m3 = _memcost(dB, dA, dC, C, B, rv(pB1), A, rv(pA1), pABp)
     m4 = _memcost(dB, dA, dC, C, B, rv(pB2), A, rv(pA2), pABp)
     if min(m1, m2) <= min(m3, m4):
-        if m1 <= m2:
-            return blas_contract_(C, A, pA1, B, pB1, pAB, alpha, beta)
-        return blas_contract_(C, A, pA2, B, pB2, pAB, alpha, beta)
+        return (False, pA1, pB1, pAB) if m1 <= m2 else (False, pA2, pB2, pAB)
     if m3 <= m4:
-        return blas_contract_(C, B, rv(pB1), A, rv(pA1), pABp, alpha, beta)
-    return blas_contract_(C, B, rv(pB2), A, rv(pA2), pABp, alpha, beta)
+        return True, rv(pB1), rv(pA1), pABp
+    return True, rv(pB2), rv(pA2), pABp
+
+
+def contract_(C, A, pA, B, pB, pAB, alpha=1.0, beta=0.0):
+    swap, pX, pY, pXY = _choose_order(C, A, pA, B, pB, pAB)
+    X, Y = (B, A) if swap else (A, B)
+    return blas_contract_(C, X, pX, Y, pY, pXY, alpha, beta)
 
 
 def _alloc(W, like):
@@ -182,13 +193,154 @@ def blas_contract_(C, A, pA, B, pB, pAB, alpha=1.0, beta=0.0, plan_hook=None):
     return C
 
 
+class _Shape(AbstractTensorMap):
+    """What the lowering needs to know of a tensor that does not exist yet: space and scalar type."""
+
+    class _Data:
+        __slots__ = ("dtype",)
+
+        def __init__(self, dtype):
+            self.dtype = dtype
+
+    def __init__(self, space, dtype):
+        self.space = space
+        self.data = _Shape._Data(dtype)
+
+
+class _Recipe:
+    """A contraction lowered once per structure: the space of the result, which operands are permuted
+    first (with their device tables and spaces), the GEMM plan per precision setting, and the final
+    permute. It holds no data. Tables and plans belong to the context's caches; a recipe whose entries
+    were evicted there is made again."""
+    __slots__ = ("W", "swap", "adj", "move", "wc", "move_c", "plans")
+
+    def usable(self):
+        for m in self.move:
+            if m is not None and m[1].handle is None:
+                return False
+        return self.move_c is None or self.move_c.handle is not None
+
+
+def _make_recipe(ctx, A, pA, conjA, B, pB, conjB, pAB):
+    r = _Recipe()
+    dt = A.data.dtype
+    r.W = tensorcontract_structure(A, pA, conjA, B, pB, conjB, pAB)
+    r.adj = (bool(conjA), bool(conjB))
+    if conjA:
+        A, pA = _adjoint(A), adjointtensorindices(A, pA)
+    if conjB:
+        B, pB = _adjoint(B), adjointtensorindices(B, pB)
+    C = _Shape(r.W, dt)
+    r.swap, pX, pY, pXY = _choose_order(C, A, pA, B, pB, pAB)
+    new, moves = [], []
+    for t, p in ((B, pX), (A, pY)) if r.swap else ((A, pX), (B, pY)):
+        if _isblas(t, p):
+            new.append(t)
+            moves.append(None)
+        else:
+            W = tensoradd_structure(t, p, False)
+            conj = 1 if isinstance(t, AdjointTensorMap) and t.is_complex() else 0
+            moves.append((W, _braid_table(ctx, W, t, p, range(1, t.numind() + 1)), conj))
+            new.append(_Shape(W, dt))
+    r.move = tuple(moves)
+    X, Y = new
+    ip = _oindABinC(pXY, (X.codomainind(), X.domainind()), (Y.codomainind(), Y.domainind()))
+    r.wc = r.move_c = None
+    if not _isblas(C, ip):
+        r.wc = tensoradd_structure(C, ip, False)
+        t = _Shape(r.wc, dt)
+        r.move_c = _braid_table(ctx, r.W, t, pXY, range(1, t.numind() + 1))
+    r.plans = {}
+    return r
+
+
+def _recipe(A, pA, conjA, B, pB, conjB, pAB):
+    """The recipe of a contraction, or None where the step-by-step path has to run (operands that it
+    refuses, launches that are being recorded)."""
+    a, b = A.data, B.data
+    if not (a.is_cuda and b.is_cuda) or a.dtype != b.dtype or _im.LAUNCH_LOG is not None or _la.FLOP_LOG is not None:
+        return None, None
+    ctx = get_context(a.device.index)
+    key = (A.space, type(A), pA, conjA, B.space, type(B), pB, conjB, pAB, a.dtype)
+    r = ctx.recipes.get(key)
+    if r is None or not r.usable():
+        r = _make_recipe(ctx, A, pA, conjA, B, pB, conjB, pAB)
+        ctx.recipes.pop(key, None)
+        ctx.recipes.get_or(key, lambda: r)
+    return ctx, r
+
+
+def _run_recipe(ctx, r, C, A, B, alpha, beta, keep):
+    """Enqueue a lowered contraction. The library stream is ordered after and before the caller's once
+    for all launches; the permuted operands are allocated on the caller's stream and released after
+    that, so their memory is not reused too early. `keep`: C was passed in (its memory may belong to
+    another stream's pool)."""
+    lib, h = ctx.lib, ctx.handle
+    out = C.data
+    dtype, device = out.dtype, out.device
+    code = dtype_code(out)
+    if r.adj[0]:
+        A = _adjoint(A)
+    if r.adj[1]:
+        B = _adjoint(B)
+    ops = [B, A] if r.swap else [A, B]
+    cur = _current_stream(ctx)
+    joined = cur != ctx.stream_handle
+    rc = lib.tkb_ctx_after(h, cur) if joined else 0
+    if rc:
+        L.check(rc, h)
+    try:
+        for i, m in enumerate(r.move):
+            if m is not None:
+                t = new_tensor(m[0], dtype, device)
+                rc = lib.tkb_treetransform(h, m[1].handle, code, t.data.data_ptr(), ops[i].data.data_ptr(), _ONE,
+                                           _ZERO, m[2])
+                if rc:
+                    L.check(rc, h)
+                ops[i] = t
+        X, Y = ops
+        D = C if r.move_c is None else new_tensor(r.wc, dtype, device)
+        mode = precision()
+        plan = r.plans.get(mode)
+        if plan is None or plan.handle is None:
+            plan = gemm_plan(ctx, D, X, Y)
+            if len(r.plans) >= 16:
+                r.plans.clear()
+            r.plans[mode] = plan
+        al = _ONE if alpha == 1.0 else _scalar(alpha)
+        be = _ZERO if beta == 0.0 else _scalar(beta)
+        if r.move_c is None:
+            rc = lib.tkb_grouped_gemm(h, plan.handle, out.data_ptr(), X.data.data_ptr(), Y.data.data_ptr(), al, be)
+        else:
+            rc = lib.tkb_grouped_gemm(h, plan.handle, D.data.data_ptr(), X.data.data_ptr(), Y.data.data_ptr(), _ONE,
+                                      _ZERO)
+            if rc == 0:
+                rc = lib.tkb_treetransform(h, r.move_c.handle, code, out.data_ptr(), D.data.data_ptr(), al, be, 0)
+        if rc:
+            L.check(rc, h)
+    finally:
+        if joined:
+            rc = lib.tkb_ctx_before(h, cur)
+            if keep:
+                out.record_stream(ctx.stream)
+            if rc:
+                L.check(rc, h)
+    return C
+
+
+def _pair(p):
+    return (tuple(p[0]), tuple(p[1]))
+
+
 def tensorcontract_(C, A, pA, conjA, B, pB, conjB, pAB, alpha=1.0, beta=0.0):
-    pA = (tuple(pA[0]), tuple(pA[1]))
-    pB = (tuple(pB[0]), tuple(pB[1]))
+    pA, pB = _pair(pA), _pair(pB)
     pABc = _canonicalize(pAB, C)
-    W = tensorcontract_structure(A, pA, conjA, B, pB, conjB, pABc)
+    ctx, r = _recipe(A, pA, conjA, B, pB, conjB, pABc)
+    W = r.W if r is not None else tensorcontract_structure(A, pA, conjA, B, pB, conjB, pABc)
     if W != C.space:
         raise SpaceMismatch(f"incompatible spaces for tensorcontract: {W} ≠ {C.space}")
+    if r is not None and C.data.dtype == A.data.dtype and C.data.device == A.data.device:
+        return _run_recipe(ctx, r, C, A, B, alpha, beta, True)
     if conjA:
         A, pA = _adjoint(A), adjointtensorindices(A, pA)
     if conjB:
@@ -197,6 +349,10 @@ def tensorcontract_(C, A, pA, conjA, B, pB, conjB, pAB, alpha=1.0, beta=0.0):
 
 
 def tensorcontract(A, pA, conjA, B, pB, conjB, pAB, alpha=1.0):
+    pA, pB, pAB = _pair(pA), _pair(pB), _pair(pAB)
+    ctx, r = _recipe(A, pA, conjA, B, pB, conjB, pAB)
+    if r is not None:
+        return _run_recipe(ctx, r, _alloc(r.W, A), A, B, alpha, 0.0, False)
     W = tensorcontract_structure(A, pA, conjA, B, pB, conjB, pAB)
     C = _alloc(W, A)
     return tensorcontract_(C, A, pA, conjA, B, pB, conjB, pAB, alpha, 0.0)
@@ -217,6 +373,12 @@ def _labels(s):
 
 def parse_tensor_expr(expr):
     """Parse 'C[a;b] := A[a;c]*conj(B[c;b])' → (lhs_name, (cod, dom), op, [(name, labels, conj)])."""
+    lhs_name, lhs, op, factors = _parsed(expr)
+    return lhs_name, lhs, op, list(factors)
+
+
+@lru_cache(maxsize=1024)
+def _parsed(expr):
     for op in (":=", "+=", "="):
         if op in expr:
             lhs, rhs = expr.split(op, 1)
@@ -238,7 +400,7 @@ def parse_tensor_expr(expr):
             raise ValueError(f"unbalanced conj in {part!r}")
         c, d = _labels(mm.group(3))
         factors.append((mm.group(2), c + d, conj))
-    return lhs_name, (lcod, ldom), op, factors
+    return lhs_name, (lcod, ldom), op, tuple(factors)
 
 
 def tensortrace_structure(A, p, conjA=False) -> HomSpace:
@@ -268,6 +430,11 @@ def tensortrace(A, p, q, conjA=False, alpha=1.0):
 def _pairwise_steps(lhs, factors):
     """Plan of pairwise contractions: list of (labelsA, conjA, labelsB, conjB, pA, pB, pAB,
     out_labels, is_final)."""
+    return list(_steps((tuple(lhs[0]), tuple(lhs[1])), tuple((n, tuple(lab), cj) for n, lab, cj in factors)))
+
+
+@lru_cache(maxsize=1024)
+def _steps(lhs, factors):
     steps = []
     cur_labels, cur_conj = factors[0][1], factors[0][2]
     n = len(factors)
@@ -295,6 +462,7 @@ def _pairwise_steps(lhs, factors):
     return steps
 
 
+@lru_cache(maxsize=1024)
 def _trace_labels(labels):
     """Leg pairs (q₁, q₂) of the labels repeated within one factor (1-based)."""
     reps = [l for l in dict.fromkeys(labels) if labels.count(l) > 1]
@@ -309,9 +477,10 @@ def _trace_labels(labels):
 def _pretrace(A, labels, conj):
     """Trace the labels a factor repeats (TensorOperations traces a factor before it enters
     a contraction); returns the traced tensor and its remaining labels."""
+    labels = tuple(labels)
     reps, q = _trace_labels(labels)
     if not reps:
-        return A, tuple(labels), conj
+        return A, labels, conj
     nout = A.numout()
     keep = [i for i, l in enumerate(labels) if l not in reps]
     p = (tuple(i + 1 for i in keep if i < nout), tuple(i + 1 for i in keep if i >= nout))
@@ -330,7 +499,7 @@ def tensor(expr, out=None, alpha=1.0, **tensors):
         lcod, ldom = lhs
         pA = (tuple(labels.index(l) + 1 for l in lcod), tuple(labels.index(l) + 1 for l in ldom))
         beta = 1.0 if op == "+=" else 0.0
-        reps, q = _trace_labels(labels)
+        reps, q = _trace_labels(tuple(labels))
         if out is None:
             out = _alloc(tensoradd_structure(A, pA, conj), A)
         if reps:
@@ -343,15 +512,11 @@ def tensor(expr, out=None, alpha=1.0, **tensors):
     for i, (la, ca, lb, cb, pA, pB, pAB, outl, final) in enumerate(steps):
         B = pre[i + 1][0]
         if final:
-            W = tensorcontract_structure(cur, pA, ca, B, pB, cb, pAB)
             if out is None:
                 if op != ":=":
                     raise ValueError("'=' and '+=' need an existing output tensor")
-                out = _alloc(W, cur)
-                beta = 0.0
-            else:
-                beta = 1.0 if op == "+=" else 0.0
-            tensorcontract_(out, cur, pA, ca, B, pB, cb, pAB, alpha, beta)
+                return tensorcontract(cur, pA, ca, B, pB, cb, pAB, alpha)
+            tensorcontract_(out, cur, pA, ca, B, pB, cb, pAB, alpha, 1.0 if op == "+=" else 0.0)
             return out
         cur = tensorcontract(cur, pA, ca, B, pB, cb, pAB, 1.0)
     raise AssertionError("unreachable")

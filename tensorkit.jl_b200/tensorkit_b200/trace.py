@@ -169,10 +169,9 @@ def trace_permute_(tdst: TensorMap, tsrc, p, q, alpha=1.0, beta=0.0):
     conj = 1 if (isinstance(tsrc, AdjointTensorMap) and tsrc.is_complex()) else 0
     if IM.LAUNCH_LOG is not None:
         IM.LAUNCH_LOG.append(("trace", table, tdst, tsrc, complex(alpha), complex(beta), conj))
-    _sync_in(ctx, tdst, tsrc)
+    _sync_in(ctx)
     L.check(ctx.lib.tkb_tracetransform(ctx.handle, table.handle, dtype_code(tdst.data),
-                                       C.c_void_p(tdst.data.data_ptr()),
-                                       C.c_void_p(tsrc.data.data_ptr()),
+                                       tdst.data.data_ptr(), tsrc.data.data_ptr(),
                                        _scalar(alpha), _scalar(beta), conj), ctx.handle)
     _sync_out(ctx, tdst)
     return tdst

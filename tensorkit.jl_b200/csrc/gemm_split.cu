@@ -110,6 +110,8 @@ struct SliceTask {  // one entry per task, with every block field the task needs
   int32_t k;        // K of the block (source values per row)
   int32_t kpad;     // padded K of the slices
   int32_t conj;     // 1: conjugate the values (op = C)
+  int32_t lr;       // staged tasks: log2 of the row slots (nrows rounded up to a power of two)
+  int32_t pad;
 };
 
 constexpr int kTaskPieces = 32;  // pieces per slicing task the planner aims at (one pass of a warp)
@@ -1423,13 +1425,24 @@ __global__ void __launch_bounds__(kFusedThreads, 1) gemm_split_fused_kernel(cons
 }
 
 // Staged slicing task, run by the whole CTA (every thread calls): nrows whole rows of one operand
-// are copied into shared memory with cp.async (consecutive threads take consecutive addresses:
-// along the rows when the rows are contiguous in memory, along K otherwise), so a task costs one
-// memory round trip. Row maxima and sums of squares then come from shared memory (one warp per
-// row), and every thread slices pieces of 16 real (8 complex) K values out of it. A stage row
-// holds kfull values plus one padding value per piece (fewer bank conflicts between pieces).
+// are brought into shared memory (consecutive threads take consecutive addresses: along the
+// rows when the rows are contiguous in memory, along K otherwise), so a task costs one memory round
+// trip, then every thread slices pieces of 16 real (8 complex) K values out of it.
+//   rows contiguous: a thread keeps one row (the row slots are a power of two), so the row's maximum and
+//     sum of squares come from the loaded values on their way into shared memory;
+//   K contiguous: cp.async copies, then 8, 16 or 32 lanes per row read the statistics back, as many as
+//     give every warp work.
+// Pieces go to the threads rows first: the 16-byte digits of neighbouring rows are neighbours in the
+// slice layout, so a store covers whole sectors (a thread per piece of one row left half of each unused).
+// A stage row holds kfull values plus one padding value per piece and one more, which keeps rows and
+// pieces on different banks. Slicing the operands of a U(1) effective Hamiltonian's second product
+// (11.6 M values, K up to 1736) takes
+// 67 us (107 with tasks of 3 - 6 rows, one warp on the statistics and two CTAs per SM), of the first product (3.7 M
+// values, K up to 256) 25 us (36).
 constexpr int kStageBytes = 48 * 1024;  // shared memory of one staged task
-constexpr int kStagedRowsMax = 64;      // rows of one staged task
+constexpr int kStagedRowsMax = 64;       // rows of one staged task
+// elements of a stage row of kfull values in pieces of LK
+__host__ __device__ __forceinline__ int64_t stage_row(int64_t kfull, int lk) { return kfull + kfull / lk + 1; }
 template <typename T>
 __device__ __forceinline__ void cp_async_elem(T *dst, const T *src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(smem_u32(dst)), "l"(src), "n"(sizeof(T))
@@ -1437,7 +1450,8 @@ __device__ __forceinline__ void cp_async_elem(T *dst, const T *src) {
 }
 template <int S, bool CPLX, int NT>
 __device__ __forceinline__ void slice_staged(const SliceTask &task, const void *Xv, int8_t *ws, unsigned long long *bst,
-                                             void *stage_v, int *rexp, unsigned long long *wstat) {
+                                             void *stage_v, int *rexp, double *rmax, double *rsum,
+                                             unsigned long long *wstat) {
   using T = typename SrcVal<CPLX>::T;
   constexpr int LK = CPLX ? 8 : 16;
   constexpr int NW = NT / 32;
@@ -1446,63 +1460,113 @@ __device__ __forceinline__ void slice_staged(const SliceTask &task, const void *
   const int op = task.operand;
   const int64_t kfull = CPLX ? task.kpad / 2 : task.kpad;
   const int nchunk = (int)(kfull / LK);
-  const int stride = (int)(kfull + kfull / LK);  // stage row length in elements (with padding)
-  const int nrows = task.nrows;
+  const int stride = (int)stage_row(kfull, LK);
+  const int nrows = task.nrows, lr = task.lr, R = 1 << lr;
   const bool rowc = task.rs == 1;
   T *stage = reinterpret_cast<T *>(stage_v);
-  const T *X = reinterpret_cast<const T *>(Xv);
+  const T *X = reinterpret_cast<const T *>(Xv) + task.xoff;
   const T z = zero_of(T{});
-  // 1. copy the rows in (zeros past k and for rows past the operand)
-  const int total = nrows * (int)kfull;
-  // element q = tid, tid + NT, … as (r, c): the fast index (r for row-contiguous, c otherwise)
-  // steps by NT mod fast with a carry into the slow one (no division per element)
-  const int fast = rowc ? nrows : (int)kfull;
-  const int fstep = NT % fast, sstep = NT / fast;
-  int fi = tid % fast, si = tid / fast;
-#pragma unroll 1
-  for (int q = tid; q < total; q += NT) {
-    const int r = rowc ? fi : si, c = rowc ? si : fi;
-    fi += fstep;
-    si += sstep;
-    if (fi >= fast) {
-      fi -= fast;
-      ++si;
-    }
-    T *dst = stage + r * stride + c + c / LK;
-    const int64_t rr = task.r0 + r;
-    if (c < task.k && rr < task.msrc) cp_async_elem(dst, X + task.xoff + rr * task.rs + (int64_t)c * task.ks);
-    else *dst = z;
-  }
-  asm volatile("cp.async.commit_group;\ncp.async.wait_all;\n" ::: "memory");
-  __syncthreads();
-  if (tid == 0) TL_STAMP(3);
-  // 2. row maxima, sums of squares, exponents: eight lanes per row, four rows per warp at a time
-  unsigned ebm = 0u;
-  double nrm = 0.0;
-  int32_t *ex = reinterpret_cast<int32_t *>(ws + task.ws_e);
-  const int sub = lane >> 3, l8 = lane & 7;
-#pragma unroll 1
-  for (int r0 = 4 * warp; r0 < nrows; r0 += 4 * NW) {
-    const int r = r0 + sub;
+  if (rowc) {
+    // 1. this thread's row r, every (NT / R)-th K value of it, eight loads in flight (zeros past k and for
+    // rows past the operand); its largest magnitude and sum of squares
+    const int r = tid & (R - 1), cstep = NT >> lr;
+    const bool rv = r < nrows && task.r0 + r < task.msrc;
+    const T *px = X + task.r0 + r;
+    T *row = stage + r * stride;
     double m = 0.0, s2 = 0.0;
-    if (r < nrows) {
-      const T *row = stage + r * stride;
-#pragma unroll 4
-      for (int c = l8; c < (int)kfull; c += 8) {
-        const T v = row[c + c / LK];
-        m = fmax(m, absmax(v));
-        s2 += sq_of(v);
+#pragma unroll 1
+    for (int c0 = tid >> lr; c0 < (int)kfull; c0 += 8 * cstep) {
+      T v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int c = c0 + u * cstep;
+        v[u] = rv && c < task.k ? __ldg(px + (int64_t)c * task.ks) : z;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int c = c0 + u * cstep;
+        m = fmax(m, absmax(v[u]));
+        s2 += sq_of(v[u]);
+        if (c < (int)kfull) row[c + c / LK] = v[u];
       }
     }
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) {
+    for (int o = R; o < 32; o <<= 1) {
       m = fmax(m, __shfl_xor_sync(full, m, o));
       s2 += __shfl_xor_sync(full, s2, o);
     }
-    if (r >= nrows) continue;
-    const int e = row_exponent<S>(m);
-    const int64_t rr = task.r0 + r;
-    if (l8 == 0) {
+    // row r's partial results: slot (warp, lane) for R ≤ 32; with 64 row slots every other warp has the row
+    if (lane < R) {
+      rmax[warp * 32 + lane] = m;
+      rsum[warp * 32 + lane] = s2;
+    }
+  } else {
+    // 1. copy the rows in (zeros past k and for rows past the operand): element q = tid, tid + NT, … as
+    // (r, c), c stepping by NT mod kfull with a carry into r (no division per element)
+    const int total = nrows * (int)kfull, fast = (int)kfull;
+    const int fstep = NT % fast, sstep = NT / fast;
+    int c = tid % fast, r = tid / fast;
+#pragma unroll 1
+    for (int q = tid; q < total; q += NT) {
+      T *dst = stage + r * stride + c + c / LK;
+      const int64_t rr = task.r0 + r;
+      if (c < task.k && rr < task.msrc) cp_async_elem(dst, X + rr * task.rs + (int64_t)c * task.ks);
+      else *dst = z;
+      c += fstep;
+      r += sstep;
+      if (c >= fast) {
+        c -= fast;
+        ++r;
+      }
+    }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+    if (tid == 0) TL_STAMP(3);
+    // 2. row maxima and sums of squares: L lanes per row
+    const int L = nrows >= 4 * NW ? 8 : nrows >= 2 * NW ? 16 : 32, per = 32 / L;
+    const int sub = lane / L, l8 = lane & (L - 1);
+#pragma unroll 1
+    for (int r0 = per * warp; r0 < nrows; r0 += per * NW) {
+      const int rq = r0 + sub;
+      double m = 0.0, s2 = 0.0;
+      if (rq < nrows) {
+        const T *row = stage + rq * stride;
+#pragma unroll 4
+        for (int cc = l8; cc < (int)kfull; cc += L) {
+          const T v = row[cc + cc / LK];
+          m = fmax(m, absmax(v));
+          s2 += sq_of(v);
+        }
+      }
+      for (int o = L >> 1; o > 0; o >>= 1) {
+        m = fmax(m, __shfl_xor_sync(full, m, o));
+        s2 += __shfl_xor_sync(full, s2, o);
+      }
+      if (rq < nrows && l8 == 0) {
+        rmax[rq] = m;
+        rsum[rq] = s2;
+      }
+    }
+  }
+  __syncthreads();
+  // row exponents and the task's block statistics (the first two warps: one row per lane)
+  int32_t *ex = reinterpret_cast<int32_t *>(ws + task.ws_e);
+  if (warp < 2) {
+    unsigned ebm = 0u;
+    double nrm = 0.0;
+    const int r = tid;
+    if (r < nrows) {
+      double m = rmax[r], s2 = rsum[r];
+      if (rowc) {  // the partial results of the warps that hold the row, in warp order
+        const int step = R > 32 ? 2 : 1, w0 = R > 32 ? r >> 5 : 0, l = r & 31;
+        m = 0.0;
+        s2 = 0.0;
+        for (int w = w0; w < NW; w += step) {
+          m = fmax(m, rmax[w * 32 + l]);
+          s2 += rsum[w * 32 + l];
+        }
+      }
+      const int e = row_exponent<S>(m);
+      const int64_t rr = task.r0 + r;
       rexp[r] = e;
       if (rr < task.msrc) {
         if (CPLX && op == 0) {
@@ -1511,38 +1575,36 @@ __device__ __forceinline__ void slice_staged(const SliceTask &task, const void *
         } else {
           ex[rr] = e;
         }
+        if (m > 0.0) {
+          ebm = (unsigned)(e + kExpBias);
+          nrm = sqrt(s2);
+        }
       }
     }
-    if (rr < task.msrc && m > 0.0) {
-      ebm = max(ebm, (unsigned)(e + kExpBias));
-      nrm = fmax(nrm, sqrt(s2));
-    }
-  }
-  // the task's block statistics: one value per warp into shared memory, one reduction per task
-  // into the block statistics after the slices (the global reductions of many CTAs onto a few
-  // addresses stay out of the way of the loads and stores)
-  ebm = __reduce_max_sync(full, ebm);
+    // one value per warp into shared memory, one reduction per task into the block statistics after
+    // the slices (the global reductions of many CTAs onto a few addresses stay out of the way)
+    ebm = __reduce_max_sync(full, ebm);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) nrm = fmax(nrm, __shfl_xor_sync(full, nrm, o));
-  if (lane == 0) {
-    wstat[warp] = ebm;
-    wstat[NW + warp] = (unsigned long long)__double_as_longlong(nrm);
+    for (int o = 16; o > 0; o >>= 1) nrm = fmax(nrm, __shfl_xor_sync(full, nrm, o));
+    if (lane == 0) {
+      wstat[warp] = ebm;
+      wstat[2 + warp] = (unsigned long long)__double_as_longlong(nrm);
+    }
   }
   __syncthreads();
   if (tid == 0) TL_STAMP(4);
-  // 3. the slices of every piece (row, p)
+  // 3. the slices of every piece (row, p), rows first
   int8_t *base = ws + task.ws_s;
-  const int npieces = nrows * nchunk;
-  const int pstep = NT % nchunk, rstep = NT / nchunk;
-  int p = tid % nchunk, r = tid / nchunk;
+  const int npieces = nrows * nchunk, rstep = NT % nrows, pstep = NT / nrows;
+  int r = tid % nrows, p = tid / nrows;
 #pragma unroll 1
   for (int q = tid; q < npieces; q += NT) {
-    const int pr = p, rr0 = r;
-    p += pstep;
+    const int rr0 = r, pr = p;
     r += rstep;
-    if (p >= nchunk) {
-      p -= nchunk;
-      ++r;
+    p += pstep;
+    if (r >= nrows) {
+      r -= nrows;
+      ++p;
     }
     const int64_t rr = task.r0 + rr0;
     if (rr >= task.msrc) continue;
@@ -1555,9 +1617,9 @@ __device__ __forceinline__ void slice_staged(const SliceTask &task, const void *
   if (tid == 0) {
     unsigned long long e8 = 0ull, n8 = 0ull;
 #pragma unroll
-    for (int w = 0; w < NW; ++w) {
+    for (int w = 0; w < 2; ++w) {
       e8 = max(e8, wstat[w]);
-      n8 = max(n8, wstat[NW + w]);  // bits of non-negative doubles order like their values
+      n8 = max(n8, wstat[2 + w]);  // bits of non-negative doubles order like their values
     }
     if (e8 != 0ull) {
       red_max_u64(&bst[4 * task.block + op], e8);
@@ -1593,12 +1655,13 @@ __device__ __forceinline__ void publish_rows(const FusedArgs &g, const SliceTask
                  : "memory");
   }
 }
-constexpr int kSliceThreads = 256;
+constexpr int kSliceThreads = 256, kSliceCtas = 3;  // threads, CTAs per SM
 template <int S, bool CPLX>
-__global__ void __launch_bounds__(kSliceThreads, 2) gemm_split_slice_kernel(const FusedArgs args) {
+__global__ void __launch_bounds__(kSliceThreads, kSliceCtas) gemm_split_slice_kernel(const FusedArgs args) {
   extern __shared__ __align__(16) unsigned char stage[];
   __shared__ int rexp[kStagedRowsMax];
-  __shared__ unsigned long long wstat[2 * (kSliceThreads / 32)];
+  __shared__ double rmax[kSliceThreads], rsum[kSliceThreads];
+  __shared__ unsigned long long wstat[4];
   const FusedArgs &g = args;
   pdl_wait();     // the operands come from earlier kernels of the stream
   pdl_trigger();  // the products launch may begin its prologue
@@ -1608,7 +1671,7 @@ __global__ void __launch_bounds__(kSliceThreads, 2) gemm_split_slice_kernel(cons
   for (int t = (int)blockIdx.x; t < g.nctasks; t += (int)gridDim.x) {
     const SliceTask task = g.stasks[t];
     slice_staged<S, CPLX, kSliceThreads>(task, task.operand == 0 ? (const void *)g.A : (const void *)g.B, g.ws,
-                                         g.bst, stage, rexp, wstat);
+                                         g.bst, stage, rexp, rmax, rsum, wstat);
     // publish the task's rows: the slices are read by bulk copies (async proxy) of the products
     fence_proxy_async_global();
     __syncthreads();
@@ -1672,9 +1735,9 @@ int launch_split(tkb_ctx *ctx, const tkb_plan *p, void *C, const void *A, const 
   if (fa.nstasks > 0) {
     auto ks = cplx ? gemm_split_slice_kernel<S, true> : gemm_split_slice_kernel<S, false>;
     TKB_CUDA_TRY(ctx, cudaFuncSetAttribute(ks, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageBytes));
-    // one CTA per staged task and one warp per warp task, where that fits two CTAs per SM
+    // one CTA per staged task and one warp per warp task, where that fits the SMs
     const int warps = kSliceThreads / 32;
-    const int grid = std::max(1, std::min(2 * ctx->num_sms,
+    const int grid = std::max(1, std::min(kSliceCtas * ctx->num_sms,
                                           std::max(fa.nctasks, (fa.nstasks - fa.nctasks + warps - 1) / warps)));
     TKB_CUDA_TRY(ctx, launch_pdl(ks, dim3((unsigned)grid), dim3(kSliceThreads), (size_t)kStageBytes, ctx->stream, fa));
     ctx->launches++;
@@ -1778,22 +1841,31 @@ int tkb_gemm_split_prepare(tkb_ctx *ctx, tkb_plan *p) {
     int64_t staged_bytes = 0;
     for (const SJob &t : sj) {
       const int64_t kfull = cplx ? p->hblocks[t.block].kpad / 2 : p->hblocks[t.block].kpad;
-      const int64_t rowb = (kfull + kfull / (cplx ? 8 : 16)) * esize;
+      const int64_t rowb = stage_row(kfull, cplx ? 8 : 16) * esize;
       if (rowb <= kStageBytes) staged_bytes += rowb * t.nsrc;
     }
-    const int64_t per_task = std::max<int64_t>(8 * 1024, staged_bytes / std::max<int64_t>(1, 2 * ctx->num_sms));
+    const int64_t per_task = std::max<int64_t>(8 * 1024, staged_bytes / std::max<int64_t>(1, kSliceCtas * ctx->num_sms));
     for (const SJob &t : sj) {
       const int64_t kfull = cplx ? p->hblocks[t.block].kpad / 2 : p->hblocks[t.block].kpad;
-      const int64_t rowb = (kfull + kfull / (cplx ? 8 : 16)) * esize;
+      const int64_t rowb = stage_row(kfull, cplx ? 8 : 16) * esize;
       if (rowb <= kStageBytes) {
-        const int32_t r = (int32_t)std::max<int64_t>(
-            1, std::min<int64_t>({(int64_t)kStagedRowsMax, kStageBytes / rowb, (per_task + rowb - 1) / rowb}));
+        // rows: at most what the stage holds; a power of two where a thread keeps one row, else whole
+        // groups of 8 (the rows whose digits are neighbours)
+        const int64_t most = std::max<int64_t>(
+            1, std::min<int64_t>({(int64_t)kStagedRowsMax, kStageBytes / rowb,
+                                  std::max<int64_t>(4, (per_task + rowb - 1) / rowb)}));
+        int32_t lr = 0;
+        while ((2ll << lr) <= most) ++lr;
+        const GBlock &tb = p->hblocks[t.block];
+        const bool rowc = t.op == 0 ? tb.opA == TKB_OP_N || tb.lda == 1 : tb.opB != TKB_OP_N || tb.ldb == 1;
+        const int32_t r = rowc ? 1 << lr : (int32_t)(most >= 8 ? most & ~7 : most);
         for (int32_t r0 = 0; r0 < t.nsrc; r0 += r) {
           SliceTask j{};
           j.block = t.block;
           j.operand = t.op;
           j.r0 = r0;
           j.nrows = std::min(r, t.nsrc - r0);
+          j.lr = lr;
           jobs.push_back(j);
         }
       } else {

@@ -1933,6 +1933,12 @@ int tkb_gemm_split_prepare(tkb_ctx *ctx, tkb_plan *p) {
   // the decomposition allows it (max_pieces ≥ 2, halves of at least min_piece_steps stages). A tile
   // whose K needs more than one exact piece (int32 accumulators stay exact over (2^31 − 1)/(S·127²)
   // K positions) is split in any case; a block whose K needs more than two runs in FP64.
+  // Beyond one round the splits even out the clusters' lists: the items are dealt longest first, and
+  // the number of tiles to split is the one that leaves the busiest cluster least (in K stages, with the
+  // epilogue's part that the next item waits for: about 6 stages of 1.05 us, 8 with the exchange). The
+  // second product of a U(1) effective Hamiltonian (212 tiles of up to 55 stages) takes 100 us (117 with
+  // tiles split only where one round holds them all).
+  constexpr int64_t kUnsplitCost = 6, kSplitCost = 8;
   std::vector<SplitTile> kt;
   int nslots = 0, npart = 0;
   {
@@ -1941,35 +1947,86 @@ int tkb_gemm_split_prepare(tkb_ctx *ctx, tkb_plan *p) {
     for (GBlock &b : p->hblocks)
       if (b.kpad / KSTAGE > 2 * maxst) b.fp64only = 1;
     const int64_t nt = (int64_t)tiles.size();
-    int64_t budget = p->max_pieces >= 2 ? std::max<int64_t>(0, 2 * ncl - nt) : 0;  // tiles to split
     struct Pair {
       SplitTile a, b;
       int64_t cost;
     };
-    std::vector<Pair> pairs;
-    std::vector<SplitTile> singles;
     const SplitTile none{0, 0, 0, 2, 0, 0, -1, 1, 0, 0};
-    for (const GTile &t : tiles) {  // longest K first
-      const int nk = t.kind == 0 ? p->hblocks[t.block].kpad / KSTAGE : 0;
-      const bool must = t.kind == 0 && nk > maxst && !p->hblocks[t.block].fp64only;
-      const bool may = t.kind == 0 && budget > 0 && nk >= 2 * p->min_piece_steps;
-      if (must || may) {
-        if (!must) --budget;
-        pairs.push_back({{t.block, t.m0, t.n0, 0, 0, nk / 2, -1, 2, 0, 0},
-                         {t.block, t.m0, t.n0, 0, nk / 2, nk, -1, 2, 1, 0}, (int64_t)(nk - nk / 2)});
-      } else {
-        singles.push_back({t.block, t.m0, t.n0, t.kind, 0, nk, -1, 1, 0, 0});
+    auto stages = [&](const GTile &t) { return t.kind == 0 ? (int64_t)(p->hblocks[t.block].kpad / KSTAGE) : 0; };
+    // the pairs when the `nsplit` longest tiles are split (as far as they may be)
+    auto pair_up = [&](int64_t nsplit) {
+      std::vector<Pair> pairs;
+      std::vector<SplitTile> singles;
+      for (const GTile &t : tiles) {  // longest K first
+        const int nk = (int)stages(t);
+        const bool must = t.kind == 0 && nk > maxst && !p->hblocks[t.block].fp64only;
+        const bool may = t.kind == 0 && nsplit > 0 && nk >= 2 * p->min_piece_steps;
+        if (must || may) {
+          if (!must) --nsplit;
+          pairs.push_back({{t.block, t.m0, t.n0, 0, 0, nk / 2, -1, 2, 0, 0},
+                           {t.block, t.m0, t.n0, 0, nk / 2, nk, -1, 2, 1, 0}, (int64_t)(nk - nk / 2) + kSplitCost});
+        } else {
+          singles.push_back({t.block, t.m0, t.n0, t.kind, 0, nk, -1, 1, 0, 0});
+        }
+      }
+      std::stable_sort(singles.begin(), singles.end(),
+                       [](const SplitTile &x, const SplitTile &y) { return (x.ke - x.kb) > (y.ke - y.kb); });
+      for (size_t q = 0; q < singles.size(); q += 2)
+        pairs.push_back({singles[q], q + 1 < singles.size() ? singles[q + 1] : none,
+                         (int64_t)(singles[q].ke - singles[q].kb) + kUnsplitCost});
+      std::stable_sort(pairs.begin(), pairs.end(), [](const Pair &x, const Pair &y) { return x.cost > y.cost; });
+      return pairs;
+    };
+    // longest pair first to the cluster with the least to do; returns the busiest cluster's cost
+    auto deal = [&](const std::vector<Pair> &pairs, std::vector<std::vector<int>> *lists) {
+      std::vector<std::pair<int64_t, int>> heap;  // (−cost, −cluster): the least loaded on top
+      for (int c = 0; c < (int)ncl; ++c) heap.push_back({0, -c});
+      std::make_heap(heap.begin(), heap.end());
+      if (lists) lists->assign((size_t)ncl, {});
+      int64_t most = 0;
+      for (size_t q = 0; q < pairs.size(); ++q) {
+        std::pop_heap(heap.begin(), heap.end());
+        auto &h = heap.back();
+        if (lists) (*lists)[(size_t)-h.second].push_back((int)q);
+        h.first -= pairs[q].cost;
+        most = std::max(most, -h.first);
+        std::push_heap(heap.begin(), heap.end());
+      }
+      return most;
+    };
+    // how many of the longest tiles to split: none, or enough to fill one round of clusters, or up to all of
+    // them, whichever leaves the busiest cluster least to do
+    const int64_t most_split = p->max_pieces >= 2 ? nt : 0;
+    std::vector<int64_t> tries{0};
+    if (most_split > 0 && nt <= 16 * ncl) {  // of many rounds the last one matters little
+      tries.push_back(std::min(most_split, std::max<int64_t>(0, 2 * ncl - nt)));
+      for (int64_t q = 1; q <= 16; ++q) tries.push_back(q * most_split / 16);
+      for (int64_t q = 1; q <= 4; ++q)
+        tries.push_back(std::max<int64_t>(0, std::min(most_split, nt - nt / (2 * ncl) * 2 * ncl - (q - 1) * ncl / 4)));
+    }
+    int64_t best = -1, best_split = 0;
+    for (const int64_t q : tries) {
+      const int64_t c = deal(pair_up(q), nullptr);
+      if (best < 0 || c < best) {
+        best = c;
+        best_split = q;
       }
     }
-    std::stable_sort(singles.begin(), singles.end(),
-                     [](const SplitTile &x, const SplitTile &y) { return (x.ke - x.kb) > (y.ke - y.kb); });
-    for (size_t q = 0; q < singles.size(); q += 2)
-      pairs.push_back({singles[q], q + 1 < singles.size() ? singles[q + 1] : none, (int64_t)(singles[q].ke - singles[q].kb)});
-    std::stable_sort(pairs.begin(), pairs.end(), [](const Pair &x, const Pair &y) { return x.cost > y.cost; });
-    for (const Pair &pr : pairs) {
-      kt.push_back(pr.a);
-      kt.push_back(pr.b);
-    }
+    const std::vector<Pair> pairs = pair_up(best_split);
+    std::vector<std::vector<int>> lists;
+    deal(pairs, &lists);
+    // cluster c of the launch runs the pairs c, c + ncl, …; lists shorter than the longest are filled up
+    // with empty pairs
+    size_t rounds = 0;
+    for (const auto &l : lists) rounds = std::max(rounds, l.size());
+    for (size_t r = 0; r < rounds; ++r)
+      for (int64_t c = 0; c < ncl; ++c) {
+        const auto &l = lists[(size_t)c];
+        kt.push_back(r < l.size() ? pairs[(size_t)l[r]].a : none);
+        kt.push_back(r < l.size() ? pairs[(size_t)l[r]].b : none);
+      }
+    while (!kt.empty() && kt.back().kind == 2) kt.pop_back();
+    if (kt.size() & 1) kt.push_back(none);
   }
   p->ws_bytes = off;
   p->nstiles = (int64_t)tiles.size();

@@ -162,7 +162,8 @@ typedef struct tkb_gemm_desc {
   int32_t precision;             /* tkb_precision */
   int32_t slices;                /* split precision: int8 slices per operand. 0 = auto: up to 7,
                                     chosen per block on the device, with an FP64 fallback for
-                                    blocks and tiles the slices cannot serve to 1e-12; 3..7 =
+                                    blocks and tiles the slices cannot serve to 1e-12 and for
+                                    plans of less than 8 MFLOP in all; 3..7 =
                                     exactly that many for every block, unchecked */
 } tkb_gemm_desc;
 

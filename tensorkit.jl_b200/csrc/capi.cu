@@ -38,7 +38,7 @@ int tkb_ensure_workspace(tkb_ctx *ctx, size_t bytes) {
 
 extern "C" {
 
-int tkb_version(void) { return 200; }
+int tkb_version(void) { return 201; }
 
 const char *tkb_last_error(const tkb_ctx *ctx) {
   if (ctx) return ctx->err.c_str();
@@ -312,7 +312,12 @@ static int plan_create(tkb_ctx *ctx, const tkb_gemm_desc *d, const tkb_gemm_tuni
   p->nth = (int64_t)th.size();
   p->flops = flops;
   int rc = TKB_OK;
-  if (d->precision == TKB_SPLIT_INT8) rc = tkb_gemm_split_prepare(ctx, p);
+  // Split precision with the slice count left to the library: small products run in FP64, like blocks
+  // that no slice count serves. Slicing and the products launch take about 18 us however small the
+  // operands are, the FP64 kernel 3 - 5 us: an SU(2) environment update (two products) takes 41.8 us
+  // sliced and 10.3 in FP64 at V dim 280, 47.1 and 16.5 at 870 (4 MFLOP per product).
+  p->small_fp64 = d->precision == TKB_SPLIT_INT8 && d->slices == 0 && flops < kSplitMinFlops;
+  if (d->precision == TKB_SPLIT_INT8 && !p->small_fp64) rc = tkb_gemm_split_prepare(ctx, p);
   else rc = tkb_gemm_plain_prepare(ctx, p);
   if (rc != TKB_OK) {
     tkb_gemm_plan_destroy(p);
@@ -367,7 +372,7 @@ int tkb_gemm_plan_destroy(tkb_plan *p) {
 int tkb_gemm_plan_info(const tkb_plan *p, double *flops, int32_t *slices) {
   if (!p) return TKB_ERR_ARG;
   if (flops) *flops = p->flops;
-  if (slices) *slices = p->precision == TKB_SPLIT_INT8 ? p->slices : 0;
+  if (slices) *slices = p->precision == TKB_SPLIT_INT8 && !p->small_fp64 ? p->slices : 0;
   return TKB_OK;
 }
 
@@ -377,7 +382,10 @@ int tkb_gemm_plan_slices(tkb_ctx *ctx, const tkb_plan *p, int32_t *out, int64_t 
   const int64_t nb = (int64_t)p->hblocks.size();
   if (n < nb + 1) return tkb_set_error(ctx, TKB_ERR_ARG, "output array shorter than nblocks + 1");
   if (!p->bslices) {
-    for (int64_t i = 0; i < nb; ++i) out[i] = -1;
+    for (int64_t i = 0; i < nb; ++i) {
+      const GBlock &b = p->hblocks[(size_t)i];
+      out[i] = p->small_fp64 && b.m > 0 && b.n > 0 && b.k > 0 && !b.skinny ? 0 : -1;
+    }
     out[nb] = 0;
     return TKB_OK;
   }
@@ -395,7 +403,7 @@ int tkb_grouped_gemm(tkb_ctx *ctx, const tkb_plan *p, void *C, const void *A, co
   int rc = tkb_gemm_skinny_launch(ctx, p, C, A, B, alpha, beta);
   if (rc == TKB_OK) rc = tkb_gemm_thin_launch(ctx, p, C, A, B, alpha, beta);
   if (rc != TKB_OK) return rc;
-  if (p->precision == TKB_SPLIT_INT8) return tkb_gemm_split_launch(ctx, p, C, A, B, alpha, beta);
+  if (p->precision == TKB_SPLIT_INT8 && !p->small_fp64) return tkb_gemm_split_launch(ctx, p, C, A, B, alpha, beta);
   return tkb_gemm_launch(ctx, p, C, A, B, alpha, beta);
 }
 

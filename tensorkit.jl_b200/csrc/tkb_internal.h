@@ -198,6 +198,7 @@ constexpr int kSkinnyMinRows = 2048;  // smaller blocks go to the tiled kernels
 constexpr int kSkinnyRows = 256;       // threads of a skinny CTA (one row each per pass)
 constexpr int kSkinnyTaskRows = 1024;  // rows of one skinny task
 
+constexpr double kSplitMinFlops = 8e6;  // split precision with fewer flops (2mnk, 8mnk complex) runs in FP64
 constexpr int kThinMax = 4;        // m and n bound of the thin path (a few dot products over a long K)
 constexpr int kThinMinK = 512;     // shorter K goes to the tiled kernels
 // one task of the thin kernel: a K range of one block's products
@@ -261,6 +262,7 @@ struct tkb_plan {
   void *sjobs = nullptr;        // slicing tasks (block, operand, rows)
   int64_t nsrows = 0;           // slicing tasks
   int64_t nsctasks = 0;         // of which the first are staged (one CTA each)
+  bool small_fp64 = false;      // split precision: too small to slice, runs in FP64
   bool plain_small = false;     // plain precision: 32×32 tiles
   // split-K knobs (tkb_gemm_plan_create_tuned): pieces per tile at most, K steps per piece at least
   int max_pieces = 8, min_piece_steps = 4;

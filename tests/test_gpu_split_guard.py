@@ -97,3 +97,21 @@ def test_wide_exponent_range_block_runs_fp64():
     assert relerr(got, ref) <= TOL
     slices, _ = plan.last_slices()
     assert sorted(s for s in slices if s >= 0) == [0, 7], slices
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_small_plans_run_fp64(cplx):
+    """Less than 8 MFLOP in all: every block in FP64 (0 slices, and the plain plan's result bit for bit);
+    a slice count that the caller fixes is used whatever the size."""
+    V, Pp = cfg2_spaces(1)
+    A = O.randn(O.Hom([V, Pp], [V]), 1, cplx)
+    B = O.randn(O.Hom([V], [V]), 2, cplx)
+    got, ref, plan = _run(A, B)
+    assert relerr(got, ref) <= TOL
+    slices, fp64_tiles = plan.last_slices()
+    assert plan.flops < 8e6 and set(slices) == {0} and fp64_tiles == 0, (slices, fp64_tiles)
+    assert np.array_equal(got, _run(A, B, "plain")[0])
+    Ad, Bd = to_device(A), to_device(B)
+    C = tk.TensorMap.zeros(to_hom(O.mul(A, B).W), dtype=Ad.dtype, device=Ad.device)
+    tk.mul_(C, Ad, Bd, 1.0, 0.0, prec="split", slices=6)
+    assert set(gemm_plan(tk.get_context(Ad.device.index), C, Ad, Bd, "split", 6).last_slices()[0]) == {6}

@@ -347,34 +347,42 @@ __global__ void __launch_bounds__(kThreads)
 // leading leg in place: every sub-block row is contiguous on both sides; a small remainder of
 // transpose groups rides along with uncoalesced reads). Tiles are exact
 // (na × nb, na the full row up to the tile target), so no lane idles on a power-of-two
-// round-up, and nothing is staged: each thread issues kBatch loads, then the kBatch scaled
-// stores, and the next task's loads follow at once. Row and column come from one multiply-high
-// by the precomputed reciprocal `mul` (exact for tile indices below 2¹⁶: Granlund–Montgomery
-// division by invariant integers). Without shared-memory tiles the kernel runs at the
-// occupancy its registers allow, which keeps enough loads in flight per SM for HBM.
-template <typename T, bool CONJ, typename OFF, bool PAIRS>
-__global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 && !PAIRS) ? 6 : 4)
+// round-up, and nothing is staged: each thread issues a batch of loads, then the scaled
+// stores. Row and column come from one multiply-high by the precomputed reciprocal `mul` (exact
+// for tile indices below 2¹⁶: Granlund–Montgomery division by invariant integers).
+//
+// GT threads share a task, and a group of threads takes one task only: the hardware starts the
+// CTAs in task order, so the reads and writes of the moment stay close together in memory, and a
+// CTA that waits for its loads is replaced by the next instead of by its own stores. Persistent
+// CTAs walking contiguous ranges drift apart: adjoint of a U(1) two-site tensor, 66.6 M
+// complex elements, 420 us with them (5.07 TB/s), 398 us with the same CTAs dealt the tasks
+// in turn, 328 us so (6.5 TB/s, what a plain copy reaches); 46.2 M doubles 156 -> 114 us.
+// Tables of many small tasks (four-leg tensors of small degeneracies) give each warp its own task
+// (GT = 32): 10.1 M doubles in tasks of 144, 127 us with a CTA per task in turn, 38 us with a warp.
+constexpr int kWarpTask = 32;             // GT of tables of small tasks
+constexpr int64_t kWarpTaskAlways = 256;  // average elements per task up to which warps are always used
+constexpr int64_t kWarpTaskReal = 3072, kWarpTaskCplx = 1024;  // and with enough tasks to fill the GPU
+constexpr int64_t kRowTileMax = 2 * kTileElemsMax;  // most elements of a row task
+
+template <typename T, bool CONJ, typename OFF, bool PAIRS, int GT>
+__global__ void __launch_bounds__(kThreads, GT < kThreads ? 4 : sizeof(T) == 16 ? 6 : PAIRS ? 4 : 6)
     treetransform_rows_kernel(const TaskRec *__restrict__ recs, int64_t ntasks, T *__restrict__ dst,
                               const T *__restrict__ src, CDbl alpha_, CDbl beta_, int beta_zero, int pairs_ok) {
-  __shared__ TaskRec rs[kRecCache];
+  constexpr int kRowBatch = sizeof(T) == 16 ? kBatchPairs : kBatch;  // the same bytes in flight
   const T alpha = scalar_from<T>(alpha_);
   const T beta = scalar_from<T>(beta_);
   const bool bz = beta_zero != 0;
-  const int64_t per = (ntasks + gridDim.x - 1) / gridDim.x;  // ≤ kRecCache (host)
-  const int64_t t_begin = (int64_t)blockIdx.x * per;
-  const int64_t t_end = min(ntasks, t_begin + per);
-  {
-    const int nw = (int)(t_end > t_begin ? t_end - t_begin : 0) * (int)(sizeof(TaskRec) / 8);
-    const int64_t *srcw = reinterpret_cast<const int64_t *>(recs + t_begin);
-    int64_t *dstw = reinterpret_cast<int64_t *>(rs);
-    for (int i = threadIdx.x; i < nw; i += kThreads) dstw[i] = __ldg(srcw + i);
-  }
-  __syncthreads();
-  pdl_wait();  // the records are static; source and destination belong to earlier kernels
-  pdl_trigger();
-
-  for (int64_t task = t_begin; task < t_end; ++task) {
-    const TaskRec &R = rs[task - t_begin];
+  bool first = true;
+  constexpr int kPer = kThreads / GT;  // tasks per CTA
+  const int lane = threadIdx.x % GT;
+  const int64_t step = (int64_t)gridDim.x * kPer;  // a second task only beyond 2^31 CTAs
+  for (int64_t task = (int64_t)blockIdx.x * kPer + threadIdx.x / GT; task < ntasks; task += step) {
+    const TaskRec R = recs[task];
+    if (first) {
+      pdl_wait();  // the records are static; source and destination belong to earlier kernels
+      pdl_trigger();
+      first = false;
+    }
     if constexpr (PAIRS) {
       if (R.pairs && pairs_ok) {
         // real rows contiguous on both sides: 16-byte loads and stores of element pairs (half as
@@ -386,17 +394,17 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 && !PAIRS) ? 6 : 4)
         double2 *db2 = reinterpret_cast<double2 *>(dst + R.dbase);
         const OFF sB2 = (OFF)(R.sB / 2), dB2 = (OFF)(R.dB / 2);
         const double a = scalar_from<double>(alpha_), bb = scalar_from<double>(beta_);
-        for (int e0 = 0; e0 < nun; e0 += kThreads * kBatchPairs) {
+        for (int e0 = 0; e0 < nun; e0 += GT * kBatchPairs) {
           double2 v[kBatchPairs];
 #pragma unroll
           for (int q = 0; q < kBatchPairs; ++q) {
-            const int e = e0 + q * kThreads + threadIdx.x;
+            const int e = e0 + q * GT + lane;
             const int row = mul2 ? (int)__umulhi((unsigned)e, mul2) : e, cp = e - row * np;
             if (e < nun) v[q] = __ldg(sb2 + (OFF)cp + (OFF)row * sB2);
           }
 #pragma unroll
           for (int q = 0; q < kBatchPairs; ++q) {
-            const int e = e0 + q * kThreads + threadIdx.x;
+            const int e = e0 + q * GT + lane;
             const int row = mul2 ? (int)__umulhi((unsigned)e, mul2) : e, cp = e - row * np;
             if (e < nun) {
               double2 *dp = db2 + (OFF)cp + (OFF)row * dB2;
@@ -419,17 +427,17 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 8 && !PAIRS) ? 6 : 4)
     const double u = R.u;
     const T *sb = src + R.sbase;
     T *db = dst + R.dbase;
-    for (int e0 = 0; e0 < nel; e0 += kThreads * kBatch) {
-      T v[kBatch];
+    for (int e0 = 0; e0 < nel; e0 += GT * kRowBatch) {
+      T v[kRowBatch];
 #pragma unroll
-      for (int q = 0; q < kBatch; ++q) {
-        const int e = e0 + q * kThreads + threadIdx.x;
+      for (int q = 0; q < kRowBatch; ++q) {
+        const int e = e0 + q * GT + lane;
         const int row = mul ? (int)__umulhi((unsigned)e, mul) : e, col = e - row * na;
         if (e < nel) v[q] = ld_val(sb + (OFF)col * sA + (OFF)row * sB, CONJ);
       }
 #pragma unroll
-      for (int q = 0; q < kBatch; ++q) {
-        const int e = e0 + q * kThreads + threadIdx.x;
+      for (int q = 0; q < kRowBatch; ++q) {
+        const int e = e0 + q * GT + lane;
         const int row = mul ? (int)__umulhi((unsigned)e, mul) : e, col = e - row * na;
         if (e < nel) {
           T *dp = db + (OFF)col * dA + (OFF)row * dB;
@@ -746,7 +754,7 @@ extern "C" int tkb_table_create(tkb_ctx *ctx, const tkb_table_desc *d, tkb_table
   int max_trees = 1, max_dst = 1;
   // tile target: 2048 elements per task, smaller when the whole transform would not give
   // every SM about four tasks (small permutes are latency-bound, not bandwidth-bound)
-  int64_t kTileElems = kTileElemsMax, kRowTileElems = kTileElemsMax, kMultiElems = kMultiTile;
+  int64_t kTileElems = kTileElemsMax, kRowTileElems = kRowTileMax, kMultiElems = kMultiTile;
   {
     int64_t total = 0;
     for (int64_t g = 0; g < G; ++g) {
@@ -755,9 +763,10 @@ extern "C" int tkb_table_create(tkb_ctx *ctx, const tkb_table_desc *d, tkb_table
       total += vol * (d->group_dst_ptr[g + 1] - d->group_dst_ptr[g]);
     }
     while (kTileElems > 256 && total / kTileElems < (int64_t)ctx->num_sms * 4) kTileElems >>= 1;
-    // row tiles: about two per SM at least; a row task costs a fixed record fetch and one load
-    // round trip, so small transforms run faster with fewer, larger row tasks
-    while (kRowTileElems > 256 && total / kRowTileElems < (int64_t)ctx->num_sms * 2) kRowTileElems >>= 1;
+    // row tiles: about four per SM at least (201 / 255 degeneracies on two legs, 1.8 / 3.0 M elements,
+    // 5.1 / 11.4 us; two per SM 6.7 / 11.4, eight 6.8 / 11.2, sixteen 12.2 / 11.9), up to twice the
+    // size of the staged tiles (66.6 M complex 337 -> 328 us, 46.2 M real 124 -> 114)
+    while (kRowTileElems > 256 && total / kRowTileElems < (int64_t)ctx->num_sms * 4) kRowTileElems >>= 1;
     while (kMultiElems > 256 && total / kMultiElems < (int64_t)ctx->num_sms * 4) kMultiElems >>= 1;
   }
 
@@ -1199,30 +1208,38 @@ int tkb_transform_launch(tkb_ctx *ctx, const tkb_table *t, int dtype, void *dst,
       !use_pipe_transform()) {
     if (dtype == TKB_F64 && (alpha.im != 0.0 || beta.im != 0.0))
       return tkb_set_error(ctx, TKB_ERR_ARG, "complex scalar with real data");
-    // persistent CTAs: as many as reside at once, with at most kRecCache tasks each
     using KD = void (*)(const TaskRec *, int64_t, double *, const double *, CDbl, CDbl, int, int);
     using KC = void (*)(const TaskRec *, int64_t, double2 *, const double2 *, CDbl, CDbl, int, int);
     KD kd = nullptr;
     KC kc = nullptr;
-    const void *kfn;
     // 16-byte pair accesses need 16-byte aligned data vectors
     const int pairs_ok = ((((uintptr_t)dst | (uintptr_t)src) & 15) == 0) ? 1 : 0;
+    const int64_t nt = t->nrow_tasks;
+    // Warps or CTAs per task: a CTA of 256 threads wastes lanes and latency on a task of
+    // a few hundred elements; a warp is slower on its own but eight times as many tasks run at once.
+    // Measured (us, CTA / warp per task; four-leg U(1) tensors): 676 real elements per task 197 / 103,
+    // 1296: 474 / 365, 2500: 1555 / 1351; complex 256: 130 / 74, 784: 265 / 262, 1156: 558 / 570.
+    // With fewer tasks than warps that fit the GPU (32 per SM here) the CTA wins: 1.3 M elements in
+    // 0.5 - 1 K tasks 3.9 / 8.0.
+    const int64_t most = dtype == TKB_F64 ? kWarpTaskReal : kWarpTaskCplx;
+    const bool warps = t->elems_read <= nt * kWarpTaskAlways ||
+                       (t->elems_read < nt * most && nt >= (int64_t)ctx->num_sms * (kThreads / 8));
     if (dtype == TKB_F64) {
       // the kernel with the 16-byte pair path (fewer resident CTAs) when most of the table can
       // use it, else the scalar one
-      kd = (pairs_ok && t->row_pair_elems * 2 >= t->elems_read) ? treetransform_rows_kernel<double, false, int32_t, true>
-                                                                : treetransform_rows_kernel<double, false, int32_t, false>;
-      kfn = (const void *)kd;
+      const bool pairs = pairs_ok && t->row_pair_elems * 2 >= t->elems_read;
+      kd = warps ? (pairs ? treetransform_rows_kernel<double, false, int32_t, true, kWarpTask>
+                          : treetransform_rows_kernel<double, false, int32_t, false, kWarpTask>)
+                 : (pairs ? treetransform_rows_kernel<double, false, int32_t, true, kThreads>
+                          : treetransform_rows_kernel<double, false, int32_t, false, kThreads>);
     } else {
-      kc = conj ? treetransform_rows_kernel<double2, true, int32_t, false>
-                : treetransform_rows_kernel<double2, false, int32_t, false>;
-      kfn = (const void *)kc;
+      kc = warps ? (conj ? treetransform_rows_kernel<double2, true, int32_t, false, kWarpTask>
+                         : treetransform_rows_kernel<double2, false, int32_t, false, kWarpTask>)
+                 : (conj ? treetransform_rows_kernel<double2, true, int32_t, false, kThreads>
+                         : treetransform_rows_kernel<double2, false, int32_t, false, kThreads>);
     }
-    const int per_sm = tkb_occupancy(ctx->device, kfn, kThreads, 0);
-    if (per_sm <= 0) return tkb_set_error(ctx, TKB_ERR_CUDA, "row transform: occupancy query failed");
-    const int64_t nt = t->nrow_tasks;
-    int64_t pg = std::min<int64_t>(nt, (int64_t)ctx->num_sms * per_sm);
-    pg = std::max<int64_t>(pg, (nt + kRecCache - 1) / kRecCache);
+    const int64_t per_cta = warps ? kThreads / kWarpTask : 1;
+    const int64_t pg = std::min<int64_t>(INT32_MAX, (nt + per_cta - 1) / per_cta);
     if (kd)
       TKB_CUDA_TRY(ctx, launch_pdl(kd, dim3((int)pg), dim3(kThreads), 0, ctx->stream, t->row_rec, nt,
                                    (double *)dst, (const double *)src, a, b, bz, pairs_ok));

@@ -154,9 +154,10 @@ int tkb_transform_launch(tkb_ctx *ctx, const tkb_table *t, int dtype, void *dst,
 // partial trace --------------------------------------------------------------------------
 struct TrGroup {
   int64_t dst_off;
-  int64_t e_begin, e_end;   // entries of this destination sub-block
+  int64_t p_begin, p_end;   // pieces of this destination sub-block
   int64_t nelem;            // product of the free sizes
   int64_t task_begin;
+  int32_t lanes;            // elements per task (a power of two; the CTA's other threads share the sum)
   int32_t size[TKB_MAX_IND];
   int64_t dstr[TKB_MAX_IND];
 };
@@ -170,6 +171,11 @@ struct TrEntry {
   int64_t tstr[TKB_MAX_IND];
 };
 
+struct TrPiece {            // n consecutive traced positions of one entry
+  int64_t t0, n;
+  int64_t entry;
+};
+
 struct tkb_trace_table {
   tkb_ctx *owner = nullptr;
   int nfree = 0, ntrace = 0;
@@ -177,6 +183,7 @@ struct tkb_trace_table {
   int64_t src_len = 0, dst_len = 0;
   TrGroup *groups = nullptr;
   TrEntry *entries = nullptr;
+  TrPiece *pieces = nullptr;
   int32_t *task_group = nullptr;
 };
 

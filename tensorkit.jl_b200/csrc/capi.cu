@@ -292,11 +292,15 @@ static int plan_create(tkb_ctx *ctx, const tkb_gemm_desc *d, const tkb_gemm_tuni
     }
     if (b.skinny == 1 && b.m > 0 && b.n > 0) p->sk_dim = std::max<int>(p->sk_dim, (int)std::max(b.n, b.k));
     p->hblocks.push_back(b);
-    if (b.m > 0 && b.n > 0) {
-      if (b.skinny == 1)
-        for (int64_t m0 = 0; m0 < b.m; m0 += kSkinnyTaskRows)
-          sk.push_back({(int32_t)i, (int32_t)m0, 0, b.k > 0 ? 0 : 1});
-    }
+  }
+  // skinny blocks: one task per pass of the width class that the kernel runs the block in
+  for (int64_t i = 0; i < nb; ++i) {
+    const GBlock &b = p->hblocks[i];
+    if (b.skinny != 1 || b.m <= 0 || b.n <= 0) continue;
+    const int launch = p->sk_dim <= 2 ? 2 : p->sk_dim <= 4 ? 4 : p->sk_dim <= 6 ? 6 : p->sk_dim <= 8 ? 8 : 16;
+    const int64_t rows = (int64_t)kSkinnyRows *
+                         tkb_skinny_rows(d->dtype == TKB_C128, std::min(launch, tkb_skinny_class((int)b.n, (int)b.k)));
+    for (int64_t m0 = 0; m0 < b.m; m0 += rows) sk.push_back({(int32_t)i, (int32_t)m0, 0, b.k > 0 ? 0 : 1});
   }
   p->nsk = (int64_t)sk.size();
   // thin blocks: about two K ranges per SM over all of them, 1024 values at least

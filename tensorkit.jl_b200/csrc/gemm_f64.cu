@@ -470,121 +470,100 @@ __device__ __forceinline__ double2 scl(double2 v, CDbl a) {
   return make_double2(a.x * v.x - a.y * v.y, a.x * v.y + a.y * v.x);
 }
 
-// D bounds n and k of every block of the launch (2, 4, 6, 8 or 16) and R rows are handled per
-// thread and pass: the R·k loads of op(A) of a pass are all issued before any arithmetic, so a
-// thread keeps up to R·k loads in flight (R·D ≈ 16 values in registers, half that for complex
-// data). Rows of a task: kSkinnyTaskRows, in passes of kSkinnyRows·R. Per element the arithmetic
-// is acc = β·c (or 0), then acc = fma(α·a_l, op(B)_lj, acc) for l = 0 … k−1; rows where a_l was
-// not loaded (invalid rows, l ≥ k) hold zeros and are not stored.
-// rows per thread and pass for a width class: ≈ 16 values of op(A) in registers (complex: 8)
-template <typename T, int DK>
-constexpr int kSkinnyRowsPerPass = sizeof(T) == 8 ? (DK <= 4 ? 4 : DK <= 8 ? 2 : 1) : (DK <= 2 ? 4 : DK <= 4 ? 2 : 1);
-
-// One task's rows in passes of kSkinnyRows·RR (rows per thread RR): all RR·k loads of op(A) are
-// issued first; blocks with n, k ≤ DK ≤ D (op(B) staged with leading dimension D)
-template <typename T, bool BZ, int D, int DK, int RR>
-__device__ __forceinline__ void skinny_passes(int64_t m0, int64_t m, int kk, int n, const T *__restrict__ pa0,
-                                              int64_t sa_i, int64_t sa_l, bool conjA, T *__restrict__ pc0,
-                                              int64_t ldc, const T *Bs, CDbl alpha, CDbl beta) {
-  static_assert(kSkinnyTaskRows % (kSkinnyRows * RR) == 0, "a task is a whole number of passes");
-  for (int p0 = 0; p0 < kSkinnyTaskRows; p0 += kSkinnyRows * RR) {
-    int64_t row[RR];
-    bool valid[RR];
-    T a[RR][DK];
+// D bounds n and k of every block of the launch (2, 4, 6, 8 or 16). A CTA takes one task: the rows of
+// one pass, R per thread. The R·k loads of op(A) are issued before op(B) is staged, so a thread
+// keeps 8 - 16 values in flight (2 - 8 complex ones, with up to six CTAs per SM) while the CTA waits for
+// op(B) as well.
+// Blocks narrower than the launch's width class DK ≤ D take more rows per thread. Per element the
+// arithmetic is acc = β·c (or 0), then acc = fma(α·a_l, op(B)_lj, acc) for l = 0 … k−1; rows where
+// a_l was not loaded (invalid rows, l ≥ k) hold zeros and are not stored.
+// Bound: HBM. 1.3 M rows of width 6: real 22 us (5.6 TB/s; 24 with persistent CTAs that staged op(B) before
+// their loads and walked tasks of 1024 rows), ComplexF64 49 us (73 at three CTAs per SM); 580 K rows of
+// width 12 31 us (41) and 82 us (135); 380 K rows of width 6 in ten blocks 6.1 us (8.0) and 10.5 us (16.3).
+template <typename T, bool BZ, int D, int DK>
+__device__ __forceinline__ void skinny_task(const GTile &tk, const GBlock &b, T *__restrict__ C, const T *__restrict__ A,
+                                            const T *__restrict__ B, CDbl alpha, CDbl beta, T *Bs) {
+  constexpr int RR = tkb_skinny_rows(sizeof(T) == 16, DK);
+  const int n = (int)b.n, k = (int)b.k, kk = tk.kind == 0 ? k : 0;
+  const int64_t m = b.m, ldc = b.ldc;
+  const bool conjA = b.opA == TKB_OP_C;
+  const int64_t sa_l = (b.opA == TKB_OP_N) ? b.lda : 1;
+  const int64_t sa_i = (b.opA == TKB_OP_N) ? 1 : b.lda;
+  const T *pa0 = A + b.offA;
+  T *pc0 = C + b.offC;
+  int64_t row[RR];
+  bool valid[RR];
+  T a[RR][DK];
 #pragma unroll
-    for (int r = 0; r < RR; ++r) {
-      row[r] = m0 + p0 + r * kSkinnyRows + threadIdx.x;
-      valid[r] = row[r] < m;
-    }
+  for (int r = 0; r < RR; ++r) {
+    row[r] = (int64_t)tk.m0 + r * kSkinnyRows + threadIdx.x;
+    valid[r] = row[r] < m;
+  }
 #pragma unroll
-    for (int r = 0; r < RR; ++r)
+  for (int r = 0; r < RR; ++r)
 #pragma unroll
-      for (int l = 0; l < DK; ++l)
-        a[r][l] = (valid[r] && l < kk) ? ldA<T>(pa0 + row[r] * sa_i + l * sa_l, conjA) : zero(T{});
-    // α·a once per element of op(A); each op(B)_lj is read from shared memory once per pass
-    // and used for the RR rows
+    for (int l = 0; l < DK; ++l)
+      a[r][l] = (valid[r] && l < kk) ? ldA<T>(pa0 + row[r] * sa_i + l * sa_l, conjA) : zero(T{});
+  // op(B)(l, j), zero outside k × n
+  for (int e = threadIdx.x; e < DK * DK; e += kSkinnyRows) {
+    const int l = e % DK, j = e / DK;
+    const int64_t idx = (b.opB == TKB_OP_N) ? b.offB + l + (int64_t)j * b.ldb : b.offB + j + (int64_t)l * b.ldb;
+    Bs[e] = (l < kk && j < n) ? ldA<T>(B + idx, b.opB == TKB_OP_C) : zero(T{});
+  }
+  __syncthreads();
+  // α·a once per element of op(A); each op(B)_lj is read from shared memory once
+  // and used for the RR rows
 #pragma unroll
-    for (int r = 0; r < RR; ++r)
+  for (int r = 0; r < RR; ++r)
 #pragma unroll
-      for (int l = 0; l < DK; ++l) a[r][l] = scl(a[r][l], alpha);
+    for (int l = 0; l < DK; ++l) a[r][l] = scl(a[r][l], alpha);
 #pragma unroll
-    for (int j = 0; j < DK; ++j) {
-      if (j < n) {
-        T acc[RR];
+  for (int j = 0; j < DK; ++j) {
+    if (j < n) {
+      T acc[RR];
 #pragma unroll
-        for (int r = 0; r < RR; ++r) {
-          acc[r] = zero(T{});
-          if constexpr (!BZ)
-            if (valid[r]) acc[r] = mac(pc0[row[r] + (int64_t)j * ldc], make_beta<T>(beta), zero(T{}));
-        }
-#pragma unroll
-        for (int l = 0; l < DK; ++l) {
-          if (l < kk) {
-            const T bl = Bs[l + j * D];
-#pragma unroll
-            for (int r = 0; r < RR; ++r) acc[r] = mac(a[r][l], bl, acc[r]);
-          }
-        }
-#pragma unroll
-        for (int r = 0; r < RR; ++r)
-          if (valid[r]) pc0[row[r] + (int64_t)j * ldc] = acc[r];
+      for (int r = 0; r < RR; ++r) {
+        acc[r] = zero(T{});
+        if constexpr (!BZ)
+          if (valid[r]) acc[r] = mac(pc0[row[r] + (int64_t)j * ldc], make_beta<T>(beta), zero(T{}));
       }
+#pragma unroll
+      for (int l = 0; l < DK; ++l) {
+        if (l < kk) {
+          const T bl = Bs[l + j * DK];
+#pragma unroll
+          for (int r = 0; r < RR; ++r) acc[r] = mac(a[r][l], bl, acc[r]);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < RR; ++r)
+        if (valid[r]) pc0[row[r] + (int64_t)j * ldc] = acc[r];
     }
   }
 }
 
-// resident CTAs asked of the register allocator: the real β = 0 passes of widths 2 and 6 fit
-// 48 registers (5 CTAs per SM), the other widths up to 8 fit 80 (3 CTAs), width 16 fits 128
+// Resident CTAs asked of the register allocator: as many as fit without spills that cost more than
+// the loads they add (the β ≠ 0 kernels also hold values of C)
 template <typename T, bool BZ, int D>
-constexpr int kSkinnyMinCtas = (sizeof(T) == 8 && BZ && (D == 2 || D == 6)) ? 5 : D <= 8 ? 3 : 2;
+constexpr int kSkinnyMinCtas = sizeof(T) == 8 ? (D <= 4 ? (BZ ? 6 : 4) : D == 6 ? (BZ ? 5 : 4) : D == 8 ? 4 : 2)
+                                              : (D <= 4 ? (BZ ? 6 : 4) : D <= 8 ? (BZ ? 5 : 4) : BZ ? 3 : 2);
 
-template <typename T, bool BZ, int D, int R>
+template <typename T, bool BZ, int D>
 __global__ void __launch_bounds__(kSkinnyRows, kSkinnyMinCtas<T, BZ, D>)
-    gemm_skinny_kernel(const GBlock *__restrict__ blocks, const GTile *__restrict__ tasks, int64_t ntasks,
-                       T *__restrict__ C, const T *__restrict__ A, const T *__restrict__ B, CDbl alpha,
-                       CDbl beta) {
+    gemm_skinny_kernel(const GBlock *__restrict__ blocks, const GTile *__restrict__ tasks, T *__restrict__ C,
+                       const T *__restrict__ A, const T *__restrict__ B, CDbl alpha, CDbl beta) {
   __shared__ T Bs[D * D];
-  // a contiguous, even share of the tasks per CTA: consecutive tasks mostly share their block,
-  // so op(B) is staged again only when the block changes
-  const int64_t t_begin = (int64_t)blockIdx.x * ntasks / gridDim.x;
-  const int64_t t_end = (int64_t)(blockIdx.x + 1) * ntasks / gridDim.x;
+  const GTile tk = tasks[blockIdx.x];
+  const GBlock &b = blocks[tk.block];
+  const int dk = tkb_skinny_class((int)b.n, (int)b.k);  // uniform over the CTA
   pdl_wait();
   pdl_trigger();
-  int staged = -1;  // block whose op(B) is in Bs
-  for (int64_t ti = t_begin; ti < t_end; ++ti) {
-    const GTile tk = tasks[ti];
-    const GBlock &b = blocks[tk.block];
-    const int n = (int)b.n, k = (int)b.k;
-    const int64_t m = b.m;
-    const int kk = tk.kind == 0 ? k : 0;
-    const bool conjA = b.opA == TKB_OP_C;
-    const int64_t sa_l = (b.opA == TKB_OP_N) ? b.lda : 1;
-    const int64_t sa_i = (b.opA == TKB_OP_N) ? 1 : b.lda;
-    const int64_t ldc = b.ldc;
-    const T *pa0 = A + b.offA;
-    T *pc0 = C + b.offC;
-    if (tk.block != staged) {  // uniform over the CTA
-      __syncthreads();
-      // op(B)(l, j), zero outside k × n (the row loops below run over the full D × D)
-      for (int e = threadIdx.x; e < D * D; e += blockDim.x) {
-        const int l = e % D, j = e / D;
-        const int64_t idx = (b.opB == TKB_OP_N) ? b.offB + l + (int64_t)j * b.ldb : b.offB + j + (int64_t)l * b.ldb;
-        Bs[e] = (l < k && j < n && tk.kind == 0) ? ldA<T>(B + idx, b.opB == TKB_OP_C) : zero(T{});
-      }
-      __syncthreads();
-      staged = tk.block;
-    }
-    // blocks narrower than the launch's width class run a narrower pass with more rows per
-    // thread (uniform per task), so their threads also keep ≈ 16 loads in flight
-    if (D > 2 && kk <= 2 && n <= 2)
-      skinny_passes<T, BZ, D, 2, kSkinnyRowsPerPass<T, 2>>(tk.m0, m, kk, n, pa0, sa_i, sa_l, conjA, pc0, ldc, Bs,
-                                                           alpha, beta);
-    else if (D > 4 && kk <= 4 && n <= 4)
-      skinny_passes<T, BZ, D, 4, kSkinnyRowsPerPass<T, 4>>(tk.m0, m, kk, n, pa0, sa_i, sa_l, conjA, pc0, ldc, Bs,
-                                                           alpha, beta);
-    else
-      skinny_passes<T, BZ, D, D, R>(tk.m0, m, kk, n, pa0, sa_i, sa_l, conjA, pc0, ldc, Bs, alpha, beta);
-  }
+  if (D > 2 && dk == 2)
+    skinny_task<T, BZ, D, 2>(tk, b, C, A, B, alpha, beta, Bs);
+  else if (D > 4 && dk == 4)
+    skinny_task<T, BZ, D, 4>(tk, b, C, A, B, alpha, beta, Bs);
+  else
+    skinny_task<T, BZ, D, D>(tk, b, C, A, B, alpha, beta, Bs);
 }
 
 }  // namespace
@@ -593,12 +572,8 @@ namespace {
 
 template <typename T, bool BZ, int D>
 int skinny_launch_t(tkb_ctx *ctx, const tkb_plan *p, T *C, const T *A, const T *B, CDbl a, CDbl bb) {
-  auto k = gemm_skinny_kernel<T, BZ, D, kSkinnyRowsPerPass<T, D>>;
-  const int per_sm = tkb_occupancy(ctx->device, (const void *)k, kSkinnyRows, 0);
-  if (per_sm <= 0) return tkb_set_error(ctx, TKB_ERR_CUDA, "skinny GEMM: occupancy query failed");
-  const int grid = (int)std::min<int64_t>(p->nsk, (int64_t)ctx->num_sms * per_sm);
-  TKB_CUDA_TRY(ctx, launch_pdl(k, dim3(grid), dim3(kSkinnyRows), 0, ctx->stream, p->blocks, p->sktasks, p->nsk, C,
-                               A, B, a, bb));
+  TKB_CUDA_TRY(ctx, launch_pdl(gemm_skinny_kernel<T, BZ, D>, dim3((unsigned)p->nsk), dim3(kSkinnyRows), 0, ctx->stream,
+                               p->blocks, p->sktasks, C, A, B, a, bb));
   return TKB_OK;
 }
 

@@ -203,7 +203,14 @@ struct GBlock {
 constexpr int kSkinnyMax = 16;        // n and k bound of the skinny (row-per-thread) path
 constexpr int kSkinnyMinRows = 2048;  // smaller blocks go to the tiled kernels
 constexpr int kSkinnyRows = 256;       // threads of a skinny CTA (one row each per pass)
-constexpr int kSkinnyTaskRows = 1024;  // rows of one skinny task
+// width class of a skinny block inside its launch (17: the launch's own class D) and the rows per
+// thread of a task of class dk
+__host__ __device__ constexpr int tkb_skinny_class(int n, int k) {
+  return n <= 2 && k <= 2 ? 2 : n <= 4 && k <= 4 ? 4 : 17;
+}
+__host__ __device__ constexpr int tkb_skinny_rows(bool cplx, int dk) {
+  return cplx ? (dk <= 2 ? 2 : 1) : (dk <= 2 ? 4 : dk <= 8 ? 2 : 1);
+}
 
 constexpr double kSplitMinFlops = 8e6;  // split precision with fewer flops (2mnk, 8mnk complex) runs in FP64
 constexpr int kThinMax = 4;        // m and n bound of the thin path (a few dot products over a long K)
@@ -235,7 +242,7 @@ struct tkb_plan {
   tkb_ctx *owner = nullptr;
   int dtype = 0, precision = 0, slices = 0;
   int64_t nblocks = 0;
-  GTile *sktasks = nullptr;     // skinny blocks: (block, first row) tasks of kSkinnyTaskRows rows
+  GTile *sktasks = nullptr;     // skinny blocks: (block, first row) tasks, one pass of its width class each
   int64_t nsk = 0;
   int sk_dim = 0;               // max(n, k) over the skinny blocks
   ThinTask *thtasks = nullptr;  // thin blocks: K ranges, their partial sums and arrival counters

@@ -131,8 +131,9 @@ def _sync_out(ctx, *ts):
 
 def _braid_table(ctx, tdst_space, tsrc, p, levels):
     lv = tuple(levels)
-    n1 = tsrc.numout()
-    return device_table(ctx, tdst_space, tsrc, p, (lv[:n1], lv[n1:]))
+    l1 = tuple(lv[i - 1] for i in tsrc.codomainind())
+    l2 = tuple(lv[i - 1] for i in tsrc.domainind())
+    return device_table(ctx, tdst_space, tsrc, p, (l1, l2))
 
 
 def braid_(tdst: TensorMap, tsrc, p, levels, alpha=1.0, beta=0.0):

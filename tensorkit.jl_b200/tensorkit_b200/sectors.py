@@ -52,6 +52,11 @@ class Sector:
     def isunit(self) -> bool:
         return self == self.unit()
 
+    # A hash of text belongs to one process, so a pickle carries the label alone and loading hashes it
+    # anew (`__setstate__` for pickles that carry the fields).
+    def __setstate__(self, state):
+        self._restore(state[1])
+
 
 # ----------------------------------------------------------------------------------------
 # U(1)
@@ -75,6 +80,12 @@ class U1Irrep(Sector):
 
     def __hash__(self):
         return self._h
+
+    def __reduce__(self):
+        return U1Irrep, (self.charge,)
+
+    def _restore(self, fields):
+        self.__init__(twice=fields["q2"])
 
     def __repr__(self):
         return f"U1Irrep({self.charge})"
@@ -125,6 +136,12 @@ class SU2Irrep(Sector):
     def __hash__(self):
         return self._h
 
+    def __reduce__(self):
+        return SU2Irrep, (self.j,)
+
+    def _restore(self, fields):
+        self.__init__(twice=fields["j2"])
+
     def __repr__(self):
         return f"SU2Irrep({self.j})"
 
@@ -170,6 +187,12 @@ class ProductSector(Sector):
 
     def __hash__(self):
         return self._h
+
+    def __reduce__(self):
+        return ProductSector, self.sectors
+
+    def _restore(self, fields):
+        self.__init__(*fields["sectors"])
 
     def __repr__(self):
         return " ⊠ ".join(repr(s) for s in self.sectors)

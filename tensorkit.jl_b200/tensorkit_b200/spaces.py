@@ -114,6 +114,14 @@ class GradedSpace:
     def __hash__(self):
         return self._h
 
+    # pickles carry the defining fields; hashes (one process's own) and kept results are made anew
+    def __reduce__(self):
+        return type(self), (tuple(zip(self._keys, self._degs)), self.dual_flag, self._unit)
+
+    def __setstate__(self, state):
+        f = state[1]
+        self.__init__(tuple(zip(f["_keys"], f["_degs"])), f["dual_flag"], f["_unit"])
+
     def __repr__(self):
         body = ", ".join(f"{c!r}=>{d}" for c, d in zip(self._keys, self._degs))
         return f"Vect[{body}]" + ("'" if self.dual_flag else "")
@@ -160,6 +168,12 @@ class ProductSpace:
 
     def __hash__(self):
         return self._h
+
+    def __reduce__(self):
+        return type(self), (self.spaces, self._unit)
+
+    def __setstate__(self, state):
+        self.__init__(state[1]["spaces"], state[1]["_unit"])
 
     def __repr__(self):
         if not self.spaces:
@@ -300,6 +314,12 @@ class HomSpace:
 
     def __hash__(self):
         return self._h
+
+    def __reduce__(self):
+        return type(self), (self.codomain, self.domain)
+
+    def __setstate__(self, state):
+        self.__init__(state[1]["codomain"], state[1]["domain"])
 
     def __repr__(self):
         return f"{self.codomain!r} ← {self.domain!r}"

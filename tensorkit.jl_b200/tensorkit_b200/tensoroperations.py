@@ -272,9 +272,10 @@ def _recipe(A, pA, conjA, B, pB, conjB, pAB):
 
 def _run_recipe(ctx, r, C, A, B, alpha, beta, keep):
     """Enqueue a lowered contraction. The library stream is ordered after and before the caller's once
-    for all launches; the permuted operands are allocated on the caller's stream and released after
-    that, so their memory is not reused too early. `keep`: C was passed in (its memory may belong to
-    another stream's pool)."""
+    for all launches. The permuted operands are allocated on the caller's stream before the first (the
+    memory may have been in use by work that another thread enqueued there a moment ago) and released
+    after the second, so it is reused neither way too early. `keep`: C was passed in (its memory may
+    belong to another stream's pool)."""
     lib, h = ctx.lib, ctx.handle
     out = C.data
     dtype, device = out.dtype, out.device
@@ -284,6 +285,8 @@ def _run_recipe(ctx, r, C, A, B, alpha, beta, keep):
     if r.adj[1]:
         B = _adjoint(B)
     ops = [B, A] if r.swap else [A, B]
+    moved = [None if m is None else new_tensor(m[0], dtype, device) for m in r.move]
+    D = C if r.move_c is None else new_tensor(r.wc, dtype, device)
     cur = _current_stream(ctx)
     joined = cur != ctx.stream_handle
     rc = lib.tkb_ctx_after(h, cur) if joined else 0
@@ -292,14 +295,13 @@ def _run_recipe(ctx, r, C, A, B, alpha, beta, keep):
     try:
         for i, m in enumerate(r.move):
             if m is not None:
-                t = new_tensor(m[0], dtype, device)
+                t = moved[i]
                 rc = lib.tkb_treetransform(h, m[1].handle, code, t.data.data_ptr(), ops[i].data.data_ptr(), _ONE,
                                            _ZERO, m[2])
                 if rc:
                     L.check(rc, h)
                 ops[i] = t
         X, Y = ops
-        D = C if r.move_c is None else new_tensor(r.wc, dtype, device)
         mode = precision()
         plan = r.plans.get(mode)
         if plan is None or plan.handle is None:

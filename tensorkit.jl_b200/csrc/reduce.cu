@@ -194,7 +194,7 @@ constexpr size_t kNoAllocSegBytes = kNoAllocMaxSeg * sizeof(RSeg);              
 constexpr size_t kNoAllocBeginOff = kNoAllocSegBytes;
 constexpr size_t kNoAllocPartialOff = (kNoAllocBeginOff + (kNoAllocMaxSeg + 1) * 8 + 255) / 256 * 256;
 constexpr size_t kNoAllocResultOff = kNoAllocPartialOff + kNoAllocMaxCta * sizeof(double2);
-constexpr size_t kNoAllocCountOff = kNoAllocResultOff + 128;  // arrival counter (zero between calls)
+constexpr size_t kNoAllocCountOff = kNoAllocResultOff + 128;  // arrival counter
 constexpr size_t kNoAllocBytes = kNoAllocResultOff + 256;                          // ~57 KiB
 }  // namespace
 
@@ -283,9 +283,12 @@ extern "C" int tkb_reduce_noalloc(int device, void *stream, int kind, int dtype,
     }
     const int nb = (int)std::max<int64_t>(1, std::min<int64_t>((total + 4095) / 4096, kNoAllocMaxCta));
     if (e == cudaSuccess) {
+      // calls that overlap share the counter: each starts it anew, so that none spoils those after it
       int *arrived = reinterpret_cast<int *>(base + kNoAllocCountOff);
-      e = dtype == TKB_F64 ? reduce_launch<double>(kind, nb, st, dsegs, dbegin, nseg, total, x, y, dpart, arrived, dres)
-                           : reduce_launch<double2>(kind, nb, st, dsegs, dbegin, nseg, total, x, y, dpart, arrived, dres);
+      e = cudaMemsetAsync(arrived, 0, sizeof(int), st);
+      if (e == cudaSuccess)
+        e = dtype == TKB_F64 ? reduce_launch<double>(kind, nb, st, dsegs, dbegin, nseg, total, x, y, dpart, arrived, dres)
+                             : reduce_launch<double2>(kind, nb, st, dsegs, dbegin, nseg, total, x, y, dpart, arrived, dres);
     }
     if (e == cudaSuccess) {
       e = cudaGetLastError();

@@ -27,30 +27,54 @@ class SpaceMismatch(ValueError):
     """Raised when spaces of tensors do not match (TensorKit's `SpaceMismatch`)."""
 
 
-# One tuple object per set of sectors, so that comparing equal spaces compares identities (bounded;
-# spaces whose tuples differ as objects still compare by value)
+class _KeySet:
+    """The sectors of a space in order, with what follows from them alone."""
+    __slots__ = ("keys", "h", "_duals")
+
+    def __init__(self, keys):
+        for a, b in zip(keys, keys[1:]):
+            if a == b:
+                raise ValueError("duplicate sector in GradedSpace")
+        self.keys = keys
+        self.h = hash(keys)
+        self._duals = None
+
+    def sectors(self, dual):
+        if not dual:
+            return self.keys
+        if self._duals is None:
+            self._duals = tuple(c.dual() for c in self.keys)
+        return self._duals
+
+
+# One set per tuple of sectors, so that comparing equal spaces compares identities and making a space
+# of sectors met before checks and hashes them once (bounded; equal sets that are different
+# objects still compare by value)
 _KEYSETS: dict = {}
 _MAX_KEYSETS = 4096
 
 
-def _shared_keys(keys):
-    if len(_KEYSETS) >= _MAX_KEYSETS:
-        _KEYSETS.clear()
-    return _KEYSETS.setdefault(keys, keys)
+def _keyset(keys) -> _KeySet:
+    ks = _KEYSETS.get(keys)
+    if ks is None:
+        ks = _KeySet(keys)
+        if len(_KEYSETS) >= _MAX_KEYSETS:
+            _KEYSETS.clear()
+        _KEYSETS[keys] = ks
+    return ks
 
 
 class GradedSpace:
     """⨁_c ℂ^{n_c} ⊗ R_c for sectors c of one sector type."""
-    __slots__ = ("_keys", "_degs", "dual_flag", "_unit", "_h", "_sectors", "_dimmap", "_dual")
+    __slots__ = ("_keys", "_degs", "dual_flag", "_unit", "_h", "_sectors", "_dimmap", "_dual", "_ks")
 
     def __init__(self, dims, dual: bool = False, unit: Sector | None = None):
         items = list(dims.items()) if isinstance(dims, dict) else list(dims)
         items = [(c, int(d)) for (c, d) in items if int(d) > 0]
         items.sort(key=lambda cd: cd[0].sortkey())
-        for i in range(1, len(items)):
-            if items[i][0] == items[i - 1][0]:
-                raise ValueError("duplicate sector in GradedSpace")
-        self._keys = _shared_keys(tuple(c for c, _ in items))
+        ks = _keyset(tuple([c for c, _ in items]))
+        self._ks = ks
+        self._keys = ks.keys
         self._degs = tuple(d for _, d in items)
         self.dual_flag = bool(dual)
         if unit is None:
@@ -58,8 +82,8 @@ class GradedSpace:
                 raise ValueError("empty GradedSpace needs an explicit unit sector")
             unit = items[0][0].unit()
         self._unit = unit
-        self._h = hash((self._keys, self._degs, self.dual_flag))
-        self._sectors = tuple(c.dual() for c in self._keys) if self.dual_flag else self._keys
+        self._h = hash((ks.h, self._degs, self.dual_flag))
+        self._sectors = ks.sectors(self.dual_flag)
         self._dimmap = dict(zip(self._keys, self._degs))
         self._dual = None
 
@@ -90,7 +114,11 @@ class GradedSpace:
     def dual(self) -> "GradedSpace":
         d = self._dual
         if d is None:
-            d = GradedSpace(list(zip(self._keys, self._degs)), not self.dual_flag, self._unit)
+            d = GradedSpace.__new__(GradedSpace)
+            d._ks, d._keys, d._degs, d._dimmap, d._unit = self._ks, self._keys, self._degs, self._dimmap, self._unit
+            d.dual_flag = not self.dual_flag
+            d._h = hash((d._ks.h, d._degs, d.dual_flag))
+            d._sectors = d._ks.sectors(d.dual_flag)
             d._dual = self
             self._dual = d
         return d
@@ -109,7 +137,7 @@ class GradedSpace:
 
     def __eq__(self, o):
         return self is o or (isinstance(o, GradedSpace) and o._h == self._h and o.dual_flag == self.dual_flag
-                             and o._degs == self._degs and o._keys == self._keys)
+                             and o._degs == self._degs and (o._ks is self._ks or o._keys == self._keys))
 
     def __hash__(self):
         return self._h

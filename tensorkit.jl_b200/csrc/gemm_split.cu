@@ -26,15 +26,14 @@
 // copy moves into shared memory (the issue rate of one producer thread, not the copy size,
 // limits the ring).
 //
-// One persistent launch per grouped GEMM (gemm_split_fused_kernel, one CTA per SM): the CTAs
-// first claim slicing tasks (up to 32 source rows over the whole K range: row maxima, exponents,
-// slices; the operand is read once), then run the products items (128×64 output tiles, or K
-// pieces of them) with a producer warp streaming the stages of A and B with cp.async.bulk into a
-// shared-memory ring as deep as fits (5 stages at S = 7), an MMA warp issuing
-// tcgen05.mma.kind::i8 (M=128, K=32, N = 64 per B slice, up to four B slices per instruction)
-// into S int32 diagonal accumulators held in tensor memory (S·64 of 512 columns), and eight
-// epilogue warps (two per TMEM lane quarter) reading the accumulators back with tcgen05.ld and
-// recombining them in FP64 while the next item's stages load.
+// Two launches per grouped GEMM: the slicing launch (gemm_split_slice_kernel, three CTAs per SM: a task is
+// a few whole rows over the whole K range; row maxima, exponents, slices; the operand is read
+// once), then the products launch (gemm_split_fused_kernel, one persistent CTA per SM in clusters of
+// two) over 128×64 output tiles or K halves of them: a producer warp streams the stages of A and B with
+// cp.async.bulk into a shared-memory ring, an MMA warp issues tcgen05.mma.kind::i8 (M=128, K=32,
+// N = 64 per B slice, up to four B slices per instruction) into S int32 diagonal accumulators held in
+// tensor memory (S·64 of 512 columns), and eight epilogue warps (two per TMEM lane quarter) read the
+// accumulators back with tcgen05.ld and recombine them in FP64 while the next item's stages load.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>

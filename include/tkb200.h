@@ -60,7 +60,7 @@ typedef struct tkb_graph tkb_graph;
 /* ---- context ------------------------------------------------------------------------ */
 int tkb_version(void);
 /* stream: a cudaStream_t (0 = legacy default stream). workspace_bytes: scratch held by
- * the context for split-precision operands and reduction partials (grown on demand). */
+ * the context for split-precision operands (grown on demand). */
 int tkb_ctx_create(int device, void *stream, size_t workspace_bytes, tkb_ctx **out);
 int tkb_ctx_destroy(tkb_ctx *ctx);
 int tkb_ctx_set_stream(tkb_ctx *ctx, void *stream);

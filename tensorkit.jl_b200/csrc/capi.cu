@@ -45,6 +45,16 @@ const char *tkb_last_error(const tkb_ctx *ctx) {
   return g_err.c_str();
 }
 
+// releases what a context holds (null where it was not made yet)
+static void ctx_free(tkb_ctx *ctx) {
+  cudaFree(ctx->ws);
+  cudaFree(ctx->counters);
+  cudaFree(ctx->red_scratch);
+  if (ctx->order) cudaEventDestroy(ctx->order);
+  cudaFreeHost(ctx->host_res);
+  delete ctx;
+}
+
 int tkb_ctx_create(int device, void *stream, size_t workspace_bytes, tkb_ctx **out) {
   if (!out) return tkb_set_error(nullptr, TKB_ERR_ARG, "null output handle");
   *out = nullptr;
@@ -65,31 +75,28 @@ int tkb_ctx_create(int device, void *stream, size_t workspace_bytes, tkb_ctx **o
   ctx->stream = (cudaStream_t)stream;
   ctx->num_sms = prop.multiProcessorCount;
   ctx->smem_optin = prop.sharedMemPerBlockOptin;
+  const size_t red = kRedSlots * (sizeof(unsigned long long) + (size_t)ctx->num_sms * kRedCtasPerSm * 16);
   e = cudaMalloc((void **)&ctx->counters, 64 * sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(ctx->counters, 0, 64 * sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->red_scratch, red);
+  if (e == cudaSuccess) e = cudaMemset(ctx->red_scratch, 0, red);
   if (e != cudaSuccess) {
-    delete ctx;
+    ctx_free(ctx);
     return tkb_set_error(nullptr, TKB_ERR_OOM, "counter allocation failed");
   }
   e = cudaEventCreateWithFlags(&ctx->order, cudaEventDisableTiming);
   if (e != cudaSuccess) {
-    cudaFree(ctx->counters);
-    delete ctx;
+    ctx_free(ctx);
     return tkb_set_error(nullptr, TKB_ERR_CUDA, cudaGetErrorString(e));
   }
   e = cudaHostAlloc((void **)&ctx->host_res, kHostSlots * 2 * sizeof(double), cudaHostAllocMapped | cudaHostAllocPortable);
   if (e != cudaSuccess) {
-    cudaEventDestroy(ctx->order);
-    cudaFree(ctx->counters);
-    delete ctx;
+    ctx_free(ctx);
     return tkb_set_error(nullptr, TKB_ERR_OOM, "result buffer allocation failed");
   }
   const size_t ws = std::max<size_t>(workspace_bytes, 1 << 20);
   if (tkb_ensure_workspace(ctx, ws) != TKB_OK) {
-    cudaEventDestroy(ctx->order);
-    cudaFree(ctx->counters);
-    cudaFreeHost(ctx->host_res);
-    delete ctx;
+    ctx_free(ctx);
     return tkb_set_error(nullptr, TKB_ERR_OOM, "workspace allocation failed");
   }
   *out = ctx;
@@ -99,11 +106,7 @@ int tkb_ctx_create(int device, void *stream, size_t workspace_bytes, tkb_ctx **o
 int tkb_ctx_destroy(tkb_ctx *ctx) {
   if (!ctx) return TKB_OK;
   cudaStreamSynchronize(ctx->stream);
-  cudaFree(ctx->ws);
-  cudaEventDestroy(ctx->order);
-  cudaFree(ctx->counters);
-  cudaFreeHost(ctx->host_res);
-  delete ctx;
+  ctx_free(ctx);
   return TKB_OK;
 }
 
@@ -432,7 +435,7 @@ int tkb_rplan_create(tkb_ctx *ctx, int64_t nseg, const int64_t *off, const int64
   p->owner = ctx;
   p->nseg = nseg;
   p->total = begin[nseg];
-  p->nblocks_launch = (int)std::max<int64_t>(1, std::min<int64_t>((p->total + 4095) / 4096, (int64_t)ctx->num_sms * 4));
+  p->nblocks_launch = (int)std::max<int64_t>(1, std::min<int64_t>((p->total + 4095) / 4096, (int64_t)ctx->num_sms * kRedCtasPerSm));
   cudaError_t e = cudaSuccess;
   if (nseg > 0) {
     e = cudaMalloc((void **)&p->segs, nseg * sizeof(RSeg));
@@ -443,11 +446,6 @@ int tkb_rplan_create(tkb_ctx *ctx, int64_t nseg, const int64_t *off, const int64
   if (e != cudaSuccess) {
     tkb_rplan_destroy(p);
     return tkb_set_error(ctx, TKB_ERR_CUDA, std::string("rplan upload: ") + cudaGetErrorString(e));
-  }
-  const int rc = tkb_ensure_workspace(ctx, (size_t)p->nblocks_launch * 16);
-  if (rc != TKB_OK) {
-    tkb_rplan_destroy(p);
-    return rc;
   }
   *out = p;
   return TKB_OK;

@@ -25,6 +25,9 @@ struct tkb_ctx {
   // doubles), and the bit mask of the slots that calls in progress hold
   double *host_res = nullptr;
   std::atomic<uint64_t> host_busy{0};
+  // reductions: kRedSlots counter words, then as many sets of partial sums; launches so far
+  unsigned char *red_scratch = nullptr;
+  std::atomic<uint64_t> red_calls{0};
   // event of tkb_ctx_after / tkb_ctx_before: recorded on one stream and waited for on the other under
   // the lock, so that threads do not re-record it between the two
   cudaEvent_t order = nullptr;
@@ -66,7 +69,10 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
 }
 
 constexpr int kHostSlots = 64;
-constexpr int kReduceSlot = 12;  // ctx->counters: CTAs of a reduction that have arrived
+// reductions: CTAs per SM at most, counters and sets of partial sums that launches take in turn, and the
+// unit of a launch's ticket (above the arrivals in its counter word)
+constexpr int kRedCtasPerSm = 4, kRedSlots = 8;
+constexpr unsigned long long kRedTicket = 1ull << 24;
 
 // status helpers ------------------------------------------------------------------------
 int tkb_set_error(tkb_ctx *ctx, int code, const std::string &msg);

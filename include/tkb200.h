@@ -5,7 +5,8 @@
  * The library only sees flat device vectors (the `data` field of a TensorMap with
  * CuVector storage), flattened tree-transformer tables and per-block GEMM descriptors.
  * Every export returns an int status (TKB_OK = 0); nothing throws across the ABI.
- * All launches are asynchronous on the context's stream. Device pointers are borrowed
+ * All launches are asynchronous on the context's stream; host threads may share a context (what one
+ * call enqueues through its scratch is enqueued together). Device pointers are borrowed
  * for the duration of the call (until stream completion); tables, plans and graphs are
  * owned by the library and released with the matching *_destroy call.
  *

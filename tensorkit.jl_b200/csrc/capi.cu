@@ -15,12 +15,16 @@ thread_local std::string g_err;
 }
 
 int tkb_set_error(tkb_ctx *ctx, int code, const std::string &msg) {
-  if (ctx) ctx->err = msg;
+  if (ctx) {
+    std::lock_guard<std::mutex> lock(ctx->err_mu);
+    ctx->err = msg;
+  }
   g_err = msg;
   return code;
 }
 
 int tkb_ensure_workspace(tkb_ctx *ctx, size_t bytes) {
+  std::lock_guard<std::mutex> lock(ctx->launch_mu);
   if (bytes <= ctx->ws_bytes) return TKB_OK;
   if (ctx->in_capture)
     return tkb_set_error(ctx, TKB_ERR_ARG, "workspace growth requested during graph capture");
@@ -41,8 +45,11 @@ extern "C" {
 int tkb_version(void) { return 201; }
 
 const char *tkb_last_error(const tkb_ctx *ctx) {
-  if (ctx) return ctx->err.c_str();
-  return g_err.c_str();
+  if (!ctx) return g_err.c_str();
+  static thread_local std::string msg;  // the caller's own copy: other threads may set the next one
+  std::lock_guard<std::mutex> lock(ctx->err_mu);
+  msg = ctx->err;
+  return msg.c_str();
 }
 
 // releases what a context holds (null where it was not made yet)
@@ -112,6 +119,7 @@ int tkb_ctx_destroy(tkb_ctx *ctx) {
 
 int tkb_ctx_set_stream(tkb_ctx *ctx, void *stream) {
   if (!ctx) return tkb_set_error(nullptr, TKB_ERR_ARG, "null context");
+  std::lock_guard<std::mutex> lock(ctx->launch_mu);
   if (ctx->in_capture) return tkb_set_error(ctx, TKB_ERR_ARG, "cannot change stream during capture");
   ctx->stream = (cudaStream_t)stream;
   return TKB_OK;
@@ -198,7 +206,7 @@ int tkb_selftest_bounded_wait(tkb_ctx *ctx, int64_t timeout_us) {
 
 int tkb_ctx_launch_count(const tkb_ctx *ctx, int64_t *count) {
   if (!ctx || !count) return TKB_ERR_ARG;
-  *count = ctx->launches;
+  *count = ctx->launches.load();
   return TKB_OK;
 }
 
@@ -407,6 +415,7 @@ int tkb_grouped_gemm(tkb_ctx *ctx, const tkb_plan *p, void *C, const void *A, co
   if (p->owner != ctx) return tkb_set_error(ctx, TKB_ERR_ARG, "plan belongs to another context");
   if (p->nblocks > 0 && (!C || (p->flops > 0 && (!A || !B))))
     return tkb_set_error(ctx, TKB_ERR_ARG, "null data pointer");
+  std::lock_guard<std::mutex> lock(ctx->launch_mu);
   int rc = tkb_gemm_skinny_launch(ctx, p, C, A, B, alpha, beta);
   if (rc == TKB_OK) rc = tkb_gemm_thin_launch(ctx, p, C, A, B, alpha, beta);
   if (rc != TKB_OK) return rc;
@@ -459,14 +468,22 @@ int tkb_rplan_destroy(tkb_rplan *p) {
   return TKB_OK;
 }
 
-int tkb_reduce_async(tkb_ctx *ctx, const tkb_rplan *p, int kind, int dtype, const void *x,
-                     const void *y, double *dev_out) {
+// under launch_mu
+static int reduce_enqueue(tkb_ctx *ctx, const tkb_rplan *p, int kind, int dtype, const void *x,
+                          const void *y, double *dev_out) {
   if (!ctx || !p || !dev_out) return tkb_set_error(ctx, TKB_ERR_ARG, "null argument");
   if (p->owner != ctx) return tkb_set_error(ctx, TKB_ERR_ARG, "plan belongs to another context");
   if (kind < TKB_NORM2 || kind > TKB_TRACE) return tkb_set_error(ctx, TKB_ERR_ARG, "unknown reduction");
   if (dtype != TKB_F64 && dtype != TKB_C128) return tkb_set_error(ctx, TKB_ERR_ARG, "unknown dtype");
   if (p->total > 0 && (!x || (kind == TKB_INNER && !y))) return tkb_set_error(ctx, TKB_ERR_ARG, "null data");
   return tkb_reduce_launch(ctx, p, kind, dtype, x, y, dev_out);
+}
+
+int tkb_reduce_async(tkb_ctx *ctx, const tkb_rplan *p, int kind, int dtype, const void *x,
+                     const void *y, double *dev_out) {
+  if (!ctx) return tkb_set_error(nullptr, TKB_ERR_ARG, "null argument");
+  std::lock_guard<std::mutex> lock(ctx->launch_mu);
+  return reduce_enqueue(ctx, p, kind, dtype, x, y, dev_out);
 }
 
 int tkb_reduce(tkb_ctx *ctx, const tkb_rplan *p, int kind, int dtype, const void *x,
@@ -484,18 +501,27 @@ int tkb_reduce(tkb_ctx *ctx, const tkb_rplan *p, int kind, int dtype, const void
       break;
     }
   }
+  cudaStream_t st = nullptr;
   if (slot < 0) {  // every slot is held: through device memory (the last 32 bytes of the counters) and a copy
     double *dres = reinterpret_cast<double *>(ctx->counters + 32);
-    const int rc = tkb_reduce_async(ctx, p, kind, dtype, x, y, dres);
+    std::unique_lock<std::mutex> lock(ctx->launch_mu);
+    st = ctx->stream;
+    const int rc = reduce_enqueue(ctx, p, kind, dtype, x, y, dres);
     if (rc != TKB_OK) return rc;
-    TKB_CUDA_TRY(ctx, cudaMemcpyAsync(host_out, dres, 2 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    TKB_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+    TKB_CUDA_TRY(ctx, cudaMemcpyAsync(host_out, dres, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
+    lock.unlock();
+    TKB_CUDA_TRY(ctx, cudaStreamSynchronize(st));
     return TKB_OK;
   }
   double *res = ctx->host_res + 2 * slot;
-  int rc = tkb_reduce_async(ctx, p, kind, dtype, x, y, res);
+  int rc;
+  {
+    std::lock_guard<std::mutex> lock(ctx->launch_mu);
+    st = ctx->stream;
+    rc = reduce_enqueue(ctx, p, kind, dtype, x, y, res);
+  }
   if (rc == TKB_OK) {
-    const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+    const cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) rc = tkb_set_error(ctx, TKB_ERR_CUDA, std::string("reduction: ") + cudaGetErrorString(e));
   }
   if (rc == TKB_OK) {

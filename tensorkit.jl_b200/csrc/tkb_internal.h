@@ -16,7 +16,7 @@ struct tkb_ctx {
   cudaStream_t stream = nullptr;
   int num_sms = 148;
   size_t smem_optin = 227 * 1024;
-  // scratch owned by the context (grown on demand, never shrunk before destroy)
+  // scratch owned by the context (grown on demand, never shrunk before destroy; under launch_mu)
   void *ws = nullptr;
   size_t ws_bytes = 0;
   // device work-queue counters for persistent kernels (zeroed once, self-resetting)
@@ -32,7 +32,11 @@ struct tkb_ctx {
   // the lock, so that threads do not re-record it between the two
   cudaEvent_t order = nullptr;
   std::mutex order_mu;
-  int64_t launches = 0;
+  // calls of several host threads overlap: what one call enqueues through the workspace (slicing and the
+  // products that read the slices) or reads back is enqueued together
+  std::mutex launch_mu;
+  std::atomic<int64_t> launches{0};
+  mutable std::mutex err_mu;
   std::string err;
   cudaGraph_t capturing = nullptr;
   bool in_capture = false;

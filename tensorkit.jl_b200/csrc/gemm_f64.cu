@@ -91,17 +91,38 @@ __device__ __forceinline__ void dmma16(double (&c)[4], const double (&a)[4], con
                : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
                : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
+// D = A B
+__device__ __forceinline__ void dmma16_first(double (&c)[4], const double (&a)[4], const double (&b)[2]) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+               : "=d"(c[0]), "=d"(c[1]), "=d"(c[2]), "=d"(c[3])
+               : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]), "d"(0.0));
+}
 
 // ---- tiled kernel ------------------------------------------------------------------------
+// Where the products of one output value meet. One accumulator that takes every product of a long K loses more
+// in rounding than several that are added in the end (64x64 sampled values of ten products of K = 31 - 1736
+// against long double: up to 1.9 times the error of Halves real, 1.7 complex).
+//   One:    a single accumulator (64×32 complex tiles, which have no registers left)
+//   Halves: one for each half of a stage
+//   Stage:  a stage is summed from zero, then added. An FP64 addition per value and stage takes 6 % of the pipe
+//           that the DMMA need, which does not show while the launch waits for latency (32×32 real tiles)
+//   Stages: the same every fourth stage (32×32 complex tiles, which also run launches bound by the DMMA: 70.7 us
+//           for an SU(2) environment update at V dim 2406, 68.8 with One, 82.4 with Stage; Halves do not reach
+//           the error of the 64-wide tiles' shorter pieces of K)
+enum class Sum { One, Halves, Stage, Stages };
+constexpr int kSumStages = 4;
+
 // Tile shape of a kernel for elements E (double, or double2 for complex data): BMxBN output tile, warps
 // of WMxWN (m16n8k8 fragments). The pitches spread the fragments of a warp over the banks.
-template <typename E_, int BM_, int BN_, int WM_, int WN_, int NST_, int MINB_>
+template <typename E_, int BM_, int BN_, int WM_, int WN_, int NST_, int MINB_, Sum SUM_>
 struct TileCfg {
   using E = E_;
   static constexpr bool CPLX = sizeof(E) == 16;
   static constexpr int BM = BM_, BN = BN_, WM = WM_, WN = WN_, NST = NST_, MINB = MINB_;
   static constexpr int WARPS_M = BM / WM, WARPS = (BM / WM) * (BN / WN), THREADS = 32 * WARPS;
   static constexpr int MI = WM / 16, NI = WN / 8, NV = MI * NI * (CPLX ? 8 : 4);  // NV: accumulators per thread
+  static constexpr Sum SUM = SUM_;
+  static constexpr int NACC = SUM == Sum::Halves || SUM == Sum::Stages ? 2 * NV : NV;  // with the second set
   // pitches: op(A) tile [k][row], op(B) tile [col][k]
   static constexpr int PA = BM + (CPLX ? 2 : 4), PB = BK + 4;
   static constexpr int A_ELEMS = BK * PA, B_ELEMS = BN * PB, STAGE = A_ELEMS + B_ELEMS;
@@ -245,10 +266,19 @@ __device__ __forceinline__ double flip(double v, int mask) {
 
 // the products of one stage: op(A) tile sa (offset to the warp's rows), op(B) tile sb
 template <typename CFG>
-__device__ __forceinline__ void stage_products(double (&acc)[CFG::NV], const typename CFG::E *sa,
+__device__ __forceinline__ void stage_products(double (&acc)[CFG::NACC], const typename CFG::E *sa,
                                                const typename CFG::E *sb, int t, int conjA, int conjB) {
+  constexpr bool STAGE = CFG::SUM == Sum::Stage;
+  [[maybe_unused]] double fresh[STAGE ? CFG::NV : 1];
 #pragma unroll
   for (int kk = 0; kk < BK; kk += 8) {
+    const bool first = STAGE && kk == 0;
+    double *sum = STAGE ? fresh : CFG::SUM == Sum::Halves && kk > 0 ? acc + CFG::NV : acc;
+    auto product = [&](int v, const double (&a)[4], const double (&b)[2], bool from_zero) {
+      double(&c)[4] = *reinterpret_cast<double(*)[4]>(sum + v);
+      if (from_zero) dmma16_first(c, a, b);
+      else dmma16(c, a, b);
+    };
     if constexpr (!CFG::CPLX) {
       double af[CFG::MI][4], bf[CFG::NI][2];
 #pragma unroll
@@ -262,8 +292,7 @@ __device__ __forceinline__ void stage_products(double (&acc)[CFG::NV], const typ
 #pragma unroll
       for (int mi = 0; mi < CFG::MI; ++mi)
 #pragma unroll
-        for (int ni = 0; ni < CFG::NI; ++ni)
-          dmma16(*reinterpret_cast<double(*)[4]>(&acc[(mi * CFG::NI + ni) * 4]), af[mi], bf[ni]);
+        for (int ni = 0; ni < CFG::NI; ++ni) product((mi * CFG::NI + ni) * 4, af[mi], bf[ni], first);
     } else {
       double br[CFG::NI][2], bi[CFG::NI][2];
 #pragma unroll
@@ -288,18 +317,22 @@ __device__ __forceinline__ void stage_products(double (&acc)[CFG::NV], const typ
         // an accumulator
 #pragma unroll
         for (int ni = 0; ni < CFG::NI; ++ni) {
-          double *c = &acc[(mi * CFG::NI + ni) * 8];
-          dmma16(*reinterpret_cast<double(*)[4]>(c), ar, br[ni]);
-          dmma16(*reinterpret_cast<double(*)[4]>(c + 4), ar, bi[ni]);
+          const int v = (mi * CFG::NI + ni) * 8;
+          product(v, ar, br[ni], first);
+          product(v + 4, ar, bi[ni], first);
         }
 #pragma unroll
         for (int ni = 0; ni < CFG::NI; ++ni) {
-          double *c = &acc[(mi * CFG::NI + ni) * 8];
-          dmma16(*reinterpret_cast<double(*)[4]>(c), an, bi[ni]);
-          dmma16(*reinterpret_cast<double(*)[4]>(c + 4), ai, br[ni]);
+          const int v = (mi * CFG::NI + ni) * 8;
+          product(v, an, bi[ni], false);
+          product(v + 4, ai, br[ni], false);
         }
       }
     }
+  }
+  if constexpr (STAGE) {
+#pragma unroll
+    for (int q = 0; q < CFG::NV; ++q) acc[q] += fresh[q];
   }
 }
 
@@ -363,22 +396,35 @@ __global__ void __launch_bounds__(CFG::THREADS, CFG::MINB)
       conjA = blocks[task.block].opA == TKB_OP_C ? (int)0x80000000 : 0;
       conjB = blocks[task.block].opB == TKB_OP_C ? (int)0x80000000 : 0;
     }
-    double acc[CFG::NV];
+    double acc[CFG::NACC];
 #pragma unroll
-    for (int q = 0; q < CFG::NV; ++q) acc[q] = 0.0;
+    for (int q = 0; q < CFG::NACC; ++q) acc[q] = 0.0;
     const int nk = task.kind == 0 ? task.ke - task.kb : 0;
     for (int kt = 0; kt < nk; ++kt) {
       cp_async_wait<CFG::NST - 2>();
       __syncthreads();  // this stage is visible to all; every warp is done with the slot before it
       const E *st = sm + slot * CFG::STAGE;
       stage_products<CFG>(acc, st + wm + g, st + CFG::A_ELEMS + (wn + g) * CFG::PB, t, conjA, conjB);
+      if constexpr (CFG::SUM == Sum::Stages) {
+        if (kt % kSumStages == kSumStages - 1) {
+#pragma unroll
+          for (int q = 0; q < CFG::NV; ++q) {
+            acc[CFG::NV + q] += acc[q];
+            acc[q] = 0.0;
+          }
+        }
+      }
       // the refill of the slot read in the previous iteration is issued while the DMMA execute
       produce(slot == 0 ? CFG::NST - 1 : slot - 1);
       slot = slot + 1 == CFG::NST ? 0 : slot + 1;
     }
+    if constexpr (CFG::NACC > CFG::NV) {
+#pragma unroll
+      for (int q = 0; q < CFG::NV; ++q) acc[q] += acc[CFG::NV + q];
+    }
     if (ntask == 0) PL_STAMP(2);
     if (ti + 1 == t_end) pdl_trigger();
-    const bool fin = splitk_reduce<CFG::NV, CFG::THREADS>(task, acc, part, pcnt, &ticket);
+    const bool fin = splitk_reduce<CFG::NV, CFG::THREADS>(task, *reinterpret_cast<double(*)[CFG::NV]>(acc), part, pcnt, &ticket);
     if (ntask == 0) {
       PL_STAMP(3);
       PL_SET(6, 2ull * task.nsplit + (fin ? 1 : 0));
@@ -429,16 +475,16 @@ __global__ void __launch_bounds__(CFG::THREADS, CFG::MINB)
   PL_STAMP(4);
 }
 
-// LargeTile: two CTAs of four 32×32 warps per SM (194 registers; three at 168 registers ran 4096³ at
-// 32.5 instead of 33.8 TFLOP/s, eight 32×16 warps at 29.7). SmallTile: six CTAs of four 16×16 warps
+// LargeTile: two CTAs of four 32×32 warps per SM (228 registers with both accumulators; with one, three CTAs
+// at 168 registers ran 4096³ at 32.5 instead of 33.8 TFLOP/s, eight 32×16 warps at 29.7). SmallTile: six CTAs of four 16×16 warps
 // per SM, for launches whose 64×64 tiles would leave most of the chip to one CTA per SM, which spends
 // 0.87 us per K step where its DMMA take 0.52.
-using LargeTile = TileCfg<double, 64, 64, 32, 32, 3, 2>;
-using SmallTile = TileCfg<double, 32, 32, 16, 16, 3, 6>;
+using LargeTile = TileCfg<double, 64, 64, 32, 32, 3, 2, Sum::Halves>;
+using SmallTile = TileCfg<double, 32, 32, 16, 16, 3, 6, Sum::Stage>;
 // Complex fragments hold twice the values, so the large tile is half as wide (212 registers; 64×64 spills
 // at the 128 registers of two CTAs).
-using LargeTileC = TileCfg<double2, 64, 32, 32, 16, 3, 2>;
-using SmallTileC = TileCfg<double2, 32, 32, 16, 16, 3, 3>;
+using LargeTileC = TileCfg<double2, 64, 32, 32, 16, 3, 2, Sum::One>;
+using SmallTileC = TileCfg<double2, 32, 32, 16, 16, 3, 3, Sum::Stages>;
 
 // ---- skinny blocks (n, k ≤ 16): one thread per output row, op(B) in shared memory -----------
 // Such blocks (tall-skinny GEMMs against small MPO bonds) are bound by reading op(A) and

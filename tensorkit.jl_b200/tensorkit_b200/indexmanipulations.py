@@ -87,9 +87,13 @@ def device_table(ctx, tdst_space, tsrc, p, levels, planar=False):
 
 
 def _check_device(*ts):
+    """One CUDA device for all: a launch takes its context, and what it may address, from the first."""
+    dev = ts[0].data.get_device()
     for t in ts:
         if not t.data.is_cuda:
             raise RuntimeError("the B200 path needs CUDA tensors (no CPU fallback)")
+        if t.data.get_device() != dev:
+            raise RuntimeError(f"operands on different devices: {[str(x.data.device) for x in ts]}")
 
 
 def add_transform_(tdst: TensorMap, tsrc, p, table: DeviceTable, alpha=1.0, beta=0.0):

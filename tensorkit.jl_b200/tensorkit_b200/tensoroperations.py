@@ -26,8 +26,8 @@ from . import _lib as L
 from . import indexmanipulations as _im
 from . import linalg as _la
 from .backend import get_context, precision
-from .indexmanipulations import (_ONE, _ZERO, _braid_table, _current_stream, _scalar, dtype_code, permute,
-                                 permute_)
+from .indexmanipulations import (_ONE, _ZERO, _braid_table, _check_device, _current_stream, _scalar, dtype_code,
+                                 permute, permute_)
 from .linalg import gemm_plan, mul_
 from .spaces import HomSpace, SpaceMismatch
 from .tensor import AbstractTensorMap, AdjointTensorMap, TensorMap, new_tensor
@@ -258,6 +258,8 @@ def _recipe(A, pA, conjA, B, pB, conjB, pAB):
     """The recipe of a contraction, or None where the step-by-step path has to run (operands that it
     refuses, launches that are being recorded)."""
     a, b = A.data, B.data
+    if a.get_device() != b.get_device():
+        _check_device(A, B)
     if not (a.is_cuda and b.is_cuda) or a.dtype != b.dtype or _im.LAUNCH_LOG is not None or _la.FLOP_LOG is not None:
         return None, None
     ctx = get_context(a.device.index)
@@ -341,7 +343,9 @@ def tensorcontract_(C, A, pA, conjA, B, pB, conjB, pAB, alpha=1.0, beta=0.0):
     W = r.W if r is not None else tensorcontract_structure(A, pA, conjA, B, pB, conjB, pABc)
     if W != C.space:
         raise SpaceMismatch(f"incompatible spaces for tensorcontract: {W} ≠ {C.space}")
-    if r is not None and C.data.dtype == A.data.dtype and C.data.device == A.data.device:
+    if C.data.get_device() != A.data.get_device():
+        _check_device(C, A)
+    if r is not None and C.data.dtype == A.data.dtype:
         return _run_recipe(ctx, r, C, A, B, alpha, beta, True)
     if conjA:
         A, pA = _adjoint(A), adjointtensorindices(A, pA)

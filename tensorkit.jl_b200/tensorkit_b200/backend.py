@@ -266,7 +266,8 @@ def launch_count(device: int | None = None) -> int:
 
 def empty_globalcaches():
     """Counterpart of TensorKit.empty_globalcaches! (src/auxiliary/caches.jl:2-5)."""
-    from . import structure, treetransformers, fusiontrees
+    from . import structure, treetransformers, fusiontrees, spaces
+    spaces._SELECTED.clear()
     structure.sectorstructure.cache_clear()
     structure.degeneracystructure.cache_clear()
     structure.fusionblocks.cache_clear()

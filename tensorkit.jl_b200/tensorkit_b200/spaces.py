@@ -300,9 +300,15 @@ def _as_product(x, unit=None) -> ProductSpace:
     raise TypeError(type(x))
 
 
+# Selections of legs by value: permuting to and fro comes back to the same objects. A space that held its own
+# selections would hold theirs too, one more for every step of a loop x = permute(x, p).
+_SELECTED: dict = {}
+_MAX_SELECTED = 4096
+
+
 class HomSpace:
     """Space of morphisms codomain ← domain."""
-    __slots__ = ("codomain", "domain", "_h", "_dim", "_adjoint", "_selected")
+    __slots__ = ("codomain", "domain", "_h", "_dim", "_adjoint")
 
     def __init__(self, codomain, domain, unit: Sector | None = None):
         cod = _as_product(codomain, unit)
@@ -312,9 +318,8 @@ class HomSpace:
         self.codomain = cod
         self.domain = dom
         self._h = hash((cod, dom))
-        self._dim = None       # the space is immutable: dim, adjoint and selections are kept
+        self._dim = None       # the space is immutable: dim and adjoint are kept (selections in _SELECTED)
         self._adjoint = None
-        self._selected = {}
 
     # -- structure ------------------------------------------------------------------
     def numout(self):
@@ -368,14 +373,15 @@ class HomSpace:
 
     def select(self, p) -> "HomSpace":
         p1, p2 = tuple(p[0]), tuple(p[1])
-        W = self._selected.get((p1, p2))
+        key = (self, p1, p2)
+        W = _SELECTED.get(key)
         if W is None:
             cod = ProductSpace(tuple(self[n] for n in p1), self.unit())
             dom = ProductSpace(tuple(self[n].dual() for n in p2), self.unit())
             W = HomSpace(cod, dom, self.unit())
-            if len(self._selected) >= 64:
-                self._selected.clear()
-            self._selected[(p1, p2)] = W
+            if len(_SELECTED) >= _MAX_SELECTED:
+                _SELECTED.clear()
+            _SELECTED[key] = W
         return W
 
     def permute(self, p) -> "HomSpace":

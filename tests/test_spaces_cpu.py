@@ -1,10 +1,12 @@
 """Spaces across processes: hashes of text differ from one to the next, loaded spaces must not."""
+import gc
 import os
 import pickle
 import subprocess
 import sys
 
 import tensorkit_b200 as tk
+from tensorkit_b200 import spaces
 from tensorkit_b200.spaces import GradedSpace, HomSpace, ProductSpace
 
 WRITE = """
@@ -50,3 +52,29 @@ def test_fields_of_an_earlier_pickle():
     assert v == V and v.dual() == V.dual() and w == W and w.dim() == W.dim() and w.adjoint() == W.adjoint()
     s = bare(tk.SU2Irrep(twice=3), ("j2",))
     assert s == tk.SU2Irrep(twice=3) and hash(s) == hash(tk.SU2Irrep(twice=3))
+
+
+def test_permuting_to_and_fro_keeps_no_chain():
+    """A loop x = permute(x, p) comes back to the same spaces instead of making two more every time."""
+    V, P = tk.Vect({tk.U1Irrep(0): 3, tk.U1Irrep(1): 2}), tk.Vect({tk.U1Irrep(0): 1, tk.U1Irrep(1): 1})
+    W = tk.HomSpace(tk.ProductSpace([V, P]), tk.ProductSpace([V, P]))
+    live = lambda: sum(type(o) is HomSpace for o in gc.get_objects())  # noqa: E731
+    x, keep = W, W  # the first space stays alive, as the caches' keys hold it
+    x = x.permute(((1, 3), (2, 4))).permute(((1, 3), (2, 4)))
+    gc.collect()
+    before = live()
+    for _ in range(500):
+        x = x.permute(((1, 3), (2, 4)))
+        x = x.permute(((1, 3), (2, 4)))
+    gc.collect()
+    assert x == keep and live() - before <= 4
+
+
+def test_selections_are_bounded():
+    P = tk.Vect({tk.U1Irrep(0): 1})
+    for d in range(1, spaces._MAX_SELECTED + 20):
+        V = tk.Vect({tk.U1Irrep(0): d})
+        W = tk.HomSpace(tk.ProductSpace([V, P]), tk.ProductSpace([V]))
+        S = W.permute(((2, 1), (3,)))
+        assert S is W.permute(((2, 1), (3,))) and S.codomain.spaces == (P, V)
+        assert len(spaces._SELECTED) <= spaces._MAX_SELECTED

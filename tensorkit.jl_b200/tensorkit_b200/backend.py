@@ -63,6 +63,9 @@ class B200Backend:
 
 
 class _LRU(OrderedDict):
+    """The least recently used entry goes first. Lowered calls reach their entries without a lookup: they set an
+    entry's `used` instead of moving it, and eviction moves an entry so marked to the back, once per mark."""
+
     def __init__(self, maxsize, on_evict=None):
         super().__init__()
         self.maxsize = maxsize
@@ -75,15 +78,19 @@ class _LRU(OrderedDict):
             return v
         v = make()
         self[key] = v
-        if len(self) > self.maxsize:
-            _, old = self.popitem(last=False)
-            if self.on_evict:
+        while len(self) > max(1, self.maxsize):
+            k, old = self.popitem(last=False)
+            if old is v or getattr(old, "used", False):
+                old.used = False
+                self[k] = old
+            elif self.on_evict:
                 self.on_evict(old)
         return v
 
 
 class DeviceTable:
     """A flattened transformer uploaded to the device."""
+    used = False  # since the last eviction that met it (see _LRU)
 
     def __init__(self, ctx: "Context", flat, src_len, dst_len):
         self.ctx = ctx
@@ -120,6 +127,8 @@ class DeviceTable:
 
 
 class GemmPlan:
+    used = False
+
     def __init__(self, ctx: "Context", blocks, lens, dtype_code, precision_code, slices, tuning=None):
         """blocks: list of (m, n, k, offA, offB, offC, lda, ldb, ldc, opA, opB); tuning:
         (max_pieces, min_piece_steps) of the split-K decomposition, or None for the default."""

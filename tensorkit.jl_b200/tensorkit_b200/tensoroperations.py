@@ -212,7 +212,7 @@ class _Recipe:
     first (with their device tables and spaces), the GEMM plan per precision setting, and the final
     permute. It holds no data. Tables and plans belong to the context's caches; a recipe whose entries
     were evicted there is made again."""
-    __slots__ = ("W", "swap", "adj", "move", "wc", "move_c", "plans")
+    __slots__ = ("W", "swap", "adj", "move", "wc", "move_c", "plans", "used")
 
     def usable(self):
         for m in self.move:
@@ -251,6 +251,7 @@ def _make_recipe(ctx, A, pA, conjA, B, pB, conjB, pAB):
         t = _Shape(r.wc, dt)
         r.move_c = _braid_table(ctx, r.W, t, pXY, range(1, t.numind() + 1))
     r.plans = {}
+    r.used = False
     return r
 
 
@@ -269,6 +270,7 @@ def _recipe(A, pA, conjA, B, pB, conjB, pAB):
         r = _make_recipe(ctx, A, pA, conjA, B, pB, conjB, pAB)
         ctx.recipes.pop(key, None)
         ctx.recipes.get_or(key, lambda: r)
+    r.used = True
     return ctx, r
 
 
@@ -298,6 +300,7 @@ def _run_recipe(ctx, r, C, A, B, alpha, beta, keep):
         for i, m in enumerate(r.move):
             if m is not None:
                 t = moved[i]
+                m[1].used = True
                 rc = lib.tkb_treetransform(h, m[1].handle, code, t.data.data_ptr(), ops[i].data.data_ptr(), _ONE,
                                            _ZERO, m[2])
                 if rc:
@@ -311,11 +314,13 @@ def _run_recipe(ctx, r, C, A, B, alpha, beta, keep):
             if len(r.plans) >= 16:
                 r.plans.clear()
             r.plans[mode] = plan
+        plan.used = True
         al = _ONE if alpha == 1.0 else _scalar(alpha)
         be = _ZERO if beta == 0.0 else _scalar(beta)
         if r.move_c is None:
             rc = lib.tkb_grouped_gemm(h, plan.handle, out.data_ptr(), X.data.data_ptr(), Y.data.data_ptr(), al, be)
         else:
+            r.move_c.used = True
             rc = lib.tkb_grouped_gemm(h, plan.handle, D.data.data_ptr(), X.data.data_ptr(), Y.data.data_ptr(), _ONE,
                                       _ZERO)
             if rc == 0:

@@ -151,6 +151,12 @@ __device__ __forceinline__ double zero_of(double) { return 0.0; }
 __device__ __forceinline__ double2 zero_of(double2) { return make_double2(0.0, 0.0); }
 __device__ __forceinline__ double absmax(double v) { return fabs(v); }
 __device__ __forceinline__ double absmax(double2 v) { return fmax(fabs(v.x), fabs(v.y)); }
+// largest of row norms (non-negative doubles order like their bits, and a NaN is above them all): a row with
+// a NaN gives its block a norm that no slice count serves, so that the block runs in FP64, which keeps it
+__device__ __forceinline__ double norm_max(double a, double b) {
+  return __longlong_as_double(max(__double_as_longlong(a), __double_as_longlong(b)));
+}
+__device__ __forceinline__ double row_norm(double s2) { return fabs(sqrt(s2)); }  // fabs: a NaN's sign
 __device__ __forceinline__ double sq_of(double v) { return v * v; }
 __device__ __forceinline__ double sq_of(double2 v) { return fma(v.x, v.x, v.y * v.y); }
 
@@ -387,9 +393,9 @@ __device__ __forceinline__ void slice_warp_task(const SliceTask &task, const voi
         ex[r] = e;
       }
     }
-    if (rv && m > 0.0) {
+    if (rv && (m > 0.0 || s2 != s2)) {
       ebm = max(ebm, (unsigned)(e + kExpBias));
-      nrm = fmax(nrm, sqrt(s2));
+      nrm = norm_max(nrm, row_norm(s2));
     }
     // pass 2: the slices of the kept piece, then of the further pieces (read again, from L2)
     if (has) store_piece<S, CPLX, LK>(v0, op, conj, r, (int64_t)gq * LK, kfull, task.kpad, base, e);
@@ -402,7 +408,7 @@ __device__ __forceinline__ void slice_warp_task(const SliceTask &task, const voi
   }
   ebm = __reduce_max_sync(full, ebm);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) nrm = fmax(nrm, __shfl_xor_sync(full, nrm, o));
+  for (int o = 16; o > 0; o >>= 1) nrm = norm_max(nrm, __shfl_xor_sync(full, nrm, o));
   if (lane == 0 && ebm != 0u) {
     red_max_u64(&bst[4 * task.block + op], (unsigned long long)ebm);
     red_max_u64(&bst[4 * task.block + 2 + op], (unsigned long long)__double_as_longlong(nrm));
@@ -1574,9 +1580,9 @@ __device__ __forceinline__ void slice_staged(const SliceTask &task, const void *
         } else {
           ex[rr] = e;
         }
-        if (m > 0.0) {
+        if (m > 0.0 || s2 != s2) {
           ebm = (unsigned)(e + kExpBias);
-          nrm = sqrt(s2);
+          nrm = row_norm(s2);
         }
       }
     }
@@ -1584,7 +1590,7 @@ __device__ __forceinline__ void slice_staged(const SliceTask &task, const void *
     // the slices (the global reductions of many CTAs onto a few addresses stay out of the way)
     ebm = __reduce_max_sync(full, ebm);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) nrm = fmax(nrm, __shfl_xor_sync(full, nrm, o));
+    for (int o = 16; o > 0; o >>= 1) nrm = norm_max(nrm, __shfl_xor_sync(full, nrm, o));
     if (lane == 0) {
       wstat[warp] = ebm;
       wstat[2 + warp] = (unsigned long long)__double_as_longlong(nrm);

@@ -120,3 +120,25 @@ def test_small_environment_update_with_slices():
     ran = [p.last_slices()[0] for k, p in ctx.plans.items() if k[0] == "gemm" and k[-2:] == ("split", 7)]
     assert any(7 in s for s in ran)
     assert relerr(got.to_host(), ref.data) <= TOL
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("adj", [False, True])
+@pytest.mark.parametrize("m,k,n", [(200, 321, 150), (40, 7000, 33)])   # 7000: rows longer than a staged task's
+@pytest.mark.parametrize("where", ["A", "B", "row of A"])
+def test_nan_is_kept(cplx, adj, m, k, n, where):
+    """One NaN, or a row of them, makes its row (column) of the product NaN and leaves the others as they are."""
+    rng = np.random.default_rng(17)
+    rnd = lambda *s: rng.standard_normal(s) + 1j * rng.standard_normal(s) if cplx else rng.standard_normal(s)  # noqa: E731
+    a, b = rnd(m, k), rnd(k, n)
+    want = a @ b
+    if where == "B":
+        b[k - 1, 5] = want[:, 5] = np.nan
+    else:
+        a[7, slice(None) if where != "A" else 3] = want[7, :] = np.nan
+    W = O.Hom([O.Space({O.U1(0): m})], [O.Space({O.U1(0): n})])
+    Cd, _ = _mul(_dev(a, adj), _dev(b, adj), W)
+    got = Cd.to_host().reshape(n, m).T
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    ok = ~np.isnan(want)
+    assert np.abs(got - want)[ok].max() <= TOL * np.abs(want[ok]).max()

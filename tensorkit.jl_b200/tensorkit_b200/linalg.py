@@ -214,6 +214,8 @@ def inner(tx, ty):
     if isinstance(tx, AdjointTensorMap) or isinstance(ty, AdjointTensorMap):
         raise NotImplementedError("inner of lazy adjoints: materialise with permute first")
     _check_device(tx, ty)
+    if tx.data.dtype != ty.data.dtype:
+        raise TypeError("inner operands must share their scalar type")
     ctx = get_context(tx.data.device.index)
     plan = _rplan(ctx, ("norm", tx.space), lambda: _block_segments(tx.space), tx.data.numel())
     r = _reduce(ctx, plan, L.TKB_INNER, tx.data, ty.data)

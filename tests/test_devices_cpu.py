@@ -1,5 +1,6 @@
-"""Operands on different GPUs are refused on the host, before anything is enqueued: a launch takes its context from
-one operand, so another GPU's pointer would be an invalid access."""
+"""Operands that one launch cannot read together are refused on the host, before anything is enqueued: on different
+GPUs (a launch takes its context from one operand, so another GPU's pointer would be an invalid access) or of
+different scalar types (the other vector would be read as the first one's type, past its end)."""
 import pytest
 import torch
 
@@ -62,3 +63,12 @@ def test_operands_on_two_gpus_are_refused(on, monkeypatch, call):
         monkeypatch.setattr(TO, "_recipe", lambda *a: (None, r))
     with pytest.raises(RuntimeError, match="different devices"):
         CALLS[call](on(0), on(1))
+
+
+@pytest.mark.parametrize("first", [torch.float64, torch.complex128])
+def test_inner_of_two_scalar_types_is_refused(on, first):
+    x, y = on(0), on(0)
+    x.data.dtype = first
+    y.data.dtype = torch.complex128 if first == torch.float64 else torch.float64
+    with pytest.raises(TypeError, match="scalar type"):
+        tk.inner(x, y)

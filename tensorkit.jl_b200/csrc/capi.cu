@@ -30,9 +30,11 @@ int tkb_ensure_workspace(tkb_ctx *ctx, size_t bytes) {
     return tkb_set_error(ctx, TKB_ERR_ARG, "workspace growth requested during graph capture");
   // the stream may still use the old workspace
   TKB_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-  cudaFree(ctx->ws);
+  if (ctx->ws_captured) ctx->ws_retired.push_back(ctx->ws);  // a graph may still run on it
+  else cudaFree(ctx->ws);
   ctx->ws = nullptr;
   ctx->ws_bytes = 0;
+  ctx->ws_captured = false;
   const size_t nb = (bytes + 255) / 256 * 256;
   cudaError_t e = cudaMalloc(&ctx->ws, nb);
   if (e != cudaSuccess) return tkb_set_error(ctx, TKB_ERR_OOM, "workspace allocation failed");
@@ -55,6 +57,7 @@ const char *tkb_last_error(const tkb_ctx *ctx) {
 // releases what a context holds (null where it was not made yet)
 static void ctx_free(tkb_ctx *ctx) {
   cudaFree(ctx->ws);
+  for (void *ws : ctx->ws_retired) cudaFree(ws);
   cudaFree(ctx->counters);
   cudaFree(ctx->red_scratch);
   if (ctx->order) cudaEventDestroy(ctx->order);
@@ -419,7 +422,12 @@ int tkb_grouped_gemm(tkb_ctx *ctx, const tkb_plan *p, void *C, const void *A, co
   int rc = tkb_gemm_skinny_launch(ctx, p, C, A, B, alpha, beta);
   if (rc == TKB_OK) rc = tkb_gemm_thin_launch(ctx, p, C, A, B, alpha, beta);
   if (rc != TKB_OK) return rc;
-  if (p->precision == TKB_SPLIT_INT8 && !p->small_fp64) return tkb_gemm_split_launch(ctx, p, C, A, B, alpha, beta);
+  if (p->precision == TKB_SPLIT_INT8 && !p->small_fp64) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    TKB_CUDA_TRY(ctx, cudaStreamIsCapturing(ctx->stream, &cap));
+    if (cap != cudaStreamCaptureStatusNone) ctx->ws_captured = true;
+    return tkb_gemm_split_launch(ctx, p, C, A, B, alpha, beta);
+  }
   return tkb_gemm_launch(ctx, p, C, A, B, alpha, beta);
 }
 

@@ -19,6 +19,10 @@ struct tkb_ctx {
   // scratch owned by the context (grown on demand, never shrunk before destroy; under launch_mu)
   void *ws = nullptr;
   size_t ws_bytes = 0;
+  // graphs hold the address of the scratch they were captured with: once a capture has used it, growing
+  // keeps it until the context goes
+  bool ws_captured = false;
+  std::vector<void *> ws_retired;
   // device work-queue counters for persistent kernels (zeroed once, self-resetting)
   int *counters = nullptr;
   // host memory that reductions write their results to (mapped; kHostSlots results of two

@@ -88,9 +88,34 @@ class _LRU(OrderedDict):
         return v
 
 
-class DeviceTable:
+class Owned:
+    """What the library holds for a structure (`handle`), as an entry of a context's cache. A captured graph runs on
+    its device memory, so graphs pin it: an entry that leaves its cache is freed when the last pin goes."""
+    used = False      # by a lowered call since the last eviction that met it (see _LRU)
+    pins = 0
+    dropped = False   # left its cache while pinned
+
+    def drop(self):
+        if self.pins:
+            self.dropped = True
+        else:
+            self.free()
+
+    def pin(self):
+        self.pins += 1
+
+    def unpin(self):
+        self.pins -= 1
+        if self.dropped and not self.pins:
+            self.free()
+
+
+# Tables and plans that calls run are recorded here while a graph is being captured
+USE_LOG: list | None = None
+
+
+class DeviceTable(Owned):
     """A flattened transformer uploaded to the device."""
-    used = False  # since the last eviction that met it (see _LRU)
 
     def __init__(self, ctx: "Context", flat, src_len, dst_len):
         self.ctx = ctx
@@ -126,9 +151,7 @@ class DeviceTable:
             pass
 
 
-class GemmPlan:
-    used = False
-
+class GemmPlan(Owned):
     def __init__(self, ctx: "Context", blocks, lens, dtype_code, precision_code, slices, tuning=None):
         """blocks: list of (m, n, k, offA, offB, offC, lda, ldb, ldc, opA, opB); tuning:
         (max_pieces, min_piece_steps) of the split-K decomposition, or None for the default."""
@@ -183,7 +206,7 @@ class GemmPlan:
             pass
 
 
-class ReducePlan:
+class ReducePlan(Owned):
     def __init__(self, ctx: "Context", segs, length):
         """segs: list of (offset, count, stride, weight)."""
         self.ctx = ctx
@@ -230,9 +253,9 @@ class Context:
         L.check(self.lib.tkb_ctx_create(device, C.c_void_p(self.stream.cuda_stream),
                                         workspace_bytes, C.byref(h)))
         self.handle = h
-        self.tables = _LRU(_DEFAULT_CACHE, lambda t: t.free())
-        self.plans = _LRU(_DEFAULT_CACHE, lambda p: p.free())
-        self.rplans = _LRU(_DEFAULT_CACHE, lambda p: p.free())
+        self.tables = _LRU(_DEFAULT_CACHE, lambda t: t.drop())
+        self.plans = _LRU(_DEFAULT_CACHE, lambda p: p.drop())
+        self.rplans = _LRU(_DEFAULT_CACHE, lambda p: p.drop())
         # lowered calls by structure (spaces, index tuples, scalar types): which transforms and which GEMM a
         # call runs; they refer to entries of the caches above, which may be freed under them
         self.recipes = _LRU(_DEFAULT_CACHE)
@@ -249,7 +272,7 @@ class Context:
         self.recipes.clear()
         for cache in (self.tables, self.plans, self.rplans):
             for v in cache.values():
-                v.free()
+                v.drop()
             cache.clear()
 
 

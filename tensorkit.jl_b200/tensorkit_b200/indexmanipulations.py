@@ -19,6 +19,7 @@ from __future__ import annotations
 import ctypes as C
 
 from . import _lib as L
+from . import backend
 from .backend import DeviceTable, get_context
 from .spaces import SpaceMismatch
 from .tensor import AdjointTensorMap, TensorMap, new_tensor
@@ -106,6 +107,8 @@ def add_transform_(tdst: TensorMap, tsrc, p, table: DeviceTable, alpha=1.0, beta
     conj = 1 if (isinstance(tsrc, AdjointTensorMap) and tsrc.is_complex()) else 0
     if LAUNCH_LOG is not None:
         LAUNCH_LOG.append(("transform", table, tdst, tsrc, complex(alpha), complex(beta), conj))
+    if backend.USE_LOG is not None:
+        backend.USE_LOG.append(table)
     _sync_in(ctx)
     L.check(ctx.lib.tkb_treetransform(ctx.handle, table.handle, code, tdst.data.data_ptr(), tsrc.data.data_ptr(),
                                       _scalar(alpha), _scalar(beta), conj), ctx.handle)

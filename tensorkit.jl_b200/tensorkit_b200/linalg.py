@@ -14,6 +14,7 @@ import ctypes as C
 import math
 
 from . import _lib as L
+from . import backend
 from .backend import GemmPlan, ReducePlan, get_context, precision
 from .indexmanipulations import _check_device, _scalar, _sync_in, _sync_out, dtype_code, permute_
 from .spaces import SpaceMismatch
@@ -158,6 +159,8 @@ def mul_(tC: TensorMap, tA, tB, alpha=1.0, beta=0.0, prec=None, slices=None):
     from . import indexmanipulations as _im
     if _im.LAUNCH_LOG is not None:
         _im.LAUNCH_LOG.append(("gemm", plan, tC, tA, tB, complex(alpha), complex(beta)))
+    if backend.USE_LOG is not None:
+        backend.USE_LOG.append(plan)
     _sync_in(ctx)
     L.check(ctx.lib.tkb_grouped_gemm(ctx.handle, plan.handle, tC.data.data_ptr(), tA.data.data_ptr(),
                                      tB.data.data_ptr(), _scalar(alpha), _scalar(beta)), ctx.handle)

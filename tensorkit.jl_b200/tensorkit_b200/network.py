@@ -14,6 +14,7 @@ from __future__ import annotations
 import ctypes as C
 
 from . import _lib as L
+from . import backend
 from . import tensor as _tensor_mod
 from .backend import get_context, using_precision
 from .tensoroperations import tensor
@@ -32,6 +33,7 @@ class NetworkPlan:
         self.graph = None
         self.output = None
         self._buffers = []
+        self._pinned = []
         self.kernels_per_replay = 0
 
     def run_eager(self):
@@ -47,7 +49,7 @@ class NetworkPlan:
         self.ctx.stream.synchronize()
         lib = self.ctx.lib
         n0 = self.ctx.launch_count()
-        _tensor_mod._ALLOC_LOG = []
+        _tensor_mod._ALLOC_LOG, backend.USE_LOG = [], []
         try:
             with torch.cuda.stream(self.ctx.stream), using_precision(self.precision, self.slices):
                 L.check(lib.tkb_graph_begin(self.ctx.handle), self.ctx.handle)
@@ -63,7 +65,11 @@ class NetworkPlan:
                 L.check(lib.tkb_graph_end(self.ctx.handle, C.byref(g)), self.ctx.handle)
         finally:
             self._buffers = _tensor_mod._ALLOC_LOG or []
-            _tensor_mod._ALLOC_LOG = None
+            ran = backend.USE_LOG or []
+            _tensor_mod._ALLOC_LOG = backend.USE_LOG = None
+        for v in ran:
+            v.pin()
+        self._pinned += ran
         self.graph = g
         self.output = out
         self.kernels_per_replay = self.ctx.launch_count() - n0
@@ -81,6 +87,8 @@ class NetworkPlan:
             self.ctx.lib.tkb_graph_destroy(self.graph)
             self.graph = None
         self._buffers = []
+        while self._pinned:
+            self._pinned.pop().unpin()
 
     def __del__(self):
         try:

@@ -23,6 +23,7 @@ import re
 from functools import lru_cache
 
 from . import _lib as L
+from . import backend
 from . import indexmanipulations as _im
 from . import linalg as _la
 from .backend import get_context, precision
@@ -327,6 +328,10 @@ def _run_recipe(ctx, r, C, A, B, alpha, beta, keep):
                 rc = lib.tkb_treetransform(h, r.move_c.handle, code, out.data_ptr(), D.data.data_ptr(), al, be, 0)
         if rc:
             L.check(rc, h)
+        if backend.USE_LOG is not None:
+            backend.USE_LOG += [m[1] for m in r.move if m is not None] + [plan]
+            if r.move_c is not None:
+                backend.USE_LOG.append(r.move_c)
     finally:
         if joined:
             rc = lib.tkb_ctx_before(h, cur)

@@ -22,7 +22,8 @@ import ctypes as C
 import numpy as np
 
 from . import _lib as L
-from .backend import get_context
+from . import backend
+from .backend import Owned, get_context
 from .fusiontrees import braid as _braid_trees
 from .fusiontrees import split
 from .spaces import SpaceMismatch
@@ -109,7 +110,7 @@ def build_trace_table(Vsrc, p, q, src_adjoint_of=None) -> TraceFlat:
     return TraceFlat(N1 + N2, len(q1), gptr, sizes, dstr, doff, sstr, tsz, tstr, soff, coef)
 
 
-class TraceTable:
+class TraceTable(Owned):
     """A trace table uploaded to the device."""
 
     def __init__(self, ctx, flat: TraceFlat, src_len, dst_len):
@@ -169,6 +170,8 @@ def trace_permute_(tdst: TensorMap, tsrc, p, q, alpha=1.0, beta=0.0):
     conj = 1 if (isinstance(tsrc, AdjointTensorMap) and tsrc.is_complex()) else 0
     if IM.LAUNCH_LOG is not None:
         IM.LAUNCH_LOG.append(("trace", table, tdst, tsrc, complex(alpha), complex(beta), conj))
+    if backend.USE_LOG is not None:
+        backend.USE_LOG.append(table)
     _sync_in(ctx)
     L.check(ctx.lib.tkb_tracetransform(ctx.handle, table.handle, dtype_code(tdst.data),
                                        tdst.data.data_ptr(), tsrc.data.data_ptr(),

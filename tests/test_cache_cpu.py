@@ -78,3 +78,30 @@ def test_entries_of_a_lowered_contraction_stay(monkeypatch):
         recipes.get_or(("cold", k), _Entry)
     assert len(made) == 1 and r.usable() and plans["hot"].handle == 1
     assert len(tables) == 8 and len(plans) == 4 and len(recipes) == 4
+
+
+def test_pinned_entries_outlive_their_cache():
+    """What a captured graph runs on is freed when the graph goes, not when it leaves the cache."""
+    from tensorkit_b200.backend import Owned
+
+    class Table(Owned):
+        handle = 1
+
+        def free(self):
+            self.handle = None
+
+    c = _LRU(1, lambda e: e.drop())
+    a = c.get_or("a", Table)
+    a.pin()
+    a.pin()     # two graphs, or twice in one
+    b = c.get_or("b", Table)
+    c.get_or("d", Table)
+    assert a.handle == 1 and b.handle is None and list(c) == ["d"]
+    a.unpin()
+    assert a.handle == 1
+    a.unpin()
+    assert a.handle is None
+    e = c.get_or("e", Table)
+    e.pin()
+    e.unpin()
+    assert e.handle == 1  # still in its cache

@@ -1,4 +1,5 @@
-"""A captured network replays into the scratch it was captured with, whatever was planned since."""
+"""A captured network replays into the scratch and with the tables and plans it was captured with, whatever was
+planned or cleared since."""
 import pytest
 import torch
 
@@ -36,3 +37,25 @@ def test_workspace_growth_keeps_the_captured_one():
         assert bool((other == 7).all())
         assert ((Y.data - want).abs().max() / want.abs().max()).item() <= 1e-12
     plan.free()
+
+
+@pytest.mark.parametrize("prec", ["plain", "split"])
+def test_cleared_caches_keep_what_a_graph_runs_on(prec):
+    from tensorkit_b200 import backend
+    tk.empty_globalcaches()
+    A, E, ref = _network(7)
+    plan = tk.NetworkPlan(ENV, prec, A=to_device(A), E=to_device(E))
+    assert relerr(plan.replay().to_host(), ref.data) <= 1e-12
+    ctx = plan.ctx
+    ran = list(ctx.tables.values()) + [p for k, p in ctx.plans.items() if p.pins]
+    assert len(ran) == 4 and all(v.pins for v in ran)   # two permutes, two products
+    tk.empty_globalcaches()
+    assert not ctx.tables and not ctx.plans and all(v.handle is not None for v in ran)
+    again = tk.tensor(ENV, A=plan.inputs["A"], E=plan.inputs["E"])   # new tables beside the pinned ones
+    plan.output.data.zero_()
+    torch.cuda.synchronize()
+    got = plan.replay()
+    ctx.synchronize()
+    assert relerr(got.to_host(), ref.data) <= 1e-12 and relerr(again.to_host(), ref.data) <= 1e-12
+    plan.free()
+    assert all(v.handle is None for v in ran) and backend.USE_LOG is None

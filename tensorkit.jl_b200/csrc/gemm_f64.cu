@@ -932,11 +932,6 @@ int tkb_gemm_plain_prepare(tkb_ctx *ctx, tkb_plan *p) {
     tasks.insert(tasks.end(), l.begin(), l.end());
     start.push_back((int32_t)tasks.size());
   }
-  for (const auto &l : lists) {  // then the K steps of every CTA
-    int32_t n = 0;
-    for (const PTask &q : l) n += q.kind == 0 ? q.ke - q.kb : 0;
-    start.push_back(n);
-  }
   p->nptasks = (int64_t)tasks.size();
   p->pgrid = (int)lists.size();
   cudaError_t e = cudaSuccess;

@@ -446,13 +446,14 @@ int tkb_rplan_create(tkb_ctx *ctx, int64_t nseg, const int64_t *off, const int64
     if (count[s] > 0 && !tkb_segment_in_bounds(off[s], count[s], stride[s], len))
       return tkb_set_error(ctx, TKB_ERR_SIZE, "segment outside the data vector");
     segs[s] = {off[s], count[s], stride[s], weight[s]};
-    begin[s + 1] = begin[s] + count[s];
+    begin[s + 1] = begin[s] + count[s] + kRedSegPad;
   }
   tkb_rplan *p = new tkb_rplan();
   p->owner = ctx;
   p->nseg = nseg;
-  p->total = begin[nseg];
-  p->nblocks_launch = (int)std::max<int64_t>(1, std::min<int64_t>((p->total + 4095) / 4096, (int64_t)ctx->num_sms * kRedCtasPerSm));
+  p->span = begin[nseg];
+  p->total = p->span - nseg * kRedSegPad;
+  p->nblocks_launch = (int)std::max<int64_t>(1, std::min<int64_t>((p->span + 4095) / 4096, (int64_t)ctx->num_sms * kRedCtasPerSm));
   cudaError_t e = cudaSuccess;
   if (nseg > 0) {
     e = cudaMalloc((void **)&p->segs, nseg * sizeof(RSeg));

@@ -1,10 +1,14 @@
 // Weighted block reductions for norm / inner / tr (src/tensors/linalg.jl:257-282, 319-327;
 // src/tensors/vectorinterface.jl:114-130): Σ_c dim(c)·f(block_c), accumulated in FP64.
 //
-// One launch: a CTA takes a contiguous range of the segments' element space and walks the
+// One launch: a warp takes a contiguous range of the segments' element space and walks the
 // segments in it, the weight applied once per segment piece; the CTA that arrives last on a
 // counter adds the partial sums in CTA order (deterministic: which CTA that is does not
-// matter) and writes the result, to host memory where the caller waits for it.
+// matter) and writes the result, to host memory where the caller waits for it. A segment is a round trip
+// to its record and to its elements however short it is, so in the element space every segment is followed by
+// kRedSegPad places without an element, which spread many short ones (the blocks of a tensor with many
+// sectors, all diagonals of a trace) over warps and CTAs. The norm of 1001 blocks of one element takes 7 us (487
+// when the whole CTA walked them one by one), the trace of 147 blocks of 40 x 40 7 us (49).
 //
 // The counter word holds the launch's ticket above the arrivals. A CTA first raises the word to its
 // launch's ticket, so every launch counts from zero whatever an earlier one left there (launches overlap
@@ -74,15 +78,15 @@ __device__ __forceinline__ double2 block_sum(double2 v) {
   return r;
 }
 
-// Σ over n values x[i·stride] (and y), the thread's share, in independent sums
+// Σ over n values x[i·stride] (and y) of a warp, the thread's share, in independent sums
 template <int KIND, typename T, typename F>
 __device__ __forceinline__ void piece_sum(const T *__restrict__ x, const T *__restrict__ y, int64_t n, int64_t stride,
                                           Acc (&a)[kRedBatch<KIND>], F &&add) {
-  for (int64_t i0 = threadIdx.x; i0 < n; i0 += RT * kRedBatch<KIND>) {
+  for (int64_t i0 = threadIdx.x & 31; i0 < n; i0 += 32 * kRedBatch<KIND>) {
     T xv[kRedBatch<KIND>], yv[kRedBatch<KIND>];
 #pragma unroll
     for (int q = 0; q < kRedBatch<KIND>; ++q) {
-      const int64_t i = i0 + q * RT;
+      const int64_t i = i0 + q * 32;
       if (i < n) {
         xv[q] = __ldg(x + i * stride);
         yv[q] = KIND == TKB_INNER ? __ldg(y + i * stride) : xv[q];
@@ -90,35 +94,47 @@ __device__ __forceinline__ void piece_sum(const T *__restrict__ x, const T *__re
     }
 #pragma unroll
     for (int q = 0; q < kRedBatch<KIND>; ++q)
-      if (i0 + q * RT < n) add(a[q], xv[q], yv[q]);
+      if (i0 + q * 32 < n) add(a[q], xv[q], yv[q]);
   }
 }
 
 template <int KIND, typename T>
 __global__ void __launch_bounds__(RT)
-    reduce_kernel(const RSeg *__restrict__ segs, const int64_t *__restrict__ seg_begin, int64_t nseg, int64_t total,
+    reduce_kernel(const RSeg *__restrict__ segs, const int64_t *__restrict__ seg_begin, int64_t nseg, int64_t span,
                   const T *__restrict__ x, const T *__restrict__ y, double2 *__restrict__ partial,
                   unsigned long long *arrived, unsigned long long ticket, double *out) {
   __shared__ int last;
   pdl_wait();  // the vectors, the partial sums and the counter belong to earlier kernels too
   pdl_trigger();
   if (threadIdx.x == 0) atomicMax(arrived, ticket);
-  const int64_t per = (total + gridDim.x - 1) / gridDim.x;
-  const int64_t cb = (int64_t)blockIdx.x * per;
-  const int64_t ce = min(total, cb + per);
+  const int lane = threadIdx.x & 31;
+  const int64_t nwarps = (int64_t)gridDim.x * (RT / 32);
+  const int64_t per = (span + nwarps - 1) / nwarps;
+  const int64_t wb = ((int64_t)blockIdx.x * (RT / 32) + threadIdx.x / 32) * per;
+  const int64_t we = min(span, wb + per);
   double2 acc = make_double2(0.0, 0.0);
-  if (cb < ce) {
-    // the last segment that begins at or before cb and is not empty
-    int64_t lo = 0, hi = nseg - 1;
-    while (lo < hi) {
-      const int64_t mid = (lo + hi + 1) >> 1;
-      if (seg_begin[mid] <= cb) lo = mid; else hi = mid - 1;
+  if (wb < we) {
+    // the last segment that begins at or before wb, in steps of 32 candidates
+    int64_t s = 0;
+    for (int64_t left = nseg; left > 1;) {
+      const int64_t step = (left + 31) / 32, at = lane * step;
+      const unsigned before = __ballot_sync(0xffffffffu, at < left && seg_begin[s + min(at, left - 1)] <= wb);
+      const int64_t k = (31 - __clz(before)) * step;  // lane 0's candidate begins before wb
+      s += k;
+      left = min(step, left - k);
     }
-    for (int64_t s = lo; s < nseg && seg_begin[s] < ce; ++s) {
-      const int64_t b = max(cb, seg_begin[s]), e = min(ce, seg_begin[s + 1]);
+    RSeg next = segs[s];
+    int64_t next_begin = seg_begin[s];
+    for (; s < nseg && next_begin < we; ++s) {
+      const RSeg sg = next;
+      const int64_t begin = next_begin;
+      if (s + 1 < nseg) {  // the next record arrives while this segment is summed
+        next = segs[s + 1];
+        next_begin = seg_begin[s + 1];
+      }
+      const int64_t b = max(wb, begin), e = min(we, begin + sg.count);
       if (b >= e) continue;
-      const RSeg sg = segs[s];
-      const int64_t at = sg.off + (b - seg_begin[s]) * sg.stride;
+      const int64_t at = sg.off + (b - begin) * sg.stride;
       const T *xp = x + at, *yp = KIND == TKB_INNER ? y + at : xp;
       int64_t n = e - b;
       Acc a[kRedBatch<KIND>];
@@ -132,7 +148,7 @@ __global__ void __launch_bounds__(RT)
           const int head = ((uintptr_t)xp & 15) ? 1 : 0;
           const int64_t np = (n - head) / 2;
           const int tail = (int)(n - head - 2 * np);
-          if (threadIdx.x == 0) {
+          if (lane == 0) {
             if (head) one(a[0], xp[0], yp[0]);
             if (tail) one(a[0], xp[n - 1], yp[n - 1]);
           }
@@ -178,12 +194,12 @@ __global__ void __launch_bounds__(RT)
 
 template <typename T>
 cudaError_t reduce_launch(int kind, int nb, cudaStream_t st, const RSeg *segs, const int64_t *begin, int64_t nseg,
-                          int64_t total, const void *x, const void *y, double2 *partial, unsigned long long *arrived,
+                          int64_t span, const void *x, const void *y, double2 *partial, unsigned long long *arrived,
                           unsigned long long ticket, double *out) {
   auto k = kind == TKB_NORM2 ? reduce_kernel<TKB_NORM2, T>
            : kind == TKB_INNER ? reduce_kernel<TKB_INNER, T>
                                : reduce_kernel<TKB_TRACE, T>;
-  return launch_pdl(k, dim3(nb), dim3(RT), 0, st, segs, begin, nseg, total, (const T *)x, (const T *)y, partial,
+  return launch_pdl(k, dim3(nb), dim3(RT), 0, st, segs, begin, nseg, span, (const T *)x, (const T *)y, partial,
                     arrived, ticket, out);
 }
 
@@ -280,7 +296,7 @@ extern "C" int tkb_reduce_noalloc(int device, void *stream, int kind, int dtype,
         const int64_t s = s0 + q;
         segs[q] = {off[s], count[s], stride[s], weight[s]};
         begin[q] = run;
-        run += count[s];
+        run += count[s] + kRedSegPad;
       }
       begin[n] = run;
       e = cudaMemcpyAsync(dsegs + s0, segs, n * sizeof(RSeg), cudaMemcpyHostToDevice, st);
@@ -288,7 +304,7 @@ extern "C" int tkb_reduce_noalloc(int device, void *stream, int kind, int dtype,
       if (e == cudaSuccess)
         e = cudaMemcpyAsync(dbegin + s0, begin, (n + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st);
     }
-    const int nb = (int)std::max<int64_t>(1, std::min<int64_t>((total + 4095) / 4096, kNoAllocMaxCta));
+    const int nb = (int)std::min<int64_t>((run + 4095) / 4096, kNoAllocMaxCta);
     if (e == cudaSuccess) {
       // calls that overlap share the counter: each starts it anew, so that none spoils those after it
       auto *arrived = reinterpret_cast<unsigned long long *>(base + kNoAllocCountOff);
@@ -296,8 +312,8 @@ extern "C" int tkb_reduce_noalloc(int device, void *stream, int kind, int dtype,
       e = cudaMemsetAsync(arrived, 0, sizeof(*arrived), st);
       if (e == cudaSuccess)
         e = dtype == TKB_F64
-                ? reduce_launch<double>(kind, nb, st, dsegs, dbegin, nseg, total, x, y, dpart, arrived, ticket, dres)
-                : reduce_launch<double2>(kind, nb, st, dsegs, dbegin, nseg, total, x, y, dpart, arrived, ticket, dres);
+                ? reduce_launch<double>(kind, nb, st, dsegs, dbegin, nseg, run, x, y, dpart, arrived, ticket, dres)
+                : reduce_launch<double2>(kind, nb, st, dsegs, dbegin, nseg, run, x, y, dpart, arrived, ticket, dres);
     }
     if (e == cudaSuccess) {
       e = cudaGetLastError();
@@ -329,9 +345,9 @@ int tkb_reduce_launch(tkb_ctx *ctx, const tkb_rplan *p, int kind, int dtype, con
   if (cap != cudaStreamCaptureStatusNone)
     TKB_CUDA_TRY(ctx, cudaMemsetAsync(arrived, 0, sizeof(*arrived), ctx->stream));
   TKB_CUDA_TRY(ctx, dtype == TKB_F64
-                        ? reduce_launch<double>(kind, nb, ctx->stream, p->segs, p->seg_begin, p->nseg, p->total, x, y,
+                        ? reduce_launch<double>(kind, nb, ctx->stream, p->segs, p->seg_begin, p->nseg, p->span, x, y,
                                                 partial, arrived, ticket, dev_out)
-                        : reduce_launch<double2>(kind, nb, ctx->stream, p->segs, p->seg_begin, p->nseg, p->total, x, y,
+                        : reduce_launch<double2>(kind, nb, ctx->stream, p->segs, p->seg_begin, p->nseg, p->span, x, y,
                                                  partial, arrived, ticket, dev_out));
   ctx->launches++;
   TKB_CUDA_TRY(ctx, cudaGetLastError());

@@ -81,6 +81,7 @@ constexpr int kHostSlots = 64;
 // unit of a launch's ticket (above the arrivals in its counter word)
 constexpr int kRedCtasPerSm = 4, kRedSlots = 8;
 constexpr unsigned long long kRedTicket = 1ull << 24;
+constexpr int64_t kRedSegPad = 128;  // places without an element behind every segment (reduce.cu)
 
 // status helpers ------------------------------------------------------------------------
 int tkb_set_error(tkb_ctx *ctx, int code, const std::string &msg);
@@ -312,9 +313,9 @@ struct RSeg {
 struct tkb_rplan {
   tkb_ctx *owner = nullptr;
   int64_t nseg = 0;
-  int64_t total = 0;
+  int64_t total = 0, span = 0;   // elements, and places with the segments' padding
   RSeg *segs = nullptr;
-  int64_t *seg_begin = nullptr;  // prefix sums of counts (device)
+  int64_t *seg_begin = nullptr;  // first place of every segment (device)
   int nblocks_launch = 0;
 };
 

@@ -28,6 +28,7 @@
 // 489 us on a U(1) effective Hamiltonian; the DMMA wait for the loads issued before them).
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "tkb_internal.h"
 
@@ -123,9 +124,11 @@ struct TileCfg {
   static constexpr int MI = WM / 16, NI = WN / 8, NV = MI * NI * (CPLX ? 8 : 4);  // NV: accumulators per thread
   static constexpr Sum SUM = SUM_;
   static constexpr int NACC = SUM == Sum::Halves || SUM == Sum::Stages ? 2 * NV : NV;  // with the second set
-  // pitches: op(A) tile [k][row], op(B) tile [col][k]
-  static constexpr int PA = BM + (CPLX ? 2 : 4), PB = BK + 4;
-  static constexpr int A_ELEMS = BK * PA, B_ELEMS = BN * PB, STAGE = A_ELEMS + B_ELEMS;
+  // pitches of an operand's tile in a stage: [k][outer] or [outer][k] (see TileCopy)
+  static constexpr int PA = BM + (CPLX ? 2 : 4), PB = BN + (CPLX ? 2 : 4), PK = BK + 4;
+  // (op(A): [k][row] real, either complex; op(B): [col][k] real, either complex)
+  static constexpr int A_ELEMS = CPLX && BM * PK > BK * PA ? BM * PK : BK * PA;
+  static constexpr int B_ELEMS = CPLX && BK * PB > BN * PK ? BK * PB : BN * PK, STAGE = A_ELEMS + B_ELEMS;
   static constexpr size_t SMEM = (size_t)NST * STAGE * sizeof(E);
 };
 
@@ -138,7 +141,11 @@ struct TileCfg {
 //   kind 0: the tile's outer index (rows of op(A), columns of op(B)) is contiguous in memory
 //   kind 1: K is contiguous
 //   kind 2: 16-byte pairs along the contiguous direction that the stage keeps contiguous too
-template <typename E, int T, int OUTER, bool IS_A, int PITCH>
+// In the stage, real tiles are always [k][outer] (op(A), pitch PO) or [outer][k] (op(B), pitch PK). Complex tiles keep
+// the direction that is contiguous in memory contiguous: 16-byte pieces that scatter in the stage are fetched one by
+// one (an adjoint op(A) with the fixed layout: twice the L2 requests, 296 instead of 249 us for 1500 x 400 x 1500;
+// 8-byte pieces do not suffer, and a second layout made small real products 0.8 us slower).
+template <typename E, int T, int OUTER, bool IS_A, int PO, int PK>
 struct TileCopy {
   const E *p, *base;  // base: the operand's first element (where copies that read nothing point)
   int64_t dr, dk;    // elements: between the copies of a stage, between stages
@@ -154,7 +161,8 @@ struct TileCopy {
     static constexpr int W = KIND == 2 ? 2 : 1;
     static constexpr int LINE = (ALONG_K ? BK : OUTER) / W;         // threads per contiguous run
     static constexpr int DO = ALONG_K ? T / LINE : 0, DL = ALONG_K ? 0 : T / LINE;
-    static constexpr int DS = IS_A ? DL * PITCH + DO : DO * PITCH + DL;
+    static constexpr bool K_IN = sizeof(E) == 16 ? KIND == 1 : !IS_A;  // the stage is [outer][k]
+    static constexpr int DS = K_IN ? DO * PK + DL : DL * PO + DO;
     static_assert(T % LINE == 0, "whole runs per pass");
   };
   template <int KIND>
@@ -165,7 +173,7 @@ struct TileCopy {
     l0 = L::ALONG_K ? a : b;
     p = base + (o0 + oo) * so + (kbeg + l0) * sk;
     dr = L::DO * so + L::DL * sk;
-    s0 = IS_A ? l0 * PITCH + oo : oo * PITCH + l0;
+    s0 = L::K_IN ? oo * PK + l0 : l0 * PO + oo;
     o = oo;
   }
   __device__ __forceinline__ void init(const E *X, int64_t off, int64_t ld, bool outer_contig, int64_t o0,
@@ -264,10 +272,14 @@ __device__ __forceinline__ double flip(double v, int mask) {
   return __hiloint2double(__double2hiint(v) ^ mask, __double2loint(v));
 }
 
-// the products of one stage: op(A) tile sa (offset to the warp's rows), op(B) tile sb
-template <typename CFG>
+// The products of one stage: op(A) tile sa and op(B) tile sb from the thread's row i and column j on. AK, BKC: the tile
+// is [outer][k]; both layouts spread the values that a warp reads at once over all banks.
+template <typename CFG, bool AK, bool BKC>
 __device__ __forceinline__ void stage_products(double (&acc)[CFG::NACC], const typename CFG::E *sa,
-                                               const typename CFG::E *sb, int t, int conjA, int conjB) {
+                                               const typename CFG::E *sb, int i, int j, int t, int conjA, int conjB) {
+  constexpr int AR = AK ? CFG::PK : 1, AL = AK ? 1 : CFG::PA, BC = BKC ? CFG::PK : 1, BL = BKC ? 1 : CFG::PB;
+  sa += i * AR + t * AL;
+  sb += j * BC + t * BL;
   constexpr bool STAGE = CFG::SUM == Sum::Stage;
   [[maybe_unused]] double fresh[STAGE ? CFG::NV : 1];
 #pragma unroll
@@ -284,11 +296,11 @@ __device__ __forceinline__ void stage_products(double (&acc)[CFG::NACC], const t
 #pragma unroll
       for (int mi = 0; mi < CFG::MI; ++mi)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) af[mi][q] = sa[(kk + t + 4 * (q >> 1)) * CFG::PA + mi * 16 + 8 * (q & 1)];
+        for (int q = 0; q < 4; ++q) af[mi][q] = sa[(kk + 4 * (q >> 1)) * AL + (mi * 16 + 8 * (q & 1)) * AR];
 #pragma unroll
       for (int ni = 0; ni < CFG::NI; ++ni)
 #pragma unroll
-        for (int q = 0; q < 2; ++q) bf[ni][q] = sb[ni * 8 * CFG::PB + kk + t + 4 * q];
+        for (int q = 0; q < 2; ++q) bf[ni][q] = sb[ni * 8 * BC + (kk + 4 * q) * BL];
 #pragma unroll
       for (int mi = 0; mi < CFG::MI; ++mi)
 #pragma unroll
@@ -299,7 +311,7 @@ __device__ __forceinline__ void stage_products(double (&acc)[CFG::NACC], const t
       for (int ni = 0; ni < CFG::NI; ++ni)
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-          const double2 v = sb[ni * 8 * CFG::PB + kk + t + 4 * q];
+          const double2 v = sb[ni * 8 * BC + (kk + 4 * q) * BL];
           br[ni][q] = v.x;
           bi[ni][q] = flip(v.y, conjB);
         }
@@ -308,7 +320,7 @@ __device__ __forceinline__ void stage_products(double (&acc)[CFG::NACC], const t
         double ar[4], ai[4], an[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const double2 v = sa[(kk + t + 4 * (q >> 1)) * CFG::PA + mi * 16 + 8 * (q & 1)];
+          const double2 v = sa[(kk + 4 * (q >> 1)) * AL + (mi * 16 + 8 * (q & 1)) * AR];
           ar[q] = v.x;
           ai[q] = flip(v.y, conjA);
           an[q] = flip(ai[q], (int)0x80000000);
@@ -354,8 +366,8 @@ __global__ void __launch_bounds__(CFG::THREADS, CFG::MINB)
   const int t_begin = start[blockIdx.x], t_end = start[blockIdx.x + 1];
   // The stages of all the CTA's tasks form one stream through the ring: the copies run NST − 1 stages
   // ahead of the products and go on into the next task while this one finishes.
-  TileCopy<E, CFG::THREADS, CFG::BM, true, CFG::PA> ca;
-  TileCopy<E, CFG::THREADS, CFG::BN, false, CFG::PB> cb;
+  TileCopy<E, CFG::THREADS, CFG::BM, true, CFG::PA, CFG::PK> ca;
+  TileCopy<E, CFG::THREADS, CFG::BN, false, CFG::PB, CFG::PK> cb;
   int next = t_begin, ahead = 0;  // the next task to copy, stages of the current one not yet copied
   int64_t left = 0;               // K positions of its block from the next stage on
   auto advance = [&]() {
@@ -400,23 +412,40 @@ __global__ void __launch_bounds__(CFG::THREADS, CFG::MINB)
 #pragma unroll
     for (int q = 0; q < CFG::NACC; ++q) acc[q] = 0.0;
     const int nk = task.kind == 0 ? task.ke - task.kb : 0;
-    for (int kt = 0; kt < nk; ++kt) {
-      cp_async_wait<CFG::NST - 2>();
-      __syncthreads();  // this stage is visible to all; every warp is done with the slot before it
-      const E *st = sm + slot * CFG::STAGE;
-      stage_products<CFG>(acc, st + wm + g, st + CFG::A_ELEMS + (wn + g) * CFG::PB, t, conjA, conjB);
-      if constexpr (CFG::SUM == Sum::Stages) {
-        if (kt % kSumStages == kSumStages - 1) {
+    auto k_loop = [&](auto ak, auto bk) {  // one loop per pair of layouts: no test inside
+      for (int kt = 0; kt < nk; ++kt) {
+        cp_async_wait<CFG::NST - 2>();
+        __syncthreads();  // this stage is visible to all; every warp is done with the slot before it
+        const E *st = sm + slot * CFG::STAGE;
+        stage_products<CFG, decltype(ak)::value, decltype(bk)::value>(acc, st, st + CFG::A_ELEMS, wm + g, wn + g, t,
+                                                                      conjA, conjB);
+        if constexpr (CFG::SUM == Sum::Stages) {
+          if (kt % kSumStages == kSumStages - 1) {
 #pragma unroll
-          for (int q = 0; q < CFG::NV; ++q) {
-            acc[CFG::NV + q] += acc[q];
-            acc[q] = 0.0;
+            for (int q = 0; q < CFG::NV; ++q) {
+              acc[CFG::NV + q] += acc[q];
+              acc[q] = 0.0;
+            }
           }
         }
+        // the refill of the slot read in the previous iteration is issued while the DMMA execute
+        produce(slot == 0 ? CFG::NST - 1 : slot - 1);
+        slot = slot + 1 == CFG::NST ? 0 : slot + 1;
       }
-      // the refill of the slot read in the previous iteration is issued while the DMMA execute
-      produce(slot == 0 ? CFG::NST - 1 : slot - 1);
-      slot = slot + 1 == CFG::NST ? 0 : slot + 1;
+    };
+    constexpr std::true_type yes{};
+    constexpr std::false_type no{};
+    if constexpr (!CFG::CPLX) {
+      k_loop(no, yes);
+    } else {
+      const bool ak = blocks[task.block].opA != TKB_OP_N, bk = blocks[task.block].opB == TKB_OP_N;
+      if (bk) {
+        if (!ak) k_loop(no, yes);
+        else k_loop(yes, yes);
+      } else {
+        if (!ak) k_loop(no, no);
+        else k_loop(yes, no);
+      }
     }
     if constexpr (CFG::NACC > CFG::NV) {
 #pragma unroll

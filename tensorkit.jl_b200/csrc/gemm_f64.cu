@@ -810,18 +810,24 @@ int tkb_gemm_thin_launch(tkb_ctx *ctx, const tkb_plan *p, void *C, const void *A
 }
 
 // Work decomposition of a plain GEMM: the tile shape and the tasks of every CTA.
-// - SmallTile runs while its tiles are at most 1.5 per SM: an SU(2) environment update (two products and
-// two permutes) takes 10.3 instead of 14.4 us at V dim 280, 15.9 instead of 22.8 at 870, 22.7
-// instead of 26.7 at 1816 (155 tiles), but 34.9 instead of 32.8 at 2410 (290 tiles). Complex launches
-// keep it up to 16 tiles per SM: 142.9 instead of 162.7 us at V dim 3632 (620 tiles and 310 of
-// 64×32), but 30.6 instead of 32.1 TFLOP/s on one 2048³ block (4096 tiles).
+// - Real: LargeTile runs where its tiles, cut in K as far as they may be, fill the chip (at least 0.85 pieces
+//   per resident CTA) and padding to it costs at most a fifth more K steps than padding to SmallTile. us, large /
+//   small: one 60x2400x2400 block (304 pieces) 37 / 45, 120x1200x1200 24 / 27, 1000x20x1000 (256) 7.0 / 9.4,
+//   512x100x512 (128) 11.9 / 7.6, 200x5000x100 (64) 46 / 29, 30 blocks of 70 (1.8 times the steps) 11.1 / 6.5,
+//   heff of V dim 750 (1.23 times) 21.5 / 19.8, 6 blocks of 300 27 / 25.
+// - Complex: SmallTileC runs up to 16 tiles per SM, LargeTileC above (2048^3: 30.6 and 32.7 TFLOP/s). Between 6 and 16
+//   tiles per SM the large one is up to a tenth faster, but it has one accumulator and fewer pieces of K.
 // - Fewer tiles than resident CTAs: the K loops of the longest tiles are cut into equal pieces of the
 //   shortest length (at least min_piece_steps K steps) whose count still fits, one task per CTA.
-// - Otherwise every CTA gets an equal share of all K steps (plus tile_cost steps per tile for its
+// - Otherwise, and where those pieces would leave a tenth of the CTAs or more without one although the work is long
+//   (24 steps of the small tile for everyone) and the tiles may be cut fine enough, every CTA gets an equal share of
+//   all K steps (plus tile_cost steps per tile for its
 //   epilogue), as a contiguous range of the tiles in order of falling K; a tile that a share ends in
 //   is cut there. Whole tiles alone leave CTAs idle for up to a tile each: on a U(1) effective
 //   Hamiltonian's second product (394 tiles of up to 109 steps for 296 CTAs) SMs were active for
-//   70 % of the launch. A CTA runs its cut tiles first, so their partial sums meet while it goes on.
+//   70 % of the launch. A CTA runs its cut tiles first, so their partial sums meet while it goes on. One complex
+//   60x2400x2400 block (300 equal pieces for 444 CTAs) takes 112 us in shares and 158 in pieces, 257x1736x400 67 and
+//   80; shorter work loses (512^3 48 and 44, 18 steps each; ten blocks of 150 22 and 17, 6 steps each).
 
 namespace {
 struct PlainKernel {
@@ -850,10 +856,25 @@ cudaError_t plain_launch(tkb_ctx *ctx, const tkb_plan *p, void *C, const void *A
 
 int tkb_gemm_plain_prepare(tkb_ctx *ctx, tkb_plan *p) {
   const bool cplx = p->dtype == TKB_C128;
-  int64_t small_tiles = 0;
-  for (const GBlock &b : p->hblocks)
-    if (!b.skinny) small_tiles += ((b.m + 31) / 32) * ((b.n + 31) / 32);
-  p->plain_small = cplx ? small_tiles <= (int64_t)ctx->num_sms * 16 : small_tiles * 2 <= (int64_t)ctx->num_sms * 3;
+  auto tiles_of = [](const GBlock &b, const PlainKernel &k) { return ((b.m + k.bm - 1) / k.bm) * ((b.n + k.bn - 1) / k.bn); };
+  const PlainKernel large = plain_kernel(cplx, false), small = plain_kernel(cplx, true);
+  int64_t small_tiles = 0, small_steps = 0, large_steps = 0, large_pieces = 0;
+  for (const GBlock &b : p->hblocks) {
+    if (b.skinny) continue;
+    const int64_t nk = (b.k + BK - 1) / BK, tl = tiles_of(b, large), ts = tiles_of(b, small);
+    small_tiles += ts;
+    small_steps += ts * nk;
+    large_steps += tl * nk;
+    large_pieces += tl * std::min<int64_t>(p->max_pieces, std::max<int64_t>(1, (nk + p->min_piece_steps - 1) / p->min_piece_steps));
+  }
+  if (cplx) {
+    p->plain_small = small_tiles <= (int64_t)ctx->num_sms * 16;
+  } else {
+    const int large_sm = tkb_occupancy(ctx->device, large.fn, large.threads, large.smem);
+    const bool fills = large_pieces * 20 >= (int64_t)ctx->num_sms * large_sm * 17;
+    const bool padded = large_steps * 4 * 5 > small_steps * 6;  // a step of the large tile is four of the small one
+    p->plain_small = !fills || padded;
+  }
   const PlainKernel pk = plain_kernel(cplx, p->plain_small);
   const int tm = pk.bm, tn = pk.bn;
   // a piece's partial sums cost as much as twice as many steps of the smaller tile; a complex step is
@@ -884,16 +905,20 @@ int tkb_gemm_plain_prepare(tkb_ctx *ctx, tkb_plan *p) {
   }
   std::vector<std::vector<PTask>> lists;  // per CTA
   int nslots = 0, npart = 0;
+  auto pieces = [&](int64_t nk, int64_t target) {
+    return (int)std::min<int64_t>(p->max_pieces, std::max<int64_t>(1, (nk + target - 1) / target));
+  };
+  int64_t target = std::max<int64_t>(min_steps, (total + slots - 1) / slots), cnt = nt;
   if (nt < slots) {
-    auto pieces = [&](int64_t nk, int64_t target) {
-      return (int)std::min<int64_t>(p->max_pieces, std::max<int64_t>(1, (nk + target - 1) / target));
-    };
-    int64_t target = std::max<int64_t>(min_steps, (total + slots - 1) / slots);
-    for (; target < maxnk; ++target) {
-      int64_t cnt = 0;
+    for (;; ++target) {
+      cnt = 0;
       for (int64_t i = 0; i < nt; ++i) cnt += pieces(nks[i], target);
-      if (cnt <= slots) break;
+      if (cnt <= slots || target >= maxnk) break;
     }
+  }
+  const bool shares = nt >= slots || (cnt * 10 < slots * 9 && nt * p->max_pieces * 2 >= slots * 3 &&
+                                      total >= slots * (p->plain_small ? 24 : 12));
+  if (!shares) {
     for (int64_t i = 0; i < nt; ++i) {
       const GTile &t = tiles[i];
       const int nk = (int)nks[i];

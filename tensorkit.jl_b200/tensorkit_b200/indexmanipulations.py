@@ -89,11 +89,11 @@ def device_table(ctx, tdst_space, tsrc, p, levels, planar=False):
 
 def _check_device(*ts):
     """One CUDA device for all: a launch takes its context, and what it may address, from the first."""
-    dev = ts[0].data.get_device()
+    dev = ts[0].data.get_device()  # negative on the CPU
     for t in ts:
-        if not t.data.is_cuda:
-            raise RuntimeError("the B200 path needs CUDA tensors (no CPU fallback)")
-        if t.data.get_device() != dev:
+        if dev < 0 or t.data.get_device() != dev:
+            if not all(x.data.is_cuda for x in ts):
+                raise RuntimeError("the B200 path needs CUDA tensors (no CPU fallback)")
             raise RuntimeError(f"operands on different devices: {[str(x.data.device) for x in ts]}")
 
 

@@ -152,7 +152,7 @@ def mul_(tC: TensorMap, tA, tB, alpha=1.0, beta=0.0, prec=None, slices=None):
     _check_device(tC, tA, tB)
     if not (tA.data.dtype == tB.data.dtype == tC.data.dtype):
         raise TypeError("mul! operands must share their scalar type")
-    ctx = get_context(tC.data.device.index)
+    ctx = get_context(tC.data.get_device())
     plan = gemm_plan(ctx, tC, tA, tB, prec, slices)
     if FLOP_LOG is not None:
         FLOP_LOG.append(plan.flops)
@@ -204,7 +204,7 @@ def _tensor_data_space(t):
 def norm(t) -> float:
     data, W, _ = _tensor_data_space(t)
     _check_device(t)
-    ctx = get_context(data.device.index)
+    ctx = get_context(data.get_device())
     plan = _rplan(ctx, ("norm", W), lambda: _block_segments(W), data.numel())
     r = _reduce(ctx, plan, L.TKB_NORM2, data)
     return math.sqrt(max(r[0], 0.0))
@@ -219,7 +219,7 @@ def inner(tx, ty):
     _check_device(tx, ty)
     if tx.data.dtype != ty.data.dtype:
         raise TypeError("inner operands must share their scalar type")
-    ctx = get_context(tx.data.device.index)
+    ctx = get_context(tx.data.get_device())
     plan = _rplan(ctx, ("norm", tx.space), lambda: _block_segments(tx.space), tx.data.numel())
     r = _reduce(ctx, plan, L.TKB_INNER, tx.data, ty.data)
     return complex(r[0], r[1]) if tx.is_complex() else float(r[0])
@@ -233,7 +233,7 @@ def tr(t):
         raise SpaceMismatch("Trace of a tensor only exist when domain == codomain")
     data, W, isadj = _tensor_data_space(t)
     _check_device(t)
-    ctx = get_context(data.device.index)
+    ctx = get_context(data.get_device())
     plan = _rplan(ctx, ("tr", W), lambda: [(a, d1, d1 + 1, float(c.dim()))
                                            for c, ((d1, d2), (a, _)) in blockstructure(W).items()], data.numel())
     r = _reduce(ctx, plan, L.TKB_TRACE, data)
@@ -249,7 +249,7 @@ def _axpby(ty: TensorMap, tx: TensorMap, alpha, beta):
     if ty.data.dtype != tx.data.dtype:
         raise TypeError("source and destination must share their scalar type")
     code = dtype_code(ty.data)
-    ctx = get_context(ty.data.device.index)
+    ctx = get_context(ty.data.get_device())
     _sync_in(ctx)
     L.check(ctx.lib.tkb_axpby(ctx.handle, code, ty.data.numel(), ty.data.data_ptr(), tx.data.data_ptr(),
                               _scalar(alpha), _scalar(beta)), ctx.handle)

@@ -300,15 +300,15 @@ def _as_product(x, unit=None) -> ProductSpace:
     raise TypeError(type(x))
 
 
-# Selections of legs by value: permuting to and fro comes back to the same objects. A space that held its own
-# selections would hold theirs too, one more for every step of a loop x = permute(x, p).
+# Selections of legs by value: permuting to and fro comes back to the same objects. Spaces that each made and kept
+# selections of their own would hold one more for every step of a loop x = permute(x, p).
 _SELECTED: dict = {}
 _MAX_SELECTED = 4096
 
 
 class HomSpace:
     """Space of morphisms codomain ← domain."""
-    __slots__ = ("codomain", "domain", "_h", "_dim", "_adjoint")
+    __slots__ = ("codomain", "domain", "_h", "_dim", "_adjoint", "_selected")
 
     def __init__(self, codomain, domain, unit: Sector | None = None):
         cod = _as_product(codomain, unit)
@@ -318,8 +318,9 @@ class HomSpace:
         self.codomain = cod
         self.domain = dom
         self._h = hash((cod, dom))
-        self._dim = None       # the space is immutable: dim and adjoint are kept (selections in _SELECTED)
+        self._dim = None       # the space is immutable: dim, adjoint and selections are kept
         self._adjoint = None
+        self._selected = {}    # from _SELECTED, without comparing this space with an equal one there
 
     # -- structure ------------------------------------------------------------------
     def numout(self):
@@ -373,15 +374,20 @@ class HomSpace:
 
     def select(self, p) -> "HomSpace":
         p1, p2 = tuple(p[0]), tuple(p[1])
-        key = (self, p1, p2)
-        W = _SELECTED.get(key)
+        W = self._selected.get((p1, p2))
         if W is None:
-            cod = ProductSpace(tuple(self[n] for n in p1), self.unit())
-            dom = ProductSpace(tuple(self[n].dual() for n in p2), self.unit())
-            W = HomSpace(cod, dom, self.unit())
-            if len(_SELECTED) >= _MAX_SELECTED:
-                _SELECTED.clear()
-            _SELECTED[key] = W
+            key = (self, p1, p2)
+            W = _SELECTED.get(key)
+            if W is None:
+                cod = ProductSpace(tuple(self[n] for n in p1), self.unit())
+                dom = ProductSpace(tuple(self[n].dual() for n in p2), self.unit())
+                W = HomSpace(cod, dom, self.unit())
+                if len(_SELECTED) >= _MAX_SELECTED:
+                    _SELECTED.clear()
+                _SELECTED[key] = W
+            if len(self._selected) >= 64:
+                self._selected.clear()
+            self._selected[(p1, p2)] = W
         return W
 
     def permute(self, p) -> "HomSpace":

@@ -260,11 +260,12 @@ def _recipe(A, pA, conjA, B, pB, conjB, pAB):
     """The recipe of a contraction, or None where the step-by-step path has to run (operands that it
     refuses, launches that are being recorded)."""
     a, b = A.data, B.data
-    if a.get_device() != b.get_device():
+    dev = a.get_device()
+    if dev != b.get_device():
         _check_device(A, B)
-    if not (a.is_cuda and b.is_cuda) or a.dtype != b.dtype or _im.LAUNCH_LOG is not None or _la.FLOP_LOG is not None:
+    if dev < 0 or a.dtype != b.dtype or _im.LAUNCH_LOG is not None or _la.FLOP_LOG is not None:
         return None, None
-    ctx = get_context(a.device.index)
+    ctx = get_context(dev)
     key = (A.space, type(A), pA, conjA, B.space, type(B), pB, conjB, pAB, a.dtype)
     r = ctx.recipes.get(key)
     if r is None or not r.usable():

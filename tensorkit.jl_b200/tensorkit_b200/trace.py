@@ -161,7 +161,7 @@ def trace_permute_(tdst: TensorMap, tsrc, p, q, alpha=1.0, beta=0.0):
     _check_device(tdst, tsrc)
     if tdst.data.dtype != tsrc.data.dtype:
         raise TypeError("source and destination must share their scalar type")
-    ctx = get_context(tdst.data.device.index)
+    ctx = get_context(tdst.data.get_device())
     parent = tsrc.parent.space if isinstance(tsrc, AdjointTensorMap) else None
     src_len = parent.dim() if parent is not None else W.dim()
     key = ("trace", tdst.space, W, p, q, parent)

@@ -64,6 +64,9 @@ int tkb_version(void);
  * the context for split-precision operands (grown on demand). */
 int tkb_ctx_create(int device, void *stream, size_t workspace_bytes, tkb_ctx **out);
 int tkb_ctx_destroy(tkb_ctx *ctx);
+/* Later calls go to `stream`; what was enqueued stays where it is. Products run on the context's and the
+ * plans' scratch: where those of the old stream may still run, let the new one wait first
+ * (tkb_ctx_before). Reductions that overlap keep apart by themselves. */
 int tkb_ctx_set_stream(tkb_ctx *ctx, void *stream);
 /* Stream ordering for callers whose data lives on a stream of their own: later work of the context
  * waits for what `stream` holds now (tkb_ctx_after), later work on `stream` waits for what the context

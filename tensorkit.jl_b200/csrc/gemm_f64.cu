@@ -5,8 +5,8 @@
 // f64 kind, so the double-precision tensor pipe is reached through DMMA; the split-precision
 // path (gemm_split.cu) is the tcgen05 one.
 //
-// Work decomposition (tkb_gemm_plain_prepare): 64×64 output tiles (32×32 where those would leave most
-// of the chip idle), whose K loops are cut into pieces (split K) where that evens out the CTAs'
+// Work decomposition (tkb_gemm_plain_prepare): 64×64 output tiles (64×32 complex; 32×32 where those would leave
+// part of the chip idle), whose K loops are cut into pieces (split K) where that evens out the CTAs'
 // shares. Every CTA has a fixed list of tasks (tile, K range). A piece of a split tile stores its
 // FP64 partial tile; the piece that arrives last on the tile's counter adds all partials in piece
 // order (deterministic, no piece waits for another) and applies α, β.
@@ -22,9 +22,9 @@
 // What bounds it: the DMMA pipe runs m16n8k8 at 64 cycles per SM sub-partition (37 TFLOP/s measured on
 // B200), and every instruction issued beside it costs: with addresses and bounds resolved once per
 // task one 4096³ block runs at 33.5 TFLOP/s (30.1 when each copy worked out its own address), one
-// 4095³ block (8-byte copies) at 33.0 (26.8). The epilogue keeps one pointer per column of a thread:
-// 9 blocks of K ≤ 256 and a 59 MB output take 152 us (176 with an address per element, 37 us of it in
-// the epilogues). Taken back: fragments of the next sub-step loaded ahead of the DMMA (517 instead of
+// 4095³ block (8-byte copies) at 32.5 (26.8), one complex 2048³ block at 32.8 (30.4). The epilogue
+// keeps one pointer per column of a thread: 9 blocks of K ≤ 256 and a 59 MB output take 152 us (176 with an
+// address per element, 37 us of it in the epilogues). Taken back: fragments of the next sub-step loaded ahead of the DMMA (517 instead of
 // 489 us on a U(1) effective Hamiltonian; the DMMA wait for the loads issued before them).
 #include <algorithm>
 #include <cstring>
@@ -40,7 +40,7 @@ struct CDbl {
   double x, y;
 };
 
-// one task of the plain kernels: a 64×64 output tile and a range of its K steps
+// one task of the plain kernels: an output tile and a range of its K steps
 struct PTask {
   int32_t block, m0, n0, kind;  // kind 0: products, 1: β-scale only (k = 0)
   int32_t kb, ke;               // K steps [kb, ke) of BK
@@ -108,8 +108,7 @@ __device__ __forceinline__ void dmma16_first(double (&c)[4], const double (&a)[4
 //   Stage:  a stage is summed from zero, then added. An FP64 addition per value and stage takes 6 % of the pipe
 //           that the DMMA need, which does not show while the launch waits for latency (32×32 real tiles)
 //   Stages: the same every fourth stage (32×32 complex tiles, which also run launches bound by the DMMA: 70.7 us
-//           for an SU(2) environment update at V dim 2406, 68.8 with One, 82.4 with Stage; Halves do not reach
-//           the error of the 64-wide tiles' shorter pieces of K)
+//           for an SU(2) environment update at V dim 2406, 68.8 with One, 82.4 with Stage)
 enum class Sum { One, Halves, Stage, Stages };
 constexpr int kSumStages = 4;
 
@@ -522,7 +521,7 @@ __global__ void __launch_bounds__(CFG::THREADS, CFG::MINB)
   PL_STAMP(4);
 }
 
-// LargeTile: two CTAs of four 32×32 warps per SM (228 registers with both accumulators; with one, three CTAs
+// LargeTile: two CTAs of four 32×32 warps per SM (240 registers with both accumulators; with one, three CTAs
 // at 168 registers ran 4096³ at 32.5 instead of 33.8 TFLOP/s, eight 32×16 warps at 29.7). SmallTile: six CTAs of four 16×16 warps
 // per SM, for launches whose 64×64 tiles would leave most of the chip to one CTA per SM, which spends
 // 0.87 us per K step where its DMMA take 0.52.

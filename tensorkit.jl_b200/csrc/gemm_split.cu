@@ -1934,12 +1934,11 @@ int tkb_gemm_split_prepare(tkb_ctx *ctx, tkb_plan *p) {
     return p->hblocks[x.block].kpad > p->hblocks[y.block].kpad;
   });
   // products items in pairs, one pair per two-CTA cluster of the persistent kernel: a split tile
-  // (its two K halves, one per CTA) or two unsplit tiles (the second may be empty). As many of the
-  // longest tiles are split as keep the pairs within one cluster round (num_sms / 2 pairs), when
+  // (its two K halves, one per CTA) or two unsplit tiles (the second may be empty). Tiles are split where
   // the decomposition allows it (max_pieces ≥ 2, halves of at least min_piece_steps stages). A tile
   // whose K needs more than one exact piece (int32 accumulators stay exact over (2^31 − 1)/(S·127²)
   // K positions) is split in any case; a block whose K needs more than two runs in FP64.
-  // Beyond one round the splits even out the clusters' lists: the items are dealt longest first, and
+  // The splits fill the clusters and even out their lists: the items are dealt longest first, and
   // the number of tiles to split is the one that leaves the busiest cluster least (in K stages, with the
   // epilogue's part that the next item waits for: about 6 stages of 1.05 us, 8 with the exchange). The
   // second product of a U(1) effective Hamiltonian (212 tiles of up to 55 stages) takes 100 us (117 with

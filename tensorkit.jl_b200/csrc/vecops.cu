@@ -3,9 +3,9 @@
 // transform table is involved: one pass over flat vectors.
 //
 // Bound: HBM. A thread keeps four 16-byte accesses of x (and of y when β ≠ 0) in flight; vectors
-// that are not 16-byte aligned take 8-byte accesses. On 10.6 M doubles
-// (SU(2) two-site tensor, cold caches): β = 0 21 us, β = 1 32.5 us (7.8 TB/s of L2 and HBM); as an
-// identity permutation through the transform table 101 and 149 us.
+// that are not 16-byte aligned take 8-byte accesses. On 10.6 M doubles (SU(2) two-site tensor, caches cold
+// at the start): β = 0 21.5 us, β = 1 32.5 us (part of the 85 MB written is still in L2 at the end: the HBM copy
+// rate would take 25.9 and 38.8); as an identity permutation through the transform table 101 and 149 us.
 #include <algorithm>
 
 #include "tkb_internal.h"

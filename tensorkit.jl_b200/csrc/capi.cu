@@ -44,7 +44,7 @@ int tkb_ensure_workspace(tkb_ctx *ctx, size_t bytes) {
 
 extern "C" {
 
-int tkb_version(void) { return 201; }
+int tkb_version(void) { return 202; }
 
 const char *tkb_last_error(const tkb_ctx *ctx) {
   if (!ctx) return g_err.c_str();

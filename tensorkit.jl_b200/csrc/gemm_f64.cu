@@ -122,6 +122,7 @@ struct TileCfg {
   static constexpr int WARPS_M = BM / WM, WARPS = (BM / WM) * (BN / WN), THREADS = 32 * WARPS;
   static constexpr int MI = WM / 16, NI = WN / 8, NV = MI * NI * (CPLX ? 8 : 4);  // NV: accumulators per thread
   static constexpr Sum SUM = SUM_;
+  static constexpr bool BETA_KERNEL = SUM != Sum::One;  // kernels of their own without and with β
   static constexpr int NACC = SUM == Sum::Halves || SUM == Sum::Stages ? 2 * NV : NV;  // with the second set
   // pitches of an operand's tile in a stage: [k][outer] or [outer][k] (see TileCopy)
   static constexpr int PA = BM + (CPLX ? 2 : 4), PB = BN + (CPLX ? 2 : 4), PK = BK + 4;
@@ -347,7 +348,10 @@ __device__ __forceinline__ void stage_products(double (&acc)[CFG::NACC], const t
   }
 }
 
-template <typename CFG>
+// BZ: β = 0 and the output is not read, in a kernel of its own (products of the sweeps 2 % faster, SU(2) update 51.2 ->
+// 50.6 us). LargeTileC runs one kernel for both: alone, its β = 0 code came out at 194 registers instead of 226
+// and one 2048³ block at 30.8 instead of 32.7 TFLOP/s.
+template <typename CFG, bool BZ>
 __global__ void __launch_bounds__(CFG::THREADS, CFG::MINB)
     gemm_plain_kernel(const GBlock *__restrict__ blocks, const PTask *__restrict__ tasks,
                       const int32_t *__restrict__ start, typename CFG::E *__restrict__ C,
@@ -361,7 +365,6 @@ __global__ void __launch_bounds__(CFG::THREADS, CFG::MINB)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wm = (warp % CFG::WARPS_M) * CFG::WM, wn = (warp / CFG::WARPS_M) * CFG::WN;
   const int g = lane >> 2, t = lane & 3;
-  const bool bz = beta.x == 0.0 && beta.y == 0.0;
   const int t_begin = start[blockIdx.x], t_end = start[blockIdx.x + 1];
   // The stages of all the CTA's tasks form one stream through the ring: the copies run NST − 1 stages
   // ahead of the products and go on into the next task while this one finishes.
@@ -473,7 +476,7 @@ __global__ void __launch_bounds__(CFG::THREADS, CFG::MINB)
       else return make_double2(alpha.x * f[0] - alpha.y * f[4], alpha.x * f[4] + alpha.y * f[0]);
     };
     auto column = [](int q) { return (q / 2) * 8 + (q % 2); };
-    if (bz) {
+    if (BZ || (!CFG::BETA_KERNEL && beta.x == 0.0 && beta.y == 0.0)) {
 #pragma unroll
       for (int q = 0; q < 2 * CFG::NI; ++q) {
         if (column(q) >= cols) continue;
@@ -482,35 +485,35 @@ __global__ void __launch_bounds__(CFG::THREADS, CFG::MINB)
         for (int h = 0; h < 2 * CFG::MI; ++h)
           if (h * 8 < rows) p[h * 8] = value(q, h);
       }
-      continue;
-    }
-    // the old values of G columns are read at a time: 16 loads in flight (one column at a time, each column waited
-    // for its own: 2048x64x2048 41.4 us with β, 36.3 so, 30.9 without)
-    constexpr int G = CFG::CPLX || CFG::NI < 2 ? 2 : 4;
+    } else if constexpr (!BZ) {
+      // the old values of G columns are read at a time: 16 loads in flight (one column at a time, each column waited
+      // for its own: 2048x64x2048 41.4 us with β, 36.3 so, 30.9 without)
+      constexpr int G = CFG::CPLX || CFG::NI < 2 ? 2 : 4;
 #pragma unroll
-    for (int q0 = 0; q0 < 2 * CFG::NI; q0 += G) {
-      E old[G][2 * CFG::MI];
+      for (int q0 = 0; q0 < 2 * CFG::NI; q0 += G) {
+        E old[G][2 * CFG::MI];
 #pragma unroll
-      for (int q = q0; q < q0 + G; ++q)
+        for (int q = q0; q < q0 + G; ++q)
 #pragma unroll
-        for (int h = 0; h < 2 * CFG::MI; ++h)
-          if (column(q) < cols && h * 8 < rows) old[q - q0][h] = pc[column(q) * ldc + h * 8];
+          for (int h = 0; h < 2 * CFG::MI; ++h)
+            if (column(q) < cols && h * 8 < rows) old[q - q0][h] = pc[column(q) * ldc + h * 8];
 #pragma unroll
-      for (int q = q0; q < q0 + G; ++q) {
-        if (column(q) >= cols) continue;
-        E *p = pc + column(q) * ldc;
+        for (int q = q0; q < q0 + G; ++q) {
+          if (column(q) >= cols) continue;
+          E *p = pc + column(q) * ldc;
 #pragma unroll
-        for (int h = 0; h < 2 * CFG::MI; ++h) {
-          if (h * 8 < rows) {
-            E r = value(q, h);
-            const E &o = old[q - q0][h];
-            if constexpr (!CFG::CPLX) {
-              r = fma(beta.x, o, r);
-            } else {
-              r.x = fma(beta.x, o.x, fma(-beta.y, o.y, r.x));
-              r.y = fma(beta.x, o.y, fma(beta.y, o.x, r.y));
+          for (int h = 0; h < 2 * CFG::MI; ++h) {
+            if (h * 8 < rows) {
+              E r = value(q, h);
+              const E &o = old[q - q0][h];
+              if constexpr (!CFG::CPLX) {
+                r = fma(beta.x, o, r);
+              } else {
+                r.x = fma(beta.x, o.x, fma(-beta.y, o.y, r.x));
+                r.y = fma(beta.x, o.y, fma(beta.y, o.x, r.y));
+              }
+              p[h * 8] = r;
             }
-            p[h * 8] = r;
           }
         }
       }
@@ -848,13 +851,19 @@ int tkb_gemm_thin_launch(tkb_ctx *ctx, const tkb_plan *p, void *C, const void *A
 
 namespace {
 struct PlainKernel {
-  const void *fn;
+  const void *fn, *fn_beta;  // without and with β
   int threads, bm, bn;
   size_t smem;
 };
 template <typename CFG>
 PlainKernel plain_kernel_of() {
-  return PlainKernel{(const void *)gemm_plain_kernel<CFG>, CFG::THREADS, CFG::BM, CFG::BN, CFG::SMEM};
+  return PlainKernel{(const void *)gemm_plain_kernel<CFG, CFG::BETA_KERNEL>, (const void *)gemm_plain_kernel<CFG, false>, CFG::THREADS,
+                     CFG::BM, CFG::BN, CFG::SMEM};
+}
+// CTAs per SM of both kernels of a shape (raises their shared memory limits)
+int plain_occupancy(tkb_ctx *ctx, const PlainKernel &k) {
+  return std::min(tkb_occupancy(ctx->device, k.fn, k.threads, k.smem),
+                  tkb_occupancy(ctx->device, k.fn_beta, k.threads, k.smem));
 }
 PlainKernel plain_kernel(bool cplx, bool small) {
   return cplx ? (small ? plain_kernel_of<SmallTileC>() : plain_kernel_of<LargeTileC>())
@@ -865,7 +874,8 @@ cudaError_t plain_launch(tkb_ctx *ctx, const tkb_plan *p, void *C, const void *A
                          tkb_scalar beta, int base_ok) {
   using E = typename CFG::E;
   // the shared-memory limit was raised when the plan queried the kernel's occupancy
-  return launch_pdl(gemm_plain_kernel<CFG>, dim3(p->pgrid), dim3(CFG::THREADS), CFG::SMEM, ctx->stream, p->blocks,
+  const auto k = beta.re == 0.0 && beta.im == 0.0 ? gemm_plain_kernel<CFG, CFG::BETA_KERNEL> : gemm_plain_kernel<CFG, false>;
+  return launch_pdl(k, dim3(p->pgrid), dim3(CFG::THREADS), CFG::SMEM, ctx->stream, p->blocks,
                     (const PTask *)p->ptasks, (const int32_t *)p->pstart, (E *)C, (const E *)A, (const E *)B,
                     CDbl{alpha.re, alpha.im}, CDbl{beta.re, beta.im}, p->part, p->pcnt, base_ok);
 }
@@ -887,7 +897,7 @@ int tkb_gemm_plain_prepare(tkb_ctx *ctx, tkb_plan *p) {
   if (cplx) {
     p->plain_small = small_tiles <= (int64_t)ctx->num_sms * 16;
   } else {
-    const int large_sm = tkb_occupancy(ctx->device, large.fn, large.threads, large.smem);
+    const int large_sm = plain_occupancy(ctx, large);
     const bool fills = large_pieces * 20 >= (int64_t)ctx->num_sms * large_sm * 17;
     const bool padded = large_steps * 4 * 5 > small_steps * 6;  // a step of the large tile is four of the small one
     p->plain_small = !fills || padded;
@@ -898,7 +908,7 @@ int tkb_gemm_plain_prepare(tkb_ctx *ctx, tkb_plan *p) {
   // four real ones
   const int min_steps = std::max(1, p->min_piece_steps * (p->plain_small ? 2 : 1) / (cplx ? 4 : 1));
   const int tile_cost = cplx ? 1 : 2;
-  const int per_sm = tkb_occupancy(ctx->device, pk.fn, pk.threads, pk.smem);
+  const int per_sm = plain_occupancy(ctx, pk);
   if (per_sm <= 0) return tkb_set_error(ctx, TKB_ERR_CUDA, "plain GEMM: occupancy query failed");
   const int64_t slots = (int64_t)ctx->num_sms * per_sm;
   std::vector<GTile> tiles;

@@ -107,8 +107,8 @@ __device__ __forceinline__ void dmma16_first(double (&c)[4], const double (&a)[4
 //   Halves: one for each half of a stage
 //   Stage:  a stage is summed from zero, then added. An FP64 addition per value and stage takes 6 % of the pipe
 //           that the DMMA need, which does not show while the launch waits for latency (32×32 real tiles)
-//   Stages: the same every fourth stage (32×32 complex tiles, which also run launches bound by the DMMA: 70.7 us
-//           for an SU(2) environment update at V dim 2406, 68.8 with One, 82.4 with Stage)
+//   Stages: the same every fourth stage (32×32 complex tiles, which also run launches bound by the DMMA: 69.7 us
+//           for an SU(2) environment update at V dim 2406, 69.6 with One, 82.4 with Stage)
 enum class Sum { One, Halves, Stage, Stages };
 constexpr int kSumStages = 4;
 
@@ -415,24 +415,29 @@ __global__ void __launch_bounds__(CFG::THREADS, CFG::MINB)
     for (int q = 0; q < CFG::NACC; ++q) acc[q] = 0.0;
     const int nk = task.kind == 0 ? task.ke - task.kb : 0;
     auto k_loop = [&](auto ak, auto bk) {  // one loop per pair of layouts: no test inside
-      for (int kt = 0; kt < nk; ++kt) {
+      auto stage = [&]() {
         cp_async_wait<CFG::NST - 2>();
         __syncthreads();  // this stage is visible to all; every warp is done with the slot before it
         const E *st = sm + slot * CFG::STAGE;
         stage_products<CFG, decltype(ak)::value, decltype(bk)::value>(acc, st, st + CFG::A_ELEMS, wm + g, wn + g, t,
                                                                       conjA, conjB);
-        if constexpr (CFG::SUM == Sum::Stages) {
-          if (kt % kSumStages == kSumStages - 1) {
-#pragma unroll
-            for (int q = 0; q < CFG::NV; ++q) {
-              acc[CFG::NV + q] += acc[q];
-              acc[q] = 0.0;
-            }
-          }
-        }
         // the refill of the slot read in the previous iteration is issued while the DMMA execute
         produce(slot == 0 ? CFG::NST - 1 : slot - 1);
         slot = slot + 1 == CFG::NST ? 0 : slot + 1;
+      };
+      if constexpr (CFG::SUM == Sum::Stages) {  // loops in a loop: the stages stay free of the test
+        for (int kt = 0; kt < nk;) {
+          const int stop = min(nk, kt + kSumStages);
+#pragma unroll 1
+          for (; kt < stop; ++kt) stage();
+#pragma unroll
+          for (int q = 0; q < CFG::NV; ++q) {
+            acc[CFG::NV + q] += acc[q];
+            acc[q] = 0.0;
+          }
+        }
+      } else {
+        for (int kt = 0; kt < nk; ++kt) stage();
       }
     };
     constexpr std::true_type yes{};

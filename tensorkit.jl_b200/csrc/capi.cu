@@ -335,8 +335,8 @@ static int plan_create(tkb_ctx *ctx, const tkb_gemm_desc *d, const tkb_gemm_tuni
   // operands are, the FP64 kernel 3 - 5 us: an SU(2) environment update (two products) takes 41.8 us
   // sliced and 10.3 in FP64 at V dim 280, 47.1 and 16.5 at 870 (4 MFLOP per product). The line is the
   // largest size at which those were measured, not the crossing, which lies far above it for real data: at 374 MFLOP
-  // per product the update takes 69.8 us sliced and 51.1 in FP64, a U(1) effective Hamiltonian (7.7 GFLOP)
-  // 433 and 434. Precision "auto" measures both for a structure.
+  // per product the update takes 69.9 us sliced and 49.9 in FP64, a U(1) effective Hamiltonian (7.7 GFLOP)
+  // 434 and 430. Precision "auto" measures both for a structure.
   p->small_fp64 = d->precision == TKB_SPLIT_INT8 && d->slices == 0 && flops < kSplitMinFlops;
   if (d->precision == TKB_SPLIT_INT8 && !p->small_fp64) rc = tkb_gemm_split_prepare(ctx, p);
   else rc = tkb_gemm_plain_prepare(ctx, p);

@@ -21,8 +21,8 @@
 //
 // What bounds it: the DMMA pipe runs m16n8k8 at 64 cycles per SM sub-partition (37 TFLOP/s measured on
 // B200), and every instruction issued beside it costs: with addresses and bounds resolved once per
-// task one 4096³ block runs at 33.5 TFLOP/s (30.1 when each copy worked out its own address), one
-// 4095³ block (8-byte copies) at 32.5 (26.8), one complex 2048³ block at 32.8 (30.4). The epilogue
+// task one 4096³ block runs at 33.7 TFLOP/s (30.1 when each copy worked out its own address), one
+// 4095³ block (8-byte copies) at 32.8 (26.8), one complex 2048³ block at 32.7 (30.4). The epilogue
 // keeps one pointer per column of a thread: 9 blocks of K ≤ 256 and a 59 MB output take 152 us (176 with an
 // address per element, 37 us of it in the epilogues). Taken back: fragments of the next sub-step loaded ahead of the DMMA (517 instead of
 // 489 us on a U(1) effective Hamiltonian; the DMMA wait for the loads issued before them).
@@ -529,7 +529,7 @@ __global__ void __launch_bounds__(CFG::THREADS, CFG::MINB)
   PL_STAMP(4);
 }
 
-// LargeTile: two CTAs of four 32×32 warps per SM (240 registers with both accumulators; with one, three CTAs
+// LargeTile: two CTAs of four 32×32 warps per SM (218 registers, 240 with β, with both accumulators; with one, three CTAs
 // at 168 registers ran 4096³ at 32.5 instead of 33.8 TFLOP/s, eight 32×16 warps at 29.7). SmallTile: six CTAs of four 16×16 warps
 // per SM, for launches whose 64×64 tiles would leave most of the chip to one CTA per SM, which spends
 // 0.87 us per K step where its DMMA take 0.52.
